@@ -127,7 +127,8 @@ def _seismic(g, b, n):
         peak = 10.0 + 50.0 * u[:, :1]
         spikes = 20 + (61 * u[:, 1:]).long()
         # one spike a layer, so that no two fall on one sample
-        layer = torch.arange(80, device=dev) + torch.rand((k, 80), generator=g, dtype=torch.float64, device=dev)
+        u = torch.rand((k, 80), generator=g, dtype=torch.float64, device=dev)
+        layer = torch.arange(80, device=dev) + 0.5 * u
         pos = (n * layer / spikes).long().clamp(max=m - 1)
         v = torch.rand((k, 80), generator=g, dtype=torch.float64, device=dev) - 0.5
         amp = -torch.sign(v) * torch.log1p(-2.0 * v.abs().clamp(max=0.4999999))
