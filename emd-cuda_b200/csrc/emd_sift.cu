@@ -45,7 +45,6 @@
 #include "emdb_internal.cuh"
 
 // Tuning knobs (compile-time; results are identical for every setting):
-//  EMDB_EVAL_PAIR  evaluate two samples per loop trip in the fused pass
 //  EMDB_PCR_PAIR   update two PCR rows per loop trip
 //  EMDB_OUTLINE    rarely taken paths as calls instead of inline copies:
 //                  1 the general evaluation and the binary segment search,
@@ -58,15 +57,6 @@
 // 1/1 208.4k signals/s, 1/0 188.1k, 2/1 195.6k, 0/0 184.9k (and 0/1 172.7k on
 // another box against 208.2k for 1/1): less sift-pass code relieves
 // instruction supply, the dominant stall after FP64 latency.
-//  EMDB_FAST_DIV   reciprocal-based correctly rounded division in evaluation:
-//                  0 none, 1 segment quotients from stored RN(1/h) plus the
-//                  division by 6, 2 the division by 6 only, 3 segment quotients
-//                  from a per-sample RN(1/h) plus the division by 6
-// Measured on B200 (16,384 seismic traces x 2048 samples): the paired loops
-// raise register pressure more than they add overlap; EMDB_FAST_DIV 0/1/2/3
-// ran at 142.5k/154.3k/150.8k/154.9k signals/s, bit-identical outputs.  The
-// gain is the straight-line evaluation: every hardware division carries its
-// own slow-path branch, which splits the sample's independent chains.
 //  EMDB_PCR_NB     branch-free division with no reciprocal at hand (div_nb)
 //                  for the two PCR quotients of each row: 241.1k vs 222.8k
 //                  signals/s on one B200.  Used everywhere (evaluation and
@@ -80,12 +70,6 @@
 //  EMDB_SCAN_UNROLL / EMDB_FILL_UNROLL  unroll factors of the extrema scan
 //                  and knot fill loops: 4 measured 231.8k / 226.3k vs 240.2k
 //                  at 2.
-//  EMDB_SORTED_NOCHECK  skip the integer evaluation's operand-range checks
-//                  on sorted knot lists (only the table bound stays): 239.6k
-//                  vs 240.2k, so off.
-#ifndef EMDB_EVAL_PAIR
-#define EMDB_EVAL_PAIR 0
-#endif
 #ifndef EMDB_PCR_PAIR
 #define EMDB_PCR_PAIR 0
 #endif
@@ -116,9 +100,6 @@
 #ifndef EMDB_OUTLINE
 #define EMDB_OUTLINE 2
 #endif
-#ifndef EMDB_FAST_DIV
-#define EMDB_FAST_DIV 3
-#endif
 #ifndef EMDB_MERGED_PLACE
 #define EMDB_MERGED_PLACE 1
 #endif
@@ -142,9 +123,6 @@
 #endif
 #ifndef EMDB_FILL_UNROLL
 #define EMDB_FILL_UNROLL 2
-#endif
-#ifndef EMDB_SORTED_NOCHECK
-#define EMDB_SORTED_NOCHECK 0
 #endif
 //  EMDB_LOAD_CLOCKS  instrumented build: thread 0 of each CTA adds the clock64
 //                  cycles of every trace's load into shared memory, of the
@@ -178,8 +156,8 @@ constexpr int kPhases = 10;
 // float.  The FP64 build's division shortcuts (reciprocal tables, Markstein
 // and branch-free quotients) are off: float quotients are the IEEE ones, and
 // the one double quotient per envelope sample (the reference's "/ 6.0")
-// takes the Markstein quotient from RN(1/6) (EMDB_FAST_DIV 2), which equals
-// the double division.
+// is formed from RN(1/6) and its residual (div6), which equals the double
+// division.
 #ifndef EMDB_F32
 #define EMDB_F32 0
 #endif
@@ -191,8 +169,6 @@ constexpr int kPhases = 10;
 #ifndef EMDB_F32_FAST
 #define EMDB_F32_FAST 1
 #endif
-#undef EMDB_FAST_DIV
-#define EMDB_FAST_DIV (EMDB_F32_FAST ? 3 : 2)
 #undef EMDB_PCR_NB
 #define EMDB_PCR_NB EMDB_F32_FAST
 namespace emdb::f32 {
@@ -205,6 +181,10 @@ using real = double;
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
+
+// two values loaded and stored as one word
+struct alignas(2 * sizeof(real)) real2 { real x, y; };
+
 constexpr int kScanUnroll = EMDB_SCAN_UNROLL;
 constexpr int kFillUnroll = EMDB_FILL_UNROLL;
 constexpr int kLaneUnroll = EMDB_LANE_UNROLL;
@@ -263,10 +243,9 @@ struct SmemLayout {
   int* wc;            // [5][NW]: w_max | w_min | w_zc | w_zre | w_trig
   real* red;        // [6][128] between passes (= arena start)
   real* imf;        // [N]
-  uint32_t* mmax;     // [nch] ballot masks of the last extrema scan
-  uint32_t* mmin;
-  uint16_t* pmax;     // per-chunk exclusive prefix within the owning warp's range
-  uint16_t* pmin;
+  uint2* mm;          // [nch] ballot masks of the last extrema scan: maxima, minima
+  uint32_t* pp;       // per-chunk exclusive prefixes within the owning warp's range:
+                      // maxima | minima << 16 (the fill makes them global)
   char* arena;        // knot arena start
   int arena_bytes;    // bytes left for the knot arena
 };
@@ -293,10 +272,8 @@ __device__ __forceinline__ SmemLayout carve(char* base, int N, int arena_total,
   char* p = base;
   L.ctl = reinterpret_cast<Ctl*>(p); p += align16(sizeof(Ctl));
   L.wc = reinterpret_cast<int*>(p); p += align16(5 * (NT / 32) * sizeof(int));
-  L.mmax = reinterpret_cast<uint32_t*>(p); p += align16(nch * 4);
-  L.mmin = reinterpret_cast<uint32_t*>(p); p += align16(nch * 4);
-  L.pmax = reinterpret_cast<uint16_t*>(p); p += align16(nch * 2);
-  L.pmin = reinterpret_cast<uint16_t*>(p); p += align16(nch * 2);
+  L.mm = reinterpret_cast<uint2*>(p); p += align16(nch * 4) * 2;
+  L.pp = reinterpret_cast<uint32_t*>(p); p += align16(nch * 2) * 2;
   // the proto-IMF directly ahead of the arena: the borrow placement uses both
   // as one region
   if (kGImf) {
@@ -312,13 +289,10 @@ __device__ __forceinline__ SmemLayout carve(char* base, int N, int arena_total,
 
 // Knot / PCR storage for one sift pass (both envelopes).  After the last PCR
 // level only the b and d arrays of the final buffers are read, so the spline
-// moments M go into buffer 0's a (upper envelope) and c (lower) arrays and the
-// segment reciprocals R into buffer 1's a and c arrays.
+// moments M go into buffer 0's a (upper envelope) and c (lower) arrays.
 struct Knots {
-  real* X[2];
-  real* Y[2];
+  real2* XY[2]; // (position, value) of each knot
   real* M[2];
-  real* R[2];   // RN(1/h) per knot segment, in buffer 1's a / c arrays
   real* P[2];   // ping-pong PCR buffers: a | b | c | d, each `cap` rows
   real* red;    // reduction lanes after the solve: buffer 1, or just past it
   int cap;
@@ -327,26 +301,22 @@ struct Knots {
 __host__ __device__ inline size_t knot_bytes(int kc0, int kc1) {
   // size_t throughout: a host-side size query must not wrap for any int input
   const size_t cap = (size_t)kc0 + (size_t)kc1;
-  // with EMDB_FAST_DIV 1 buffer 1 holds the segment reciprocals during evaluation
-  const size_t red_extra = (EMDB_FAST_DIV != 1 && 4 * cap >= (size_t)kRedDoubles) ? 0 : kRedBytes;
+  const size_t red_extra = (4 * cap >= (size_t)kRedDoubles) ? 0 : kRedBytes;
   return (2 * cap + 8 * cap) * sizeof(real) + red_extra;
 }
 
 __device__ __forceinline__ Knots place_knots(char* base, int kc0, int kc1) {
   Knots K;
   real* p = reinterpret_cast<real*>(base);
-  K.X[0] = p; p += kc0;
-  K.Y[0] = p; p += kc0;
-  K.X[1] = p; p += kc1;
-  K.Y[1] = p; p += kc1;
+  K.XY[0] = reinterpret_cast<real2*>(p);
+  K.XY[1] = K.XY[0] + kc0;
+  p += 2 * (kc0 + kc1);
   K.cap = kc0 + kc1;
   K.P[0] = p; p += 4 * K.cap;
   K.P[1] = p;
   K.M[0] = K.P[0];
   K.M[1] = K.P[0] + 2 * K.cap;
-  K.R[0] = K.P[1];
-  K.R[1] = K.P[1] + 2 * K.cap;
-  K.red = (EMDB_FAST_DIV != 1 && 4 * K.cap >= kRedDoubles) ? K.P[1] : K.P[1] + 4 * K.cap;
+  K.red = (4 * K.cap >= kRedDoubles) ? K.P[1] : K.P[1] + 4 * K.cap;
   return K;
 }
 
@@ -362,21 +332,18 @@ __device__ __forceinline__ Knots place_knots_split(char* sbase, int sbytes, char
                                                    int kc1) {
   Knots K;
   real* p = reinterpret_cast<real*>(sbase);
-  K.X[0] = p; p += kc0;
-  K.Y[0] = p; p += kc0;
-  K.X[1] = p; p += kc1;
-  K.Y[1] = p; p += kc1;
+  K.XY[0] = reinterpret_cast<real2*>(p);
+  K.XY[1] = K.XY[0] + kc0;
+  p += 2 * (kc0 + kc1);
   K.cap = kc0 + kc1;
   K.P[0] = p; p += 4 * K.cap;
   K.P[1] = reinterpret_cast<real*>(gbase);
   K.M[0] = K.P[0];
   K.M[1] = K.P[0] + 2 * K.cap;
-  K.R[0] = K.P[1];
-  K.R[1] = K.P[1] + 2 * K.cap;
   // reduction lanes: shared memory past buffer 0 when they fit, else the slab
   // (buffer 1 is dead after the solve; the slab holds knot_bytes of the largest pass)
   if (split_bytes(kc0, kc1) + kRedBytes <= (size_t)sbytes) K.red = p;
-  else K.red = (EMDB_FAST_DIV != 1 && 4 * K.cap >= kRedDoubles) ? K.P[1] : K.P[1] + 4 * K.cap;
+  else K.red = (4 * K.cap >= kRedDoubles) ? K.P[1] : K.P[1] + 4 * K.cap;
   return K;
 }
 
@@ -390,7 +357,7 @@ __host__ __device__ inline bool borrow_fits(int N, int arena_bytes, size_t slab_
                                             int kc1) {
   const size_t cap = (size_t)kc0 + (size_t)kc1;
   const size_t region = align16((size_t)N * sizeof(real)) + (size_t)arena_bytes;
-  return EMDB_FAST_DIV != 1 && 6 * cap * sizeof(real) <= (size_t)arena_bytes &&
+  return 6 * cap * sizeof(real) <= (size_t)arena_bytes &&
          10 * cap * sizeof(real) <= region &&
          (align16((size_t)N * sizeof(real)) + kRedBytes) <= slab_stride;
 }
@@ -402,16 +369,13 @@ __device__ __forceinline__ Knots place_knots_borrow(real* imf, char* arena, int 
   Knots K;
   K.cap = kc0 + kc1;
   real* p = reinterpret_cast<real*>(arena + arena_bytes) - 6 * K.cap;
-  K.X[0] = p; p += kc0;
-  K.Y[0] = p; p += kc0;
-  K.X[1] = p; p += kc1;
-  K.Y[1] = p; p += kc1;
+  K.XY[0] = reinterpret_cast<real2*>(p);
+  K.XY[1] = K.XY[0] + kc0;
+  p += 2 * (kc0 + kc1);
   K.P[0] = p;
   K.P[1] = imf;
   K.M[0] = K.P[0];
   K.M[1] = K.P[0] + 2 * K.cap;
-  K.R[0] = K.P[1];
-  K.R[1] = K.P[1] + 2 * K.cap;
   K.red = reinterpret_cast<real*>(slab + align16((size_t)N * sizeof(real)));
   return K;
 }
@@ -427,7 +391,7 @@ __host__ __device__ inline bool borrow2_fits(int N, int arena_bytes, size_t slab
                                              int kc1) {
   const size_t cap = (size_t)kc0 + (size_t)kc1;
   const size_t region = align16((size_t)N * sizeof(real)) + (size_t)arena_bytes;
-  return EMDB_FAST_DIV != 1 && 3 * cap * sizeof(real) <= (size_t)arena_bytes &&
+  return 3 * cap * sizeof(real) <= (size_t)arena_bytes &&
          11 * cap * sizeof(real) <= region &&
          (align16((size_t)N * sizeof(real)) + kRedBytes) <= slab_stride;
 }
@@ -437,16 +401,13 @@ __device__ __forceinline__ Knots place_knots_borrow2(real* imf, char* arena, int
   Knots K;
   K.cap = kc0 + kc1;
   real* p = reinterpret_cast<real*>(arena + arena_bytes) - 3 * K.cap;
-  K.X[0] = p; p += kc0;
-  K.Y[0] = p; p += kc0;
-  K.X[1] = p; p += kc1;
-  K.Y[1] = p; p += kc1;
   K.M[0] = p;
   K.M[1] = p + kc0;
+  p += K.cap;         // the pairs last: 16-byte aligned whatever the knot count
+  K.XY[0] = reinterpret_cast<real2*>(p);
+  K.XY[1] = K.XY[0] + kc0;
   K.P[0] = imf;
   K.P[1] = imf + 4 * K.cap;
-  K.R[0] = K.P[1];
-  K.R[1] = K.P[1] + 2 * K.cap;
   K.red = reinterpret_cast<real*>(slab + align16((size_t)N * sizeof(real)));
   return K;
 }
@@ -463,7 +424,7 @@ __host__ __device__ inline bool park_fits(int N, int arena_bytes, size_t slab_st
                                           int kc1) {
   const size_t cap = (size_t)kc0 + (size_t)kc1;
   const size_t imfb = align16((size_t)N * sizeof(real));
-  return EMDB_FAST_DIV != 1 && 4 * cap * sizeof(real) <= imfb + (size_t)arena_bytes &&
+  return 4 * cap * sizeof(real) <= imfb + (size_t)arena_bytes &&
          imfb + 6 * cap * sizeof(real) <= slab_stride;
 }
 
@@ -472,16 +433,13 @@ __device__ __forceinline__ Knots place_knots_park(real* imf, char* slab, int N, 
   Knots K;
   K.cap = kc0 + kc1;
   real* p = reinterpret_cast<real*>(slab + align16((size_t)N * sizeof(real)));
-  K.X[0] = p; p += kc0;
-  K.Y[0] = p; p += kc0;
-  K.X[1] = p; p += kc1;
-  K.Y[1] = p; p += kc1;
+  K.XY[0] = reinterpret_cast<real2*>(p);
+  K.XY[1] = K.XY[0] + kc0;
+  p += 2 * (kc0 + kc1);
   K.P[0] = p;
   K.P[1] = imf;
   K.M[0] = K.P[0];
   K.M[1] = K.P[0] + 2 * K.cap;
-  K.R[0] = K.P[1];
-  K.R[1] = K.P[1] + 2 * K.cap;
   K.red = red;
   return K;
 }
@@ -575,12 +533,11 @@ __device__ __forceinline__ float div_nb(float a, float b, bool& slow) {
 // the fast quotients' range, knot lists that are not strictly increasing) as
 // calls to one out-of-line body each, instead of an inline copy per call site:
 // keeps the hot loops' code small.  Defined after eval_seg / search_seg.
-__device__ __noinline__ real eval_seg_cold(const real* x, const real* y, const real* M,
-                                             int n, real t, int lo);
-__device__ __noinline__ int search_seg_cold(const real* x, int n, real t);
+__device__ __noinline__ real eval_seg_cold(const real2* xy, const real* M, int n, real t, int lo);
+__device__ __noinline__ int search_seg_cold(const real2* xy, int n, real t);
 #if EMDB_OUTLINE >= 1
-#define EMDB_EVAL_RARE(sv, t, lo) eval_seg_cold((sv).x, (sv).y, (sv).M, (sv).n, (t), (lo))
-#define EMDB_SEARCH_RARE(sv, t) search_seg_cold((sv).x, (sv).n, (t))
+#define EMDB_EVAL_RARE(sv, t, lo) eval_seg_cold((sv).xy, (sv).M, (sv).n, (t), (lo))
+#define EMDB_SEARCH_RARE(sv, t) search_seg_cold((sv).xy, (sv).n, (t))
 #else
 #define EMDB_EVAL_RARE(sv, t, lo) eval_seg((sv), (t), (lo))
 #define EMDB_SEARCH_RARE(sv, t) search_seg((sv), (t))
@@ -643,7 +600,27 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
   return slow ? div_slow(a, b) : q;
 }
 #endif
-constexpr double kInv6 = 1.0 / 6.0;   // RN(1/6), folded at compile time
+
+// RN(x / 6) for the spline term (kernels.py:733) in two operations: with
+// 1/6 = C + c, C = RN(1/6), the product x*C plus the rounded correction x*c is
+// within 2^-104 |x/6| of x/6 before its one rounding (multiplication by a
+// constant held as two words: Brisebarre and Muller, IEEE Trans. Computers
+// 57(2), 2008), and x/6 is never closer than a sixth of its ulp u to a
+// rounding boundary m: x is a multiple of 4u and 6m an odd multiple of u, so
+// |x - 6m| >= u.  `slow` is set for a non-zero x outside
+// [2^-900, 2^900) (subnormal products, infinities, NaN).  Checked against the
+// division by emdb_check_division mode 1.
+constexpr double kInv6 = 1.0 / 6.0;
+constexpr double kInv6Lo = kInv6 / 18014398509481984.0;   // RN(1/6 - RN(1/6)) = RN(1/6) / 2^54
+__device__ __forceinline__ bool odd_range(double x) {
+  const unsigned v = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  // exponents [-900, 900): biased 123..1922
+  return (v - (123u << 20)) >= (1800u << 20) && (v | (unsigned)__double2loint(x)) != 0u;
+}
+__device__ __forceinline__ double div6(double x, bool& slow) {
+  slow |= odd_range(x);
+  return fma(x, kInv6, x * kInv6Lo);
+}
 
 // RN(1/h) for integer h in [1, kRcpTab], built at compile time by IEEE
 // division and shipped initialised in the module.
@@ -707,8 +684,8 @@ __device__ __forceinline__ void extrema_count(const SmemLayout& L, int N, int sl
     uint32_t bmax = __ballot_sync(kFull, ismax);
     uint32_t bmin = __ballot_sync(kFull, ismin);
     if (lane == 0) {
-      L.mmax[c] = bmax; L.mmin[c] = bmin;
-      L.pmax[c] = (uint16_t)rmax; L.pmin[c] = (uint16_t)rmin;
+      L.mm[c] = make_uint2(bmax, bmin);
+      L.pp[c] = (uint32_t)rmax | ((uint32_t)rmin << 16);
     }
     rmax += __popc(bmax);
     rmin += __popc(bmin);
@@ -836,10 +813,7 @@ __device__ __forceinline__ bool fill_true_knots(const SmemLayout& L, const Knots
                       : e.off_min + pn + __popc(bn & lt);
     int nq = q == 0 ? e.n_max : e.n_min;
     if (rank < nq) {
-      real* Xq = q == 0 ? K.X[0] : K.X[1];
-      real* Yq = q == 0 ? K.Y[0] : K.Y[1];
-      Xq[NB + rank] = T(ii);
-      Yq[NB + rank] = v;
+      (q == 0 ? K.XY[0] : K.XY[1])[NB + rank] = real2{T(ii), v};
       bad |= q == 0 ? (v < 0.0) : (v > 0.0);
       if (rank <= NB) C.head[q][rank] = ii;
       int fe = nq - 1 - rank;
@@ -850,8 +824,8 @@ __device__ __forceinline__ bool fill_true_knots(const SmemLayout& L, const Knots
     // no exact zeros or flat runs in this proto-IMF: every extremum is strict
 #pragma unroll kFillUnroll
     for (int c = c0; c < c1; ++c) {
-      const uint32_t bm = L.mmax[c], bn = L.mmin[c];
-      const int pm = L.pmax[c], pn = L.pmin[c];
+      const uint32_t bm = L.mm[c].x, bn = L.mm[c].y;
+      const int pm = L.pp[c] & 0xffff, pn = L.pp[c] >> 16;
       if (((bm | bn) >> lane) & 1u) {
         const int i = (c << 5) + lane;
         put(bm, bn, pm, pn, i, imf[i]);
@@ -859,8 +833,8 @@ __device__ __forceinline__ bool fill_true_knots(const SmemLayout& L, const Knots
     }
   } else {
     for (int c = c0; c < c1; ++c) {
-      const uint32_t bm = L.mmax[c], bn = L.mmin[c];
-      const int pm = L.pmax[c], pn = L.pmin[c];
+      const uint32_t bm = L.mm[c].x, bn = L.mm[c].y;
+      const int pm = L.pp[c] & 0xffff, pn = L.pp[c] >> 16;
       if (!(((bm | bn) >> lane) & 1u)) continue;
       int i = (c << 5) + lane;
       int ii = i;
@@ -878,10 +852,8 @@ __device__ __forceinline__ bool fill_true_knots(const SmemLayout& L, const Knots
   // the chunks' prefixes become global (warp offset added) for the evaluation
   // pass's segment counts, once every lane has taken its ranks
   __syncwarp();
-  for (int c = c0 + lane; c < c1; c += 32) {
-    L.pmax[c] = (uint16_t)(L.pmax[c] + e.off_max);
-    L.pmin[c] = (uint16_t)(L.pmin[c] + e.off_min);
-  }
+  const uint32_t off = (uint32_t)e.off_max | ((uint32_t)e.off_min << 16);
+  for (int c = c0 + lane; c < c1; c += 32) L.pp[c] += off;
   return bad;
 }
 
@@ -1015,8 +987,7 @@ __device__ __forceinline__ bool mirror_both(const SmemLayout& L, const Knots& K,
     real val = S[idx];
     int nside = side == 0 ? nM : nm;
     int slot = left ? (NB - cq + j) : (NB + nside + j);
-    (side == 0 ? K.X[0] : K.X[1])[slot] = pos;
-    (side == 0 ? K.Y[0] : K.Y[1])[slot] = val;
+    (side == 0 ? K.XY[0] : K.XY[1])[slot] = real2{pos, val};
     bad |= side == 0 ? (val < 0.0) : (val > 0.0);
   }
   return bad;
@@ -1025,14 +996,26 @@ __device__ __forceinline__ bool mirror_both(const SmemLayout& L, const Knots& K,
 // ---------------------------------------------------------------------------
 // Not-a-knot spline: reduced system + PCR + moments (kernels.py:607-697).
 // ---------------------------------------------------------------------------
+// the two halves of a pair array
+struct PairX {
+  const real2* p;
+  __device__ __forceinline__ real operator[](int i) const { return p[i].x; }
+};
+struct PairY {
+  const real2* p;
+  __device__ __forceinline__ real operator[](int i) const { return p[i].y; }
+};
+
 // kInt: integer time axis (T = arange), where knot spacings are integers and
 // the interior rows' slope quotients take RN(1/h) from the table and the exact
 // two-step Markstein quotient (div_q) instead of two divisions; spacings
 // outside the table (or not positive integers, as unsorted knot lists can
 // give) take the divisions.
 template <bool kInt = false>
-__device__ __forceinline__ void setup_row(const real* x, const real* y, int n, int k, int m,
+__device__ __forceinline__ void setup_row(const real2* xy, int n, int k, int m,
                                           real& a, real& b, real& c, real& d) {
+  const PairX x{xy};
+  const PairY y{xy};
   if (k == 0) {
     real h0 = x[1] - x[0], h1 = x[2] - x[1];
     real rhs1 = 6.0 * ((y[2] - y[1]) / h1 - (y[1] - y[0]) / h0);
@@ -1107,17 +1090,13 @@ __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kb
   const int m1 = kcnt1 >= 4 ? kcnt1 - 2 : 0;
   const int mt = m0 + m1;
   const int cap = K.cap;
-  const real* x0b = K.X[0] + kbase0;
-  const real* x1b = K.X[1] + kbase1;
-  const real* y0b = K.Y[0] + kbase0;
-  const real* y1b = K.Y[1] + kbase1;
+  const real2* xy0 = K.XY[0] + kbase0;
+  const real2* xy1 = K.XY[1] + kbase1;
   for (int r = tid; r < mt; r += NT) {
     const bool s0 = r < m0;
     const int k = s0 ? r : r - m0;
-    const real* x = s0 ? x0b : x1b;
-    const real* y = s0 ? y0b : y1b;
     real a, b, c, d;
-    setup_row<kInt>(x, y, s0 ? kcnt0 : kcnt1, k, s0 ? m0 : m1, a, b, c, d);
+    setup_row<kInt>(s0 ? xy0 : xy1, s0 ? kcnt0 : kcnt1, k, s0 ? m0 : m1, a, b, c, d);
     real* P = K.P[0];
     P[r] = a; P[cap + r] = b; P[2 * cap + r] = c; P[3 * cap + r] = d;
   }
@@ -1162,14 +1141,9 @@ __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kb
     const int n = s0 ? kcnt0 : kcnt1;
     const real* Pf = (s0 ? fin0 : fin1) ? K.P[1] : K.P[0];
     real* M = s0 ? K.M[0] : K.M[1];
-    const real* x = s0 ? x0b : x1b;
+    const PairX x{s0 ? xy0 : xy1};
     real Mk1 = Pf[3 * cap + r] / Pf[cap + r];
     M[k + 1] = Mk1;
-#if EMDB_FAST_DIV == 1
-    real* R = s0 ? K.R[0] : K.R[1];
-    R[k] = 1.0 / (x[k + 1] - x[k]);
-    if (k == mq - 1) R[k + 1] = 1.0 / (x[k + 2] - x[k + 1]);
-#endif
     if (k == 0) {
       real M2 = Pf[3 * cap + r + 1] / Pf[cap + r + 1];
       real h0 = x[1] - x[0], h1 = x[2] - x[1];
@@ -1185,20 +1159,18 @@ __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kb
   if (C) EMDB_PH(C, 4);
 }
 
-// One PCR row update (kernels.py:651-668), in the reference's operation order.
+// One envelope's spline: knots, moments, knot count, mirrored-left and true knots.
 struct SideView {
-  const real* x;
-  const real* y;
+  const real2* xy;
   const real* M;
-  const real* R;
-  int n;          // knots
-  int nl, nt;     // mirrored-left and true knots
+  int n;
+  int nl, nt;
 };
 
 // Envelope value at t in knot segment lo (kernels.py:706-733).
 __device__ __forceinline__ real eval_seg(const SideView& s, real t, int lo) {
-  const real* x = s.x;
-  const real* y = s.y;
+  const PairX x{s.xy};
+  const PairY y{s.xy};
   if (s.n == 2) {
     real slope = (y[1] - y[0]) / (x[1] - x[0]);
     return y[0] + slope * (t - x[0]);
@@ -1218,31 +1190,20 @@ __device__ __forceinline__ real eval_seg(const SideView& s, real t, int lo) {
   return A * y0 + B * y1 + ((A * A * A - A) * M0 + (B * B * B - B) * M1) * (h * h) / 6.0;
 }
 
-// eval_seg with the quotients taken from reciprocals (EMDB_FAST_DIV 1..3), in
-// the same operation order; sets `slow` when a quotient needs the division,
-// and the caller then re-evaluates the sample with eval_seg.
-__device__ __forceinline__ real eval_seg_q(const SideView& s, real t, int lo, bool& slow) {
-  if (s.n < 4) return EMDB_EVAL_RARE(s, t, lo);
-  const real* x = s.x;
-  const real* y = s.y;
-  real x0 = x[lo], x1 = x[lo + 1];
-  real y0 = y[lo], y1 = y[lo + 1];
-  real M0 = s.M[lo], M1 = s.M[lo + 1];
-  real h = x1 - x0;
-#if EMDB_FAST_DIV == 2
-  real A = (x1 - t) / h;
-  real B = (t - x0) / h;
-#else
-#if EMDB_FAST_DIV == 1
-  real rh = s.R[lo];
-#else
+// eval_seg for n >= 4 knots with the quotients formed without the division's
+// slow-path branch, in the same operation order; sets `slow` for operands
+// outside the exact range, and the caller then re-evaluates the sample with
+// eval_seg.
+__device__ __forceinline__ real eval_seg_q(const real2* xy, const real* M, real t, int lo,
+                                           bool& slow) {
+  const real2 p0 = xy[lo], p1 = xy[lo + 1];
+  const real M0 = M[lo], M1 = M[lo + 1];
+  const real h = p1.x - p0.x;
   const real rh = real(1) / h;
-#endif
-  real A = div_q(x1 - t, h, rh, slow);
-  real B = div_q(t - x0, h, rh, slow);
-#endif
-  real num = ((A * A * A - A) * M0 + (B * B * B - B) * M1) * (h * h);
-  return (A * y0 + B * y1) + div_q(num, 6.0, kInv6, slow);
+  const real A = div_q(p1.x - t, h, rh, slow);
+  const real B = div_q(t - p0.x, h, rh, slow);
+  const real num = ((A * A * A - A) * M0 + (B * B * B - B) * M1) * (h * h);
+  return (A * p0.y + B * p1.y) + div6(num, slow);
 }
 
 // The reference's per-sample binary search (kernels.py:722-726).
@@ -1250,22 +1211,17 @@ __device__ __forceinline__ int search_seg(const SideView& s, real t) {
   int lo = 0, hi = s.n - 2;
   while (lo < hi) {
     int mid = (lo + hi + 1) >> 1;
-    if (s.x[mid] <= t) lo = mid; else hi = mid - 1;
+    if (s.xy[mid].x <= t) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
 
 // Out-of-line bodies of the rare paths declared with div_slow.
-__device__ __noinline__ real eval_seg_cold(const real* x, const real* y, const real* M,
-                                             int n, real t, int lo) {
-  SideView s;
-  s.x = x; s.y = y; s.M = M; s.R = nullptr; s.n = n; s.nl = 0; s.nt = 0;
-  return eval_seg(s, t, lo);
+__device__ __noinline__ real eval_seg_cold(const real2* xy, const real* M, int n, real t, int lo) {
+  return eval_seg(SideView{xy, M, n, 0, 0}, t, lo);
 }
-__device__ __noinline__ int search_seg_cold(const real* x, int n, real t) {
-  SideView s;
-  s.x = x; s.y = nullptr; s.M = nullptr; s.R = nullptr; s.n = n; s.nl = 0; s.nt = 0;
-  return search_seg(s, t);
+__device__ __noinline__ int search_seg_cold(const real2* xy, int n, real t) {
+  return search_seg(SideView{xy, nullptr, n, 0, 0}, t);
 }
 
 // 128-lane tree of the reference (kernels.py:794-804), on warp 0, for a value
@@ -1372,45 +1328,108 @@ __device__ __forceinline__ void wide_lane_sums(real* red, const real* __restrict
   }
 }
 
-// eval_seg for the time axis T = arange(N): knot positions (true and
-// mirrored) and sample times are integers, so A = (x1-t)/h and B = (t-x0)/h
-// are quotients of integers 0 <= a <= h.  For those, q0 = RN(a*y) with
-// y = RN(1/h) and one correction RN(q0 + (a - h*q0)*y) equal RN(a/h): checked
-// exhaustively for every pair with h <= 65536 (2.1e9 pairs).  Anything outside
-// (h beyond the table, a not in [0, h]) sets `slow`, and the caller redoes the
-// sample with eval_seg.  Same operation order as eval_seg otherwise.
+// eval_seg for the time axis T = arange(N) on a strictly increasing knot list
+// of n >= 4 knots, t inside segment lo: knot positions (true and mirrored) and
+// sample times are integers, so A = (x1-t)/h and B = (t-x0)/h are quotients of
+// integers 0 <= a <= h.  For those, q0 = RN(a*y) with y = RN(1/h) and one
+// correction RN(q0 + (a - h*q0)*y) equal RN(a/h): checked exhaustively for
+// every pair with h <= 65536 (2.1e9 pairs).  A spacing past the table sets
+// `slow`, and the caller redoes the sample with eval_seg.  h + 2^52 holds the
+// integer h in its low word (no conversion instruction).
 #if !EMDB_F32
-__device__ __forceinline__ real eval_seg_int(const SideView& s, real t, int lo, bool& slow,
-                                               bool sorted = false) {
-  if (s.n < 4) return EMDB_EVAL_RARE(s, t, lo);
-  const real* x = s.x;
-  const real* y = s.y;
-  real x0 = x[lo], x1 = x[lo + 1];
-  real y0 = y[lo], y1 = y[lo + 1];
-  real M0 = s.M[lo], M1 = s.M[lo + 1];
-  real h = x1 - x0;
-  const real a = x1 - t, b = t - x0;
-  int hi;
-  if (EMDB_SORTED_NOCHECK && sorted) {
-    // strictly increasing integer knots and the segment that holds t: h is an
-    // integer >= 1 and a, b lie in [0, h]; only the table bound is left
-    const bool in = h <= (real)kRcpTab;
-    hi = in ? (int)h : 1;
-    slow |= !in;
-  } else {
-    const bool in = h >= 1.0 && h <= (real)kRcpTab && a >= 0.0 && b >= 0.0 && a <= h && b <= h;
-    hi = in ? (int)h : 1;
-    slow |= !in || (real)hi != h;
-  }
-  const real r = g_rcp.v[hi];
+__device__ __forceinline__ real eval_seg_int(const real2* xy, const real* M, real t, int lo,
+                                             bool& slow) {
+  const real2 p0 = xy[lo], p1 = xy[lo + 1];
+  const real M0 = M[lo], M1 = M[lo + 1];
+  const real h = p1.x - p0.x;
+  const real a = p1.x - t, b = t - p0.x;
+  const unsigned hi = (unsigned)__double2loint(h + 0x1p52);
+  slow |= hi > (unsigned)kRcpTab;
+  const real r = g_rcp.v[min(hi, (unsigned)kRcpTab)];
   real A = a * r;
   A = fma(fma(-A, h, a), r, A);
   real B = b * r;
   B = fma(fma(-B, h, b), r, B);
-  real num = ((A * A * A - A) * M0 + (B * B * B - B) * M1) * (h * h);
-  return (A * y0 + B * y1) + div_q(num, 6.0, kInv6, slow);
+  const real num = ((A * A * A - A) * M0 + (B * B * B - B) * M1) * (h * h);
+  return (A * p0.y + B * p1.y) + div6(num, slow);
 }
 #endif
+
+// Both envelopes at sample i (kernels.py:706-733).
+//
+// O(1) segments: for a strictly increasing knot list (nbsym <= 2, no flat
+// runs -- a plateau extremum sits at the run's midpoint, not at its flagged
+// first sample) the reference's binary search returns (number of knots at
+// or left of t) - 1, clamped to [0, n-2].  Otherwise run the search.  The
+// true knots at or left of a sample come from the scan's ballot masks
+// (global chunk prefix + popc).  Every left-mirrored knot lies at or left
+// of T[lsym] and every right-mirrored one at or right of T[rsym], so only
+// the chunks outside [lsym, rsym) compare them one by one; inside, with at
+// least one mirrored knot at each end, no clamp is needed either.
+//
+// A sample takes 27 FP64 operations per envelope on the integer axis; with the
+// range tests as compares of doubles, the two-step quotient by 6 and the
+// mirrored knots' compares in every chunk it took about 45.  The loop over
+// samples is kept rolled: the pass is bound by instruction supply as much as
+// by FP64 latency (unrolled by the compiler 93.5 ms, rolled 85.1 ms, 16,384 x
+// 2048 seismic).
+template <bool kInt>
+struct EnvEval {
+  const SideView s0, s1;
+  const bool fast;
+  const int iL, iR;
+  const unsigned incl;
+  __device__ __forceinline__ EnvEval(const SmemLayout& L, const Knots& K, const SideView& a,
+                                     const SideView& b, int NB, bool trig, int lane)
+      : s0(a), s1(b), fast(NB <= 2 && !trig && a.n >= 4 && b.n >= 4), iL(L.ctl->lsym),
+        iR(L.ctl->rsym), incl(lane == 31 ? kFull : ((2u << lane) - 1u)) {}
+  // segment of t, counted from the last left-mirrored knot, near the ends
+  static __device__ __forceinline__ int edge_seg(const SideView& s, int k, real t) {
+#pragma unroll 1
+    for (int j = 0; j < s.nl; ++j) k += s.xy[j].x <= t;
+#pragma unroll 1
+    for (int j = s.nl + s.nt; j < s.n; ++j) k += s.xy[j].x <= t;
+    return min(max(k - 1, 0), s.n - 2) - (s.nl - 1);
+  }
+  __device__ __forceinline__ void operator()(const SmemLayout& L, int i, real t, real& emax,
+                                             real& emin) const {
+    bool slow = !fast;
+    int lo0 = 0, lo1 = 0;
+    if (fast) {
+      const int c = i >> 5;
+      const uint2 m = L.mm[c];
+      const uint32_t pp = L.pp[c];
+      lo0 = min((int)(pp & 0xffffu) + __popc(m.x & incl), s0.nt);
+      lo1 = min((int)(pp >> 16) + __popc(m.y & incl), s1.nt);
+      if ((c << 5) < iL || (c << 5) + 31 >= iR) {
+        lo0 = edge_seg(s0, lo0, t);
+        lo1 = edge_seg(s1, lo1, t);
+      }
+      lo0 += s0.nl - 1;
+      lo1 += s1.nl - 1;
+#if !EMDB_F32
+      // (the FP32 build has no integer-axis shortcut: a float quotient formed
+      // in double from the table's RN(1/h) would be rounded twice)
+      if (kInt) {
+        emax = eval_seg_int(s0.xy, s0.M, t, lo0, slow);
+        emin = eval_seg_int(s1.xy, s1.M, t, lo1, slow);
+      } else
+#endif
+      {
+        emax = eval_seg_q(s0.xy, s0.M, t, lo0, slow);
+        emin = eval_seg_q(s1.xy, s1.M, t, lo1, slow);
+      }
+    }
+    if (slow) {
+      if (!fast) {
+        lo0 = s0.n >= 4 ? EMDB_SEARCH_RARE(s0, t) : 0;
+        lo1 = s1.n >= 4 ? EMDB_SEARCH_RARE(s1, t) : 0;
+      }
+      emax = EMDB_EVAL_RARE(s0, t, lo0);
+      emin = EMDB_EVAL_RARE(s1, t, lo1);
+    }
+  }
+};
 
 // One sift pass after the extrema scan of the current proto-IMF: knots,
 // mirroring, both splines, then the fused envelope / mean / update / partial
@@ -1457,13 +1476,16 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
   bad = __syncthreads_or(bad);
   EMDB_PH(&C, 0);
   bool mbad = false;
+  const bool lend = kPlace == kPlaceBorrow || kPlace == kPlaceBorrow2 || kPlace == kPlacePark;
+  // the wide instances also park it for the stop-test lanes, which read the
+  // old samples back after the update
+  const bool parked = lend || (kWide && !bad);
   if (warp == 0) {
     mbad = mirror_both(L, K, e, N, NB, T, lane);
   } else if (kWide) {
-    // park the proto-IMF while warp 0 mirrors: the lanes read the old samples
-    // back after the update (and the PCR buffers may overwrite imf[])
-    for (int i = tid - 32; i < N; i += NT - 32) park_old[i] = imf[i];
-  } else if (kPlace == kPlaceBorrow || kPlace == kPlaceBorrow2 || kPlace == kPlacePark) {
+    if (parked)
+      for (int i = tid - 32; i < N; i += NT - 32) park_old[i] = imf[i];
+  } else if (lend) {
     // park the proto-IMF while warp 0 mirrors; the PCR buffers overwrite it
     real* save = borrow_save(slab);
     for (int i = tid - 32; i < N; i += kThreads - 32) save[i] = imf[i];
@@ -1473,128 +1495,45 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
   const int kb0 = C.kbase[0], kb1 = C.kbase[1], kn0 = C.kcnt[0], kn1 = C.kcnt[1];
   solve_splines<NT, kInt && EMDB_SETUP_TAB>(K, kb0, kb1, kn0, kn1, tid,
                                              EMDB_LOAD_CLOCKS ? &C : nullptr);
-  const real* oldv = kWide ? park_old
-                     : (kPlace == kPlaceBorrow || kPlace == kPlaceBorrow2 || kPlace == kPlacePark)
-                            ? borrow_save(slab) : imf;
+  const real* oldv = !parked ? imf : kWide ? park_old : borrow_save(slab);
+  // A pass with a maximum below zero or a minimum above it is never the last
+  // one of its IMF, whatever the stop tests say (the reference forms their
+  // sums first and then drops them, kernels.py:773-776), so their terms,
+  // lane sums and trees are formed for the other passes only: 19 % of the
+  // passes of 2048-sample seismic traces, 9-11 % at 4096-8192.  B200, before /
+  // after: 256 x 8192 seismic 104.2 / 97.9 ms, 96 x 1501 2.09 / 1.84 ms.
+  const bool sums = !ps.bad;
 
-  SideView sv0, sv1;
-  sv0.x = K.X[0] + kb0; sv0.y = K.Y[0] + kb0; sv0.M = K.M[0]; sv0.R = K.R[0];
-  sv0.n = kn0; sv0.nl = NB - kb0; sv0.nt = e.n_max;
-  sv1.x = K.X[1] + kb1; sv1.y = K.Y[1] + kb1; sv1.M = K.M[1]; sv1.R = K.R[1];
-  sv1.n = kn1; sv1.nl = NB - kb1; sv1.nt = e.n_min;
+  const SideView sv0{K.XY[0] + kb0, K.M[0], kn0, NB - kb0, e.n_max};
+  const SideView sv1{K.XY[1] + kb1, K.M[1], kn1, NB - kb1, e.n_min};
 
   ps.sq = ps.dsq = ps.osq = ps.std_ = 0.0;
   ps.omax = -1e30;
   ps.omin = 1e30;
   bool oor = false;
-  // O(1) segments: for a strictly increasing knot list (nbsym <= 2, no flat
-  // runs -- a plateau extremum sits at the run's midpoint, not at its flagged
-  // first sample) the reference's binary search returns (number of knots at
-  // or left of t) - 1, clamped to [0, n-2].  Otherwise run the search.
-  const bool fast = NB <= 2 && !e.trig;
-  const int nch = (N + 31) >> 5;
-  // chunk c = (tid>>5) + 4j is scanned by warp wc(c); its rank offset is woff[wc] + pre[c]
-  // mirrored knots of both envelopes, for the O(1) segment count (nbsym <= 2)
-  constexpr real kInf = __builtin_huge_val();
-  const real l00 = sv0.nl > 0 ? sv0.x[0] : kInf, l01 = sv0.nl > 1 ? sv0.x[1] : kInf;
-  const real l10 = sv1.nl > 0 ? sv1.x[0] : kInf, l11 = sv1.nl > 1 ? sv1.x[1] : kInf;
-  const int nr0 = sv0.n - sv0.nl - sv0.nt, nr1 = sv1.n - sv1.nl - sv1.nt;
-  const real r00 = nr0 > 0 ? sv0.x[sv0.nl + sv0.nt] : kInf, r01 = nr0 > 1 ? sv0.x[sv0.nl + sv0.nt + 1] : kInf;
-  const real r10 = nr1 > 0 ? sv1.x[sv1.nl + sv1.nt] : kInf, r11 = nr1 > 1 ? sv1.x[sv1.nl + sv1.nt + 1] : kInf;
-  (void)nch;
-  const unsigned incl = lane == 31 ? kFull : ((2u << lane) - 1u);
-  // knot segment of sample i for both envelopes
-  auto segs = [&](int i, real t, int& lo0, int& lo1) {
-    lo0 = 0;
-    lo1 = 0;
-    if (fast) {
-      // knots at or left of t: mirrored ones compared directly, true ones
-      // counted from the scan's ballot masks (global chunk prefix + popc)
-      const int c = i >> 5;
-      int k0 = min((int)L.pmax[c] + __popc(L.mmax[c] & incl), sv0.nt);
-      int k1 = min((int)L.pmin[c] + __popc(L.mmin[c] & incl), sv1.nt);
-      k0 += (l00 <= t) + (l01 <= t) + (r00 <= t) + (r01 <= t);
-      k1 += (l10 <= t) + (l11 <= t) + (r10 <= t) + (r11 <= t);
-      lo0 = min(max(k0 - 1, 0), sv0.n - 2);
-      lo1 = min(max(k1 - 1, 0), sv1.n - 2);
-    } else {
-      if (sv0.n >= 4) lo0 = EMDB_SEARCH_RARE(sv0, t);
-      if (sv1.n >= 4) lo1 = EMDB_SEARCH_RARE(sv1, t);
-    }
-  };
+  const EnvEval<kInt> eval(L, K, sv0, sv1, NB, e.trig, lane);
   // T is strictly increasing, so the knot spans cover every sample iff they
   // cover the first and the last one
   if (N > 0) {
     const real t0 = T(0), tN = T(N - 1);
-    oor = (t0 < sv0.x[0]) || (tN > sv0.x[sv0.n - 1]) || (t0 < sv1.x[0]) || (tN > sv1.x[sv1.n - 1]);
+    oor = (t0 < sv0.xy[0].x) || (tN > sv0.xy[sv0.n - 1].x) || (t0 < sv1.xy[0].x) ||
+          (tN > sv1.xy[sv1.n - 1].x);
   }
-  // two samples per trip (i, i+NT): independent evaluation chains overlap;
-  // each lane still accumulates its samples in increasing order
-  for (int i = tid; i < N; i += (1 + EMDB_EVAL_PAIR) * NT) {
-    const int i2 = i + NT;
-    const bool has2 = EMDB_EVAL_PAIR && i2 < N;
-    const real t = T(i);
-    const real t2 = has2 ? T(i2) : t;
-    int lo0, lo1, lo0b, lo1b;
-    segs(i, t, lo0, lo1);
-    if (has2) segs(i2, t2, lo0b, lo1b); else { lo0b = lo0; lo1b = lo1; }
-#if EMDB_FAST_DIV
-    bool slow = false;
-    real emax, emin, emax2 = 0.0, emin2 = 0.0;
-#if !EMDB_F32
-    // (the FP32 build has no integer-axis shortcut: a float quotient formed
-    // in double from the table's RN(1/h) would be rounded twice)
-    if (kInt) {
-      emax = eval_seg_int(sv0, t, lo0, slow, fast);
-      emin = eval_seg_int(sv1, t, lo1, slow, fast);
-      if (has2) {
-        emax2 = eval_seg_int(sv0, t2, lo0b, slow, fast);
-        emin2 = eval_seg_int(sv1, t2, lo1b, slow, fast);
-      }
-    } else
-#endif
-    {
-      emax = eval_seg_q(sv0, t, lo0, slow);
-      emin = eval_seg_q(sv1, t, lo1, slow);
-      if (has2) {
-        emax2 = eval_seg_q(sv0, t2, lo0b, slow);
-        emin2 = eval_seg_q(sv1, t2, lo1b, slow);
-      }
-    }
-    if (slow) {
-      emax = EMDB_EVAL_RARE(sv0, t, lo0);
-      emin = EMDB_EVAL_RARE(sv1, t, lo1);
-      emax2 = EMDB_EVAL_RARE(sv0, t2, lo0b);
-      emin2 = EMDB_EVAL_RARE(sv1, t2, lo1b);
-    }
-#else
-    const real emax = eval_seg(sv0, t, lo0);
-    const real emin = eval_seg(sv1, t, lo1);
-    const real emax2 = eval_seg(sv0, t2, lo0b);
-    const real emin2 = eval_seg(sv1, t2, lo1b);
-#endif
-    if (kWide) {
-      // the update, and accumulate()'s quotient from the same operands
-      const real old = oldv[i];
-      const real mean = 0.5 * (emax + emin);
-      const real nw = old - mean;
-      imf[i] = nw;
-      qbuf[i] = (nw - old) / nw;
-      continue;
-    }
-    {
-      const real mean = 0.5 * (emax + emin);
-      const real old = oldv[i];
-      const real nw = old - mean;
-      imf[i] = nw;
-      accumulate(ps, old, nw);
-    }
-    if (has2) {
-      const real mean = 0.5 * (emax2 + emin2);
-      const real old = oldv[i2];
-      const real nw = old - mean;
-      imf[i2] = nw;
-      accumulate(ps, old, nw);
+  real ti = kInt ? (real)tid : real(0);
+#pragma unroll 1
+  for (int i = tid; i < N; i += NT) {
+    const real t = kInt ? ti : T(i);
+    ti += (real)NT;
+    const real old = oldv[i];
+    real emax, emin;
+    eval(L, i, t, emax, emin);
+    const real mean = 0.5 * (emax + emin);
+    const real nw = old - mean;
+    imf[i] = nw;
+    if (sums) {
+      // the wide instances sum per reference lane after the update
+      if (kWide) qbuf[i] = (nw - old) / nw;
+      else accumulate(ps, old, nw);
     }
   }
   // per-lane partial sums, then the reference's 128-lane trees on warp 0
@@ -1602,7 +1541,7 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
   if constexpr (kWide && !EMDB_WIDE_OVERLAP) {
     __syncthreads();
     EMDB_PH(&C, 5);
-    wide_lane_sums<NT>(red, oldv, imf, qbuf, N, tid);
+    if (sums) wide_lane_sums<NT>(red, oldv, imf, qbuf, N, tid);
   } else if (kWide) {
     // the reference's 128 lanes, each summing its samples in increasing order;
     // meanwhile the other warps run the next pass's extrema count on the
@@ -1625,7 +1564,7 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
     }
     if (EMDB_WIDE_OVERLAP && tid == 0) C.chunk_bad = 0;
   }
-  if (!kWide || (EMDB_WIDE_OVERLAP && tid < kThreads)) {
+  if (sums && (!kWide || (EMDB_WIDE_OVERLAP && tid < kThreads))) {
     red[tid] = ps.sq; red[128 + tid] = ps.dsq; red[256 + tid] = ps.osq;
     red[384 + tid] = ps.std_; red[512 + tid] = ps.omax; red[640 + tid] = ps.omin;
   }
@@ -1634,7 +1573,7 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
 #if EMDB_TREE_SPLIT
   // the six trees spread over the warps (warp w: sum w; warps 0/1 also the
   // max / min tree); the next extrema scan's barrier publishes C.sums
-  if (!kWide || warp < kWarps) {
+  if (sums && (!kWide || warp < kWarps)) {
     const real a = lane_tree(red + 128 * warp, lane, 0);
     if (lane == 0) C.sums[warp] = a;
     if (warp < 2) {
@@ -1738,7 +1677,7 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
     const real* S = p.values + off;
     real* out = p.imfs + (int64_t)MAXI * off;
     TimeAxis T;
-    T.arange = p.t_mode == kTArange;
+    T.arange = kInt;            // the launch picks the build by p.t_mode
     T.T = p.t_mode == kTShared ? p.T : (p.t_mode == kTPerTrace ? p.T + off : nullptr);
 
     if (fixed_bytes<NT, kGImf>(N) + kRedBytes + 64 > (size_t)p.arena_bytes ||
@@ -2040,7 +1979,9 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
 // reference scans with find_extrema_serial here; the extrema lists are the
 // same as the sift scan's (plateau rule included) and n_zer is not reported.
 // ---------------------------------------------------------------------------
-template <bool kSmem>
+// kInt: integer time axis (T = arange), with the sift's evaluation; any other
+// axis, which this entry point takes as it is given, is searched per sample.
+template <bool kSmem, bool kInt>
 __device__ __forceinline__ void envelope_pass(const SmemLayout& L, char* slab, const ExtInfo& e,
                                               int N, int NB, const TimeAxis& T, int tid, int warp,
                                               int lane, real* emax_out, real* emin_out,
@@ -2055,21 +1996,28 @@ __device__ __forceinline__ void envelope_pass(const SmemLayout& L, char* slab, c
   __syncthreads();
   const int kb0 = C.kbase[0], kb1 = C.kbase[1], kn0 = C.kcnt[0], kn1 = C.kcnt[1];
   solve_splines<kThreads>(K, kb0, kb1, kn0, kn1, tid);
-  SideView sv[2];
-  sv[0].x = K.X[0] + kb0; sv[0].y = K.Y[0] + kb0; sv[0].M = K.M[0]; sv[0].R = K.R[0]; sv[0].n = kn0;
-  sv[0].nl = NB - kb0; sv[0].nt = e.n_max;
-  sv[1].x = K.X[1] + kb1; sv[1].y = K.Y[1] + kb1; sv[1].M = K.M[1]; sv[1].R = K.R[1]; sv[1].n = kn1;
-  sv[1].nl = NB - kb1; sv[1].nt = e.n_min;
+  const SideView sv[2] = {{K.XY[0] + kb0, K.M[0], kn0, NB - kb0, e.n_max},
+                          {K.XY[1] + kb1, K.M[1], kn1, NB - kb1, e.n_min}};
   nk[0] = kn0;
   nk[1] = kn1;
   const int kcnt[2] = {kn0, kn1};
   bool oor = false;
+  const EnvEval<kInt> eval(L, K, sv[0], sv[1], NB, e.trig, lane);
+#pragma unroll 1
   for (int i = tid; i < N; i += kThreads) {
     real t = T(i);
+    if (kInt) {
+      // arange: the knot span covers every sample (see the mirroring)
+      real a, c;
+      eval(L, i, t, a, c);
+      emax_out[i] = a;
+      emin_out[i] = c;
+      continue;
+    }
     int lo0 = sv[0].n >= 4 ? search_seg(sv[0], t) : 0;
     int lo1 = sv[1].n >= 4 ? search_seg(sv[1], t) : 0;
-    bool r0 = !(t < sv[0].x[0] || t > sv[0].x[sv[0].n - 1]);
-    bool r1 = !(t < sv[1].x[0] || t > sv[1].x[sv[1].n - 1]);
+    bool r0 = !(t < sv[0].xy[0].x || t > sv[0].xy[sv[0].n - 1].x);
+    bool r1 = !(t < sv[1].xy[0].x || t > sv[1].xy[sv[1].n - 1].x);
     real a = eval_seg(sv[0], t, lo0);
     real c = eval_seg(sv[1], t, lo1);
     emax_out[i] = r0 ? a : 0.0;
@@ -2079,11 +2027,12 @@ __device__ __forceinline__ void envelope_pass(const SmemLayout& L, char* slab, c
   if (oor) atomicOr(status, kStatusStaleEnvelope);
   for (int q = 0; q < 2; ++q)
     for (int k = tid; k < mbuf; k += kThreads) {
-      kp[q][k] = k < kcnt[q] ? sv[q].x[k] : 0.0;
-      kv[q][k] = k < kcnt[q] ? sv[q].y[k] : 0.0;
+      kp[q][k] = k < kcnt[q] ? sv[q].xy[k].x : 0.0;
+      kv[q][k] = k < kcnt[q] ? sv[q].xy[k].y : 0.0;
     }
 }
 
+template <bool kInt>
 __global__ void __launch_bounds__(kThreads, 4) emd_envelope_kernel(EnvParams p) {
   extern __shared__ __align__(16) char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -2103,7 +2052,7 @@ __global__ void __launch_bounds__(kThreads, 4) emd_envelope_kernel(EnvParams p) 
     real* kp[2] = {p.max_kpos + (int64_t)b * p.mbuf, p.min_kpos + (int64_t)b * p.mbuf};
     real* kv[2] = {p.max_kval + (int64_t)b * p.mbuf, p.min_kval + (int64_t)b * p.mbuf};
     TimeAxis T;
-    T.arange = p.t_mode == kTArange;
+    T.arange = kInt;
     T.T = p.t_mode == kTShared ? p.T : (p.t_mode == kTPerTrace ? p.T + off : nullptr);
     if (fixed_bytes(N) + kRedBytes + 64 > (size_t)p.arena_bytes) {
       if (tid == 0) {
@@ -2124,10 +2073,10 @@ __global__ void __launch_bounds__(kThreads, 4) emd_envelope_kernel(EnvParams p) 
     if (!degenerate) {
       const int kc0 = e.n_max + 2 * NB + 2, kc1 = e.n_min + 2 * NB + 2;
       if (knot_bytes(kc0, kc1) <= (size_t)L.arena_bytes)
-        envelope_pass<true>(L, slab, e, N, NB, T, tid, warp, lane, emax_out, emin_out, kp, kv,
+        envelope_pass<true, kInt>(L, slab, e, N, NB, T, tid, warp, lane, emax_out, emin_out, kp, kv,
                             p.mbuf, nk, p.status);
       else
-        envelope_pass<false>(L, slab, e, N, NB, T, tid, warp, lane, emax_out, emin_out, kp, kv,
+        envelope_pass<false, kInt>(L, slab, e, N, NB, T, tid, warp, lane, emax_out, emin_out, kp, kv,
                              p.mbuf, nk, p.status);
     } else {
       for (int i = tid; i < N; i += kThreads) { emax_out[i] = 0.0; emin_out[i] = 0.0; }
@@ -2218,7 +2167,10 @@ __global__ void div_check_kernel(int mode, long long n, unsigned long long seed,
       if (h2 & 2) b = -b;
       if (__double_as_longlong(div_rn(a, b, 1.0 / b)) != __double_as_longlong(a / b)) ++bad0;
       // division by 6 (the spline term's divisor)
-      if (__double_as_longlong(div_rn(a, 6.0, kInv6)) != __double_as_longlong(a / 6.0)) ++bad1;
+      bool slow = false;
+      double q6 = div6(a, slow);
+      if (slow) q6 = div_slow(a, 6.0);
+      if (__double_as_longlong(q6) != __double_as_longlong(a / 6.0)) ++bad1;
       // segment quotients: 0 <= a <= b, b a spacing in [1, 65536] with a random fraction
       double bi = (double)((h2 >> 40) % 65536 + 1) + (double)((h2 >> 8) & 0xffff) * 0x1p-16;
       double ai = bi * ((double)((h1 >> 11) & 0xfffffffffffffull) * 0x1p-52);
@@ -2335,7 +2287,7 @@ int sift_pass_placement(int N, int arena_total, size_t slab_stride, int kc0, int
 size_t sift_slab_bytes(int max_extrema, int nbsym) {
   const long long kc = (long long)max_extrema + 2LL * nbsym + 2;
   const size_t cap = (size_t)(2 * kc);
-  const size_t red_extra = (EMDB_FAST_DIV != 1 && 4 * cap >= (size_t)kRedDoubles) ? 0 : kRedBytes;
+  const size_t red_extra = (4 * cap >= (size_t)kRedDoubles) ? 0 : kRedBytes;
   return align16(10 * cap * sizeof(real) + red_extra);
 }
 
@@ -2414,20 +2366,37 @@ cudaError_t launch_sift(const SiftParams& p, int grid, cudaStream_t stream) {
   }
 }
 
-cudaError_t envelope_occupancy(int arena_bytes, int* ctas_per_sm) {
-  cudaError_t e = cudaFuncSetAttribute(emd_envelope_kernel,
+namespace {
+template <bool kInt>
+cudaError_t envelope_occupancy_t(int arena_bytes, int* ctas_per_sm) {
+  cudaError_t e = cudaFuncSetAttribute(emd_envelope_kernel<kInt>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, arena_bytes);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, emd_envelope_kernel, kThreads,
-                                                       arena_bytes);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, emd_envelope_kernel<kInt>,
+                                                       kThreads, arena_bytes);
+}
+template <bool kInt>
+cudaError_t launch_envelope_t(const EnvParams& p, int grid, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(emd_envelope_kernel<kInt>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, p.arena_bytes);
+  if (e != cudaSuccess) return e;
+  emd_envelope_kernel<kInt><<<grid, kThreads, p.arena_bytes, stream>>>(p);
+  return cudaGetLastError();
+}
+}  // namespace
+
+// CTAs per SM that both builds reach
+cudaError_t envelope_occupancy(int arena_bytes, int* ctas_per_sm) {
+  int a = 0, b = 0;
+  cudaError_t e = envelope_occupancy_t<true>(arena_bytes, &a);
+  if (e == cudaSuccess) e = envelope_occupancy_t<false>(arena_bytes, &b);
+  *ctas_per_sm = a < b ? a : b;
+  return e;
 }
 
 cudaError_t launch_envelope(const EnvParams& p, int grid, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(emd_envelope_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, p.arena_bytes);
-  if (e != cudaSuccess) return e;
-  emd_envelope_kernel<<<grid, kThreads, p.arena_bytes, stream>>>(p);
-  return cudaGetLastError();
+  return p.t_mode == kTArange ? launch_envelope_t<true>(p, grid, stream)
+                              : launch_envelope_t<false>(p, grid, stream);
 }
 
 }  // namespace emdb
