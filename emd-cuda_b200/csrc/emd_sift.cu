@@ -45,7 +45,6 @@
 #include "emdb_internal.cuh"
 
 // Tuning knobs (compile-time; results are identical for every setting):
-//  EMDB_PCR_PAIR   update two PCR rows per loop trip
 //  EMDB_OUTLINE    rarely taken paths as calls instead of inline copies:
 //                  1 the general evaluation and the binary segment search,
 //                  2 also the IEEE-division fallbacks of the PCR and setup rows
@@ -57,26 +56,9 @@
 // 1/1 208.4k signals/s, 1/0 188.1k, 2/1 195.6k, 0/0 184.9k (and 0/1 172.7k on
 // another box against 208.2k for 1/1): less sift-pass code relieves
 // instruction supply, the dominant stall after FP64 latency.
-//  EMDB_PCR_NB     branch-free division with no reciprocal at hand (div_nb)
-//                  for the two PCR quotients of each row: 241.1k vs 222.8k
-//                  signals/s on one B200.  Used everywhere (evaluation and
-//                  stop-test quotients too) it ran slower, 160k vs 180k: there
-//                  the extra instructions outweigh the overlap.
-//  EMDB_ACC_NB / EMDB_SETUP_NB  the same division for the stop-test quotient
-//                  diff/new and the spline rows' slopes: 231.0k / 236.7k vs
-//                  240.9k signals/s, so off.
-//  EMDB_SETUP_TAB  on the integer time axis, the spline rows' slopes from the
-//                  reciprocal table and div_q: 238.0k vs 241.2k, so off.
 //  EMDB_SCAN_UNROLL / EMDB_FILL_UNROLL  unroll factors of the extrema scan
 //                  and knot fill loops: 4 measured 231.8k / 226.3k vs 240.2k
 //                  at 2.
-#ifndef EMDB_PCR_PAIR
-#define EMDB_PCR_PAIR 0
-#endif
-//  EMDB_WIDE_PCR_PAIR  the same for the wide (256 / 512-thread) instances
-#ifndef EMDB_WIDE_PCR_PAIR
-#define EMDB_WIDE_PCR_PAIR 0
-#endif
 //  EMDB_WIDE_OVERLAP  wide instances: the warps past the 128 reduction lanes
 //                  run the post-update extrema scan while the lanes sum the
 //                  stop-test terms (the scan then has NT/32 - 4 slots).
@@ -84,7 +66,6 @@
 //                  1024 x 8192 seismic 291.2 vs 292.3 ms, 2048 x 4096 50.9 vs
 //                  51.6 ms; 256 threads, 2048 x 4096 50.4 vs 46.4 ms (its
 //                  knot fill then has 4 warps of 8) -- so off.
-//  EMDB_WIDE_PCR_PAIR 1: 291.1 / 51.2 ms, no gain.
 #ifndef EMDB_WIDE_OVERLAP
 #define EMDB_WIDE_OVERLAP 0
 #endif
@@ -105,18 +86,6 @@
 #endif
 #ifndef EMDB_TREE_SPLIT
 #define EMDB_TREE_SPLIT 1
-#endif
-#ifndef EMDB_PCR_NB
-#define EMDB_PCR_NB 1
-#endif
-#ifndef EMDB_ACC_NB
-#define EMDB_ACC_NB 0
-#endif
-#ifndef EMDB_SETUP_NB
-#define EMDB_SETUP_NB 0
-#endif
-#ifndef EMDB_SETUP_TAB
-#define EMDB_SETUP_TAB 0
 #endif
 #ifndef EMDB_SCAN_UNROLL
 #define EMDB_SCAN_UNROLL 2
@@ -153,24 +122,16 @@ constexpr int kPhases = 10;
 // the sift computes is a `real`; the reference kernel's double literals keep
 // their C++ meaning, so float expressions that mix them are evaluated in
 // double and rounded once, as in the reference source compiled with REAL_T =
-// float.  The FP64 build's division shortcuts (reciprocal tables, Markstein
-// and branch-free quotients) are off: float quotients are the IEEE ones, and
-// the one double quotient per envelope sample (the reference's "/ 6.0")
+// float.  The FP64 build's branch-free quotients have float counterparts
+// (div_q from an IEEE reciprocal for the segment quotients, div_nb for the PCR
+// rows), self-tested against the float division by emdb_check_division modes 3
+// and 4; the one double quotient per envelope sample (the reference's "/ 6.0")
 // is formed from RN(1/6) and its residual (div6), which equals the double
 // division.
 #ifndef EMDB_F32
 #define EMDB_F32 0
 #endif
 #if EMDB_F32
-//  EMDB_F32_FAST  the float counterparts of the FP64 build's branch-free
-//                  quotients (div_q from an IEEE reciprocal for the segment
-//                  quotients, div_nb for the PCR rows), self-tested against
-//                  the float division by emdb_check_division modes 3 and 4
-#ifndef EMDB_F32_FAST
-#define EMDB_F32_FAST 1
-#endif
-#undef EMDB_PCR_NB
-#define EMDB_PCR_NB EMDB_F32_FAST
 namespace emdb::f32 {
 using real = float;
 #else
@@ -205,7 +166,7 @@ struct Ctl {
   int head[2][kMaxNbsym + 1];  // first NB+1 extrema indices per side (0 = max, 1 = min)
   int tail[2][kMaxNbsym + 1];  // tail[q][k] = index of extremum n_q-1-k
   int mlist[4][kMaxNbsym + 1]; // mirrored index lists: lmax, lmin, rmax, rmin
-  int mcnt[4];
+  int mcnt[4];                 // entries per list; [0], [1] hold a range during the solve
   int lsym, rsym;
   int kbase[2], kcnt[2];
   int dbg_n[kMaxImfsCap], dbg_e[kMaxImfsCap], dbg_z[kMaxImfsCap];
@@ -287,15 +248,20 @@ __device__ __forceinline__ SmemLayout carve(char* base, int N, int arena_total,
   return L;
 }
 
-// Knot / PCR storage for one sift pass (both envelopes).  After the last PCR
-// level only the b and d arrays of the final buffers are read, so the spline
-// moments M go into buffer 0's a (upper envelope) and c (lower) arrays.
+// Knot / PCR storage for one sift pass (both envelopes).  A PCR buffer holds
+// each row's off-diagonals as (a, c) pairs, then its (b, d) pairs, one 16-byte
+// word each.  The spline moments M take the place of buffer 0's (a, c) pairs,
+// which nothing reads any more by then.
 struct Knots {
   real2* XY[2]; // (position, value) of each knot
   real* M[2];
-  real* P[2];   // ping-pong PCR buffers: a | b | c | d, each `cap` rows
+  real* P[2];   // ping-pong PCR buffers: (a, c) | (b, d), each `cap` rows
   real* red;    // reduction lanes after the solve: buffer 1, or just past it
   int cap;
+  __device__ __forceinline__ real2* ac(int q) const { return reinterpret_cast<real2*>(P[q]); }
+  __device__ __forceinline__ real2* bd(int q) const {
+    return reinterpret_cast<real2*>(P[q] + 2 * cap);
+  }
 };
 
 __host__ __device__ inline size_t knot_bytes(int kc0, int kc1) {
@@ -315,7 +281,7 @@ __device__ __forceinline__ Knots place_knots(char* base, int kc0, int kc1) {
   K.P[0] = p; p += 4 * K.cap;
   K.P[1] = p;
   K.M[0] = K.P[0];
-  K.M[1] = K.P[0] + 2 * K.cap;
+  K.M[1] = K.P[0] + kc0;
   K.red = (4 * K.cap >= kRedDoubles) ? K.P[1] : K.P[1] + 4 * K.cap;
   return K;
 }
@@ -339,7 +305,7 @@ __device__ __forceinline__ Knots place_knots_split(char* sbase, int sbytes, char
   K.P[0] = p; p += 4 * K.cap;
   K.P[1] = reinterpret_cast<real*>(gbase);
   K.M[0] = K.P[0];
-  K.M[1] = K.P[0] + 2 * K.cap;
+  K.M[1] = K.P[0] + kc0;
   // reduction lanes: shared memory past buffer 0 when they fit, else the slab
   // (buffer 1 is dead after the solve; the slab holds knot_bytes of the largest pass)
   if (split_bytes(kc0, kc1) + kRedBytes <= (size_t)sbytes) K.red = p;
@@ -375,7 +341,7 @@ __device__ __forceinline__ Knots place_knots_borrow(real* imf, char* arena, int 
   K.P[0] = p;
   K.P[1] = imf;
   K.M[0] = K.P[0];
-  K.M[1] = K.P[0] + 2 * K.cap;
+  K.M[1] = K.P[0] + kc0;
   K.red = reinterpret_cast<real*>(slab + align16((size_t)N * sizeof(real)));
   return K;
 }
@@ -439,7 +405,7 @@ __device__ __forceinline__ Knots place_knots_park(real* imf, char* slab, int N, 
   K.P[0] = p;
   K.P[1] = imf;
   K.M[0] = K.P[0];
-  K.M[1] = K.P[0] + 2 * K.cap;
+  K.M[1] = K.P[0] + kc0;
   K.red = red;
   return K;
 }
@@ -560,38 +526,58 @@ __device__ __forceinline__ double div_q(double a, double b, double y, bool& slow
   return zero ? q0 : q2;
 }
 
-#if EMDB_PCR_NB || EMDB_ACC_NB || EMDB_SETUP_NB
-// Branch-free RN(a/b) with no reciprocal at hand (FMA division schemes in
-// Muller et al., "Handbook of Floating-Point Arithmetic", 2nd ed., ch. 4.9 /
-// 5.3): y ~ 1/b from the PTX approximate reciprocal and two Newton steps;
-// q1 = q0 + (a - b*q0)*y is a faithful rounding of a/b; the exact remainders
-// of q1 and of its neighbour towards a/b pick the nearer one (a quotient of
-// two 53-bit numbers is never an exact midpoint).  `slow` is set outside the
-// ranges where every step is exact: |a|, |q| in (2^-900, 2^900), |b| in
-// (2^-1000, 2^1000); zero numerators only with such a b.
+#if !EMDB_F32
+// Branch-free RN(a/b) with no reciprocal at hand (FMA division schemes of
+// Markstein, IBM J. Res. Dev. 1990, and Muller et al., "Handbook of
+// Floating-Point Arithmetic", 2nd ed., ch. 4.7): y from the PTX approximate
+// reciprocal, one cubic step (1/b = y(1 + e + e^2 + ...), e = 1 - by) and one
+// linear one, whose argument is within 2^-104 of 1/b before its rounding, so y
+// is within (1/2 + 2^-51) ulp of it; q1 = RN(q0 + (a - b q0) y) is then within
+// (1/2 + 2^-50) ulp of a/b, its remainder r = a - b q1 exact, and q1 + r y
+// differs from a/b by at most |r/b| times y's relative error, below
+// 2^-55 m_b ulp(q) (m_b in [1, 2) the significand of b; the 2^-51 adds nothing
+// that matters: for m_b = 2 - 2^-52 y's error is at most half an ulp of 1/b
+// to within 2^-53).  A quotient of 53-bit numbers is never closer than
+// 2^-53 / m_b ulp(q) to a rounding boundary without lying on it, and never
+// lies on it, so the last FMA rounds as the division does.
+//
+// `slow` is set unless |a|, |b| and |q| are in [2^-511, 2^512), where no step
+// underflows or overflows: exponent fields 512..1535 are those whose two top
+// bits differ, i.e. whose high word plus 2^29 has bit 30 set.  A zero
+// numerator gives q0 = a*y, the correctly signed zero, and needs only b.
+// 10 FP64 operations and integer checks; the form before it (two linear
+// steps, a neighbour choice by two exact remainders and range compares on the
+// doubles) took 8 and 11 compares, which cost as much as arithmetic.
+__device__ __forceinline__ unsigned range_bits(double x) {
+  return (unsigned)__double2hiint(x) + 0x20000000u;
+}
 __device__ __forceinline__ double div_nb(double a, double b, bool& slow) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
   double e = fma(-b, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-b, y, 1.0);
-  y = fma(y, e, y);
+  e = fma(e, e, e);
+  y = fma(e, y, y);
   const double q0 = a * y;
+  e = fma(-b, y, 1.0);
+  y = fma(e, y, y);
   const double r0 = fma(-q0, b, a);
   const double q1 = fma(r0, y, q0);
   const double r1 = fma(-q1, b, a);
-  const bool up = (r1 > 0.0) == (b > 0.0);
-  const long long step = (up == (q1 > 0.0)) ? 1 : -1;
-  const double qn = __longlong_as_double(__double_as_longlong(q1) + step);
-  const double rn = fma(-qn, b, a);
-  const double q = fabs(rn) < fabs(r1) ? qn : q1;
-  const double aa = fabs(a), qa = fabs(q1), ba = fabs(b);
-  const bool bok = ba > 0x1p-1000 && ba < 0x1p+1000;
+  const double q2 = fma(r1, y, q1);
   const bool zero = a == 0.0;
-  slow |= !bok || (!zero && !(aa > 0x1p-900 && aa < 0x1p+900 && qa > 0x1p-900 && qa < 0x1p+900));
-  return zero ? q0 : q;
+  const unsigned aq = range_bits(a) & range_bits(q2);
+  slow |= !(range_bits(b) & (zero ? 0x40000000u : aq) & 0x40000000u);
+  return zero ? q0 : q2;
 }
 #endif
+// high word of |x|: orders magnitudes, and (as a fixed-point number with 20
+// fraction bits) is within 0.0861 below log2|x| plus the exponent bias
+__device__ __forceinline__ unsigned mag(double x) {
+  return (unsigned)__double2hiint(x) & 0x7fffffffu;
+}
+__device__ __forceinline__ unsigned mag(float x) {
+  return (unsigned)__float_as_int(x) & 0x7fffffffu;
+}
 
 #if !EMDB_F32
 __device__ __forceinline__ double div_rn(double a, double b, double y) {
@@ -1006,12 +992,6 @@ struct PairY {
   __device__ __forceinline__ real operator[](int i) const { return p[i].y; }
 };
 
-// kInt: integer time axis (T = arange), where knot spacings are integers and
-// the interior rows' slope quotients take RN(1/h) from the table and the exact
-// two-step Markstein quotient (div_q) instead of two divisions; spacings
-// outside the table (or not positive integers, as unsorted knot lists can
-// give) take the divisions.
-template <bool kInt = false>
 __device__ __forceinline__ void setup_row(const real2* xy, int n, int k, int m,
                                           real& a, real& b, real& c, real& d) {
   const PairX x{xy};
@@ -1028,135 +1008,196 @@ __device__ __forceinline__ void setup_row(const real2* xy, int n, int k, int m,
     int i = k + 1;
     real h_im1 = x[i] - x[i - 1], h_i = x[i + 1] - x[i];
     a = h_im1; b = 2.0 * (h_im1 + h_i); c = h_i;
-#if EMDB_SETUP_NB
-    bool slow = false;
-    const real sr = div_nb(y[i + 1] - y[i], h_i, slow);
-    const real sl = div_nb(y[i] - y[i - 1], h_im1, slow);
-    d = slow ? 6.0 * ((y[i + 1] - y[i]) / h_i - (y[i] - y[i - 1]) / h_im1) : 6.0 * (sr - sl);
-#else
-    if (kInt) {
-      const bool ok = h_i >= 1.0 && h_i <= (real)kRcpTab && h_im1 >= 1.0 &&
-                      h_im1 <= (real)kRcpTab;
-      const int ji = ok ? (int)h_i : 1, jm = ok ? (int)h_im1 : 1;
-      bool slow = !ok || (real)ji != h_i || (real)jm != h_im1;
-      const real sr = div_q(y[i + 1] - y[i], h_i, g_rcp.v[ji], slow);
-      const real sl = div_q(y[i] - y[i - 1], h_im1, g_rcp.v[jm], slow);
-      d = slow ? 6.0 * (EMDB_DIV_RARE(y[i + 1] - y[i], h_i) - EMDB_DIV_RARE(y[i] - y[i - 1], h_im1))
-               : 6.0 * (sr - sl);
-    } else {
-      d = 6.0 * ((y[i + 1] - y[i]) / h_i - (y[i] - y[i - 1]) / h_im1);
-    }
-#endif
+    d = 6.0 * ((y[i + 1] - y[i]) / h_i - (y[i] - y[i - 1]) / h_im1);
   }
 }
 
-__device__ __forceinline__ void pcr_row(const real* __restrict__ Pa, real* __restrict__ Pn,
-                                        int cap, int r, int k, int s, int mq) {
-  const bool hl = k - s >= 0, hr = k + s < mq;
-  const int rl = r - s, rr = r + s;
-  const real ak = Pa[r], bk = Pa[cap + r], ck = Pa[2 * cap + r], dk = Pa[3 * cap + r];
-  const real b_left = hl ? Pa[cap + rl] : 1.0;
-  const real b_right = hr ? Pa[cap + rr] : 1.0;
-#if EMDB_PCR_NB
+// One PCR row update (kernels.py:651-668), in the reference's operation order;
+// returns the larger magnitude word of its two multipliers.
+__device__ __forceinline__ unsigned pcr_row(const real2* __restrict__ ac,
+                                            const real2* __restrict__ bd,
+                                            real2* __restrict__ acn, real2* __restrict__ bdn,
+                                            int r, int k, int s, int mq) {
+  const bool hl = k >= s, hr = k + s < mq;
+  const real2 zero{real(0), real(0)}, one{real(1), real(0)};
+  const real2 o = ac[r], p = bd[r];
+  const real2 pl = hl ? bd[r - s] : one, pr = hr ? bd[r + s] : one;
+  const real2 ol = hl ? ac[r - s] : zero, orr = hr ? ac[r + s] : zero;
   bool sl = false, sr = false;
-  const real ql = div_nb(ak, b_left, sl);
-  const real qr = div_nb(ck, b_right, sr);
-  real alpha = hl ? ql : 0.0;
-  real beta = hr ? qr : 0.0;
+  const real ql = div_nb(o.x, pl.x, sl);
+  const real qr = div_nb(o.y, pr.x, sr);
+  real alpha = hl ? ql : real(0);
+  real beta = hr ? qr : real(0);
   if ((hl && sl) || (hr && sr)) {
-    alpha = hl ? EMDB_DIV_RARE(ak, b_left) : 0.0;
-    beta = hr ? EMDB_DIV_RARE(ck, b_right) : 0.0;
+    alpha = hl ? EMDB_DIV_RARE(o.x, pl.x) : real(0);
+    beta = hr ? EMDB_DIV_RARE(o.y, pr.x) : real(0);
   }
-#else
-  const real alpha = hl ? ak / b_left : 0.0;
-  const real beta = hr ? ck / b_right : 0.0;
-#endif
-  const real a_left = hl ? Pa[rl] : 0.0;
-  const real c_left = hl ? Pa[2 * cap + rl] : 0.0;
-  const real d_left = hl ? Pa[3 * cap + rl] : 0.0;
-  const real a_right = hr ? Pa[rr] : 0.0;
-  const real c_right = hr ? Pa[2 * cap + rr] : 0.0;
-  const real d_right = hr ? Pa[3 * cap + rr] : 0.0;
-  Pn[r] = -alpha * a_left;
-  Pn[2 * cap + r] = -beta * c_right;
-  Pn[cap + r] = bk - alpha * c_left - beta * a_right;
-  Pn[3 * cap + r] = dk - alpha * d_left - beta * d_right;
+  acn[r] = real2{-alpha * ol.x, -beta * orr.y};
+  bdn[r] = real2{p.x - alpha * ol.y - beta * orr.x, p.y - alpha * pl.y - beta * pr.y};
+  return max(mag(alpha), mag(beta));
 }
 
-template <int NT, bool kInt = false>
+// The last PCR level of a system whose multipliers have died out (see
+// solve_splines), for row k (index r): the right-hand side after it, d.  The
+// diagonal stays as it is.  A neighbour's term is formed only where it can
+// reach the rounding of d: RN(d - x) = d for |x| below a quarter ulp, and the
+// magnitude words bound |a d_l| against |d b_l| from both sides (each is at
+// most 0.0861 below its logarithm).
+__device__ __forceinline__ real pcr_last(const real2* ac, const real2* bd, int r, int k, int s,
+                                         int mq) {
+  constexpr int kFrac = sizeof(real) == 8 ? 20 : 23;
+  constexpr int kGap = ((sizeof(real) == 8 ? 55 : 26) << kFrac) + (1 << kFrac) / 4;
+  const real2 o = ac[r];
+  const bool hl = k >= s, hr = k + s < mq;
+  const real2 pl = hl ? bd[r - s] : real2{real(1), real(0)};
+  const real2 pr = hr ? bd[r + s] : real2{real(1), real(0)};
+  real d = bd[r].y;
+  const int dm = (int)mag(d);
+  const bool l = hl && dm - (int)mag(o.x) <= (int)mag(pl.y) - (int)mag(pl.x) + kGap;
+  const bool rr = hr && dm - (int)mag(o.y) <= (int)mag(pr.y) - (int)mag(pr.x) + kGap;
+  if (l) d -= EMDB_DIV_RARE(o.x, pl.x) * pl.y;
+  if (rr) d -= EMDB_DIV_RARE(o.y, pr.x) * pr.y;
+  return d;
+}
+
+// Spline rows, parallel cyclic reduction and the moments of both envelopes
+// (kernels.py:607-697), every row rounded as the reference rounds it.
+//
+// The reference halves the coupling until the stride passes the system,
+// ceil(log2 m) levels.  The multipliers square from level to level (1/4, 1/14,
+// 1/194, 2^-15, 2^-30, 2^-61 on equal spacing; at most 1/2, 1/7, 1/97, ... on
+// any), so from some level on no row changes any more, and those levels are
+// left out once that is certain.  With every multiplier of the fifth level
+// (stride 16) at most e <= 2^-26:
+//   * the sixth has multipliers a_k/b_l = -alpha_k alpha_l <= e^2 (1 + 2^-40)
+//     and the diagonal's changes, alpha_k beta_l b_k <= e^4 b_k, are far below
+//     its half ulp: b is final after the fifth level;
+//   * when the magnitudes of all d are within 2^46 of each other, the sixth
+//     level changes none of them by more than 2^-5 of itself, and from the
+//     seventh on, with multipliers of at most e^4 (1 + 2^-40), |alpha d_l| <
+//     2^-104 2^47 |d| is below the quarter ulp: d cannot change either.
+// (All magnitudes normal and finite, which the vote checks too.)
+// What is left after five levels is the sixth level's d, in which most terms
+// round away too (pcr_last), and the division by the diagonal, fused.  One
+// vote decides for both systems; systems for which it fails (and those of at
+// most 32 rows) run every level.
+// Bound by FP64 issue and latency: per row and level two quotients (20 FP64
+// operations) and 8 more, six 16-byte loads.  On 2048-sample seismic traces
+// the row-levels fall from 4.25 to 3.0 million per 24 traces, at 8192 samples
+// from 16.4 to 9.7; no pass of those needed a seventh level.  B200, all levels
+// with the former quotients / as here: 16,384 x 2048 seismic 84.8 / 72.7 ms,
+// 1,024 x 4096 64.0 / 41.1, 256 x 8192 89.0 / 66.9; envelopes alone, 4,096 x
+// 2048: 0.53 / 0.38 ms.
+template <int NT>
 __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kbase1, int kcnt0,
-                                              int kcnt1, int tid, Ctl* C = nullptr) {
+                                              int kcnt1, int tid, Ctl& C) {
   const int m0 = kcnt0 >= 4 ? kcnt0 - 2 : 0;
   const int m1 = kcnt1 >= 4 ? kcnt1 - 2 : 0;
   const int mt = m0 + m1;
-  const int cap = K.cap;
   const real2* xy0 = K.XY[0] + kbase0;
   const real2* xy1 = K.XY[1] + kbase1;
+  unsigned* const range = reinterpret_cast<unsigned*>(C.mcnt);   // free until the next mirroring
+  if (tid == 0) {
+    range[0] = 0u;
+    range[1] = 0xffffffffu;
+  }
+#pragma unroll 1
   for (int r = tid; r < mt; r += NT) {
     const bool s0 = r < m0;
     const int k = s0 ? r : r - m0;
     real a, b, c, d;
-    setup_row<kInt>(s0 ? xy0 : xy1, s0 ? kcnt0 : kcnt1, k, s0 ? m0 : m1, a, b, c, d);
-    real* P = K.P[0];
-    P[r] = a; P[cap + r] = b; P[2 * cap + r] = c; P[3 * cap + r] = d;
+    setup_row(s0 ? xy0 : xy1, s0 ? kcnt0 : kcnt1, k, s0 ? m0 : m1, a, b, c, d);
+    K.ac(0)[r] = real2{a, c};
+    K.bd(0)[r] = real2{b, d};
   }
   __syncthreads();
-  if (C) EMDB_PH(C, 2);
+  EMDB_PH(&C, 2);
+  constexpr int kLast = 32;                     // stride of the fused level
+  constexpr unsigned kSmall = (sizeof(real) == 8 ? (1023u - 26u) << 20 : (127u - 26u) << 23);
+  constexpr unsigned kNormal = sizeof(real) == 8 ? 1u << 20 : 1u << 23;
+  constexpr unsigned kRange = 46u * kNormal;
+  constexpr unsigned kInfMag = sizeof(real) == 8 ? 0x7ff00000u : 0x7f800000u;
   const int mmax = max(m0, m1);
   int cur = 0;
-  int fin0 = 0, fin1 = 0;
+  bool fused = false;
+#pragma unroll 1
   for (int s = 1; s < mmax; s *= 2) {
-    const real* __restrict__ Pa = cur ? K.P[1] : K.P[0];
-    real* __restrict__ Pn = cur ? K.P[0] : K.P[1];
-    // two rows per trip: independent division chains overlap
-    constexpr int kPair = NT > kThreads ? EMDB_WIDE_PCR_PAIR : EMDB_PCR_PAIR;
-    for (int r = tid; r < mt; r += (1 + kPair) * NT) {
-      const int r2 = kPair ? r + NT : mt;
-      {
-        const bool s0 = r < m0;
-        const int mq = s0 ? m0 : m1;
-        if (s < mq) pcr_row(Pa, Pn, cap, r, s0 ? r : r - m0, s, mq);
-      }
-      if (r2 < mt) {
-        const bool s0 = r2 < m0;
-        const int mq = s0 ? m0 : m1;
-        if (s < mq) pcr_row(Pa, Pn, cap, r2, s0 ? r2 : r2 - m0, s, mq);
+    // the level whose multipliers and right-hand sides are looked at
+    const bool vote = 2 * s == kLast && mmax > kLast;
+    unsigned mult = 0u, dmax = 0u, dmin = 0xffffffffu;
+#pragma unroll 1
+    for (int r = tid; r < mt; r += NT) {
+      const bool s0 = r < m0;
+      mult = max(mult, pcr_row(K.ac(cur), K.bd(cur), K.ac(cur ^ 1), K.bd(cur ^ 1), r,
+                               s0 ? r : r - m0, s, s0 ? m0 : m1));
+      if (vote) {
+        const real2 p = K.bd(cur ^ 1)[r];
+        dmax = max(dmax, mag(p.y));
+        dmin = min(dmin, mag(p.y));
+        if (mag(p.x) < kNormal) mult = 0xffffffffu;
       }
     }
-    if (s < m0) fin0 ^= 1;
-    if (s < m1) fin1 ^= 1;
     cur ^= 1;
-    // Rows are owned by thread r mod NT, so a level with stride >= NT reads
-    // and writes only the calling thread's rows: no barrier is needed before
-    // the next such level.  Earlier levels read other threads' rows, and the
-    // solve below does too, so those transitions keep the barrier.
-    if (s < NT || 2 * s >= mmax) __syncthreads();
+    if (vote) {
+      dmax = __reduce_max_sync(kFull, dmax);
+      dmin = __reduce_min_sync(kFull, dmin);
+      if ((tid & 31) == 0) {
+        atomicMax(range, dmax);
+        atomicMin(range + 1, dmin);
+      }
+      const int bad = __syncthreads_or(mult > kSmall);
+      const unsigned hi = range[0], lo = range[1];
+      if (!bad && hi < kInfMag && lo >= kNormal && hi - lo < kRange) {
+        fused = true;
+        break;
+      }
+    } else if (s < NT || 2 * s >= mmax) {
+      // Rows are owned by thread r mod NT, so a level with stride >= NT reads
+      // and writes only the calling thread's rows: no barrier is needed before
+      // the next such level.  Earlier levels read other threads' rows, and the
+      // solve below does too, so those transitions keep the barrier.
+      __syncthreads();
+    }
   }
-  if (C) EMDB_PH(C, 3);
+  EMDB_PH(&C, 3);
   // diagonal solve + end-moment recovery (M[0], M[n-1] by the owners of the end rows)
+  const real2* ac = K.ac(cur);
+  const real2* bd = K.bd(cur);
+  auto moment = [&](int r, int k, int mq) {
+    const real d = fused ? pcr_last(ac, bd, r, k, kLast, mq) : bd[r].y;
+    const real b = bd[r].x;
+    bool slow = false;
+    const real q = div_nb(d, b, slow);
+    return slow ? EMDB_DIV_RARE(d, b) : q;
+  };
+#pragma unroll 1
   for (int r = tid; r < mt; r += NT) {
     const bool s0 = r < m0;
     const int k = s0 ? r : r - m0;
     const int mq = s0 ? m0 : m1;
-    const int n = s0 ? kcnt0 : kcnt1;
-    const real* Pf = (s0 ? fin0 : fin1) ? K.P[1] : K.P[0];
-    real* M = s0 ? K.M[0] : K.M[1];
-    const PairX x{s0 ? xy0 : xy1};
-    real Mk1 = Pf[3 * cap + r] / Pf[cap + r];
-    M[k + 1] = Mk1;
-    if (k == 0) {
-      real M2 = Pf[3 * cap + r + 1] / Pf[cap + r + 1];
-      real h0 = x[1] - x[0], h1 = x[2] - x[1];
-      M[0] = ((h0 + h1) * Mk1 - h0 * M2) / h1;
-    }
-    if (k == mq - 1) {
-      real Mnm3 = Pf[3 * cap + r - 1] / Pf[cap + r - 1];
-      real hnm3 = x[n - 2] - x[n - 3], hnm2 = x[n - 1] - x[n - 2];
-      M[n - 1] = ((hnm3 + hnm2) * Mk1 - hnm2 * Mnm3) / hnm3;
+    const real Mk1 = moment(r, k, mq);
+    (s0 ? K.M[0] : K.M[1])[k + 1] = Mk1;
+  }
+  __syncthreads();
+  // end moments from the first and last two (the reference forms the same
+  // quotients d/b again)
+  if (tid < 4) {
+    const int q = tid >> 1;
+    const int n = q == 0 ? kcnt0 : kcnt1;
+    if (n >= 4) {
+      const PairX x{q == 0 ? xy0 : xy1};
+      real* M = q == 0 ? K.M[0] : K.M[1];
+      if ((tid & 1) == 0) {
+        const real h0 = x[1] - x[0], h1 = x[2] - x[1];
+        M[0] = ((h0 + h1) * M[1] - h0 * M[2]) / h1;
+      } else {
+        const real hnm3 = x[n - 2] - x[n - 3], hnm2 = x[n - 1] - x[n - 2];
+        M[n - 1] = ((hnm3 + hnm2) * M[n - 2] - hnm2 * M[n - 3]) / hnm3;
+      }
     }
   }
   __syncthreads();
-  if (C) EMDB_PH(C, 4);
+  EMDB_PH(&C, 4);
 }
 
 // One envelope's spline: knots, moments, knot count, mirrored-left and true knots.
@@ -1253,13 +1294,7 @@ __device__ __forceinline__ void accumulate(PassSums& ps, real old, real nw) {
   ps.sq += nw * nw;
   ps.dsq += diff * diff;
   ps.osq += old * old;
-#if EMDB_ACC_NB
-  bool slow = false;
-  real qd = div_nb(diff, nw, slow);
-  if (slow) qd = diff / nw;
-#else
   real qd = diff / nw;
-#endif
   ps.std_ += qd * qd;
   ps.omax = fmax(ps.omax, old);
   ps.omin = fmin(ps.omin, old);
@@ -1493,8 +1528,7 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
   ps.bad = __syncthreads_or(bad || mbad) != 0;
   EMDB_PH(&C, 1);
   const int kb0 = C.kbase[0], kb1 = C.kbase[1], kn0 = C.kcnt[0], kn1 = C.kcnt[1];
-  solve_splines<NT, kInt && EMDB_SETUP_TAB>(K, kb0, kb1, kn0, kn1, tid,
-                                             EMDB_LOAD_CLOCKS ? &C : nullptr);
+  solve_splines<NT>(K, kb0, kb1, kn0, kn1, tid, C);
   const real* oldv = !parked ? imf : kWide ? park_old : borrow_save(slab);
   // A pass with a maximum below zero or a minimum above it is never the last
   // one of its IMF, whatever the stop tests say (the reference forms their
@@ -1995,7 +2029,7 @@ __device__ __forceinline__ void envelope_pass(const SmemLayout& L, char* slab, c
   if (warp == 0) mirror_both(L, K, e, N, NB, T, lane);
   __syncthreads();
   const int kb0 = C.kbase[0], kb1 = C.kbase[1], kn0 = C.kcnt[0], kn1 = C.kcnt[1];
-  solve_splines<kThreads>(K, kb0, kb1, kn0, kn1, tid);
+  solve_splines<kThreads>(K, kb0, kb1, kn0, kn1, tid, C);
   const SideView sv[2] = {{K.XY[0] + kb0, K.M[0], kn0, NB - kb0, e.n_max},
                           {K.XY[1] + kb1, K.M[1], kn1, NB - kb1, e.n_min}};
   nk[0] = kn0;
@@ -2123,7 +2157,6 @@ __global__ void div_check_kernel(int mode, long long n, unsigned long long seed,
         if (__double_as_longlong(div_rn(a, b, y)) != __double_as_longlong(a / b)) ++bad0;
       }
     }
-#if EMDB_PCR_NB || EMDB_ACC_NB || EMDB_SETUP_NB
   } else if (mode == 2) {
     // div_nb: [0] random a/b over [2^-1100, 2^1100] (zeros, subnormals, infinities
     // through the fallback), [1] all-ones / power-of-two significands of b,
@@ -2154,7 +2187,6 @@ __global__ void div_check_kernel(int mode, long long n, unsigned long long seed,
       if (slow) q = div_slow(a3, b3);
       if (__double_as_longlong(q) != __double_as_longlong(div_slow(a3, b3))) ++bad2;
     }
-#endif
   } else {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
       uint64_t h1 = mix64(seed ^ (uint64_t)i), h2 = mix64(h1 ^ 0x5bd1e995ull);
