@@ -48,27 +48,11 @@
 //  EMDB_OUTLINE    rarely taken paths as calls instead of inline copies:
 //                  1 the general evaluation and the binary segment search,
 //                  2 also the IEEE-division fallbacks of the PCR and setup rows
-//  EMDB_MERGED_PLACE  0: one sift-pass instance per knot placement; 1: one
-//                  for the on-chip placements and one for the off-chip ones
-//                  (placement chosen at run time); 2: one for all
-//  EMDB_TREE_SPLIT the six end-of-pass reduction trees spread over the warps
-// Same B200, same clocks, 16,384 x 2048 seismic: MERGED_PLACE/TREE_SPLIT
-// 1/1 208.4k signals/s, 1/0 188.1k, 2/1 195.6k, 0/0 184.9k (and 0/1 172.7k on
-// another box against 208.2k for 1/1): less sift-pass code relieves
-// instruction supply, the dominant stall after FP64 latency.
-//  EMDB_SCAN_UNROLL / EMDB_FILL_UNROLL  unroll factors of the extrema scan
-//                  and knot fill loops: 4 measured 231.8k / 226.3k vs 240.2k
-//                  at 2.
-//  EMDB_WIDE_OVERLAP  wide instances: the warps past the 128 reduction lanes
-//                  run the post-update extrema scan while the lanes sum the
-//                  stop-test terms (the scan then has NT/32 - 4 slots).
-//                  Same bits; measured on B200 (best of two): 512 threads,
-//                  1024 x 8192 seismic 291.2 vs 292.3 ms, 2048 x 4096 50.9 vs
-//                  51.6 ms; 256 threads, 2048 x 4096 50.4 vs 46.4 ms (its
-//                  knot fill then has 4 warps of 8) -- so off.
-#ifndef EMDB_WIDE_OVERLAP
-#define EMDB_WIDE_OVERLAP 0
-#endif
+// Settled: one sift-pass instance for the on-chip placements and one for the
+// off-chip ones (16,384 x 2048 seismic 208.4k signals/s; one instance for all
+// 195.6k, one per placement 184.9k), the six end-of-pass trees spread over the
+// warps (188.1k on one warp): instruction supply decides as much as FP64
+// latency.
 //  EMDB_LANE_UNROLL  wide instances: unroll factor of the lane-sum loops (the
 //                  loads of a lane's samples in flight at once).  With the
 //                  six sums split over the 128-lane groups, B200, 512 threads
@@ -80,18 +64,6 @@
 #endif
 #ifndef EMDB_OUTLINE
 #define EMDB_OUTLINE 2
-#endif
-#ifndef EMDB_MERGED_PLACE
-#define EMDB_MERGED_PLACE 1
-#endif
-#ifndef EMDB_TREE_SPLIT
-#define EMDB_TREE_SPLIT 1
-#endif
-#ifndef EMDB_SCAN_UNROLL
-#define EMDB_SCAN_UNROLL 2
-#endif
-#ifndef EMDB_FILL_UNROLL
-#define EMDB_FILL_UNROLL 2
 #endif
 //  EMDB_LOAD_CLOCKS  instrumented build: thread 0 of each CTA adds the clock64
 //                  cycles of every trace's load into shared memory, of the
@@ -146,8 +118,6 @@ constexpr unsigned kFull = 0xffffffffu;
 // two values loaded and stored as one word
 struct alignas(2 * sizeof(real)) real2 { real x, y; };
 
-constexpr int kScanUnroll = EMDB_SCAN_UNROLL;
-constexpr int kFillUnroll = EMDB_FILL_UNROLL;
 constexpr int kLaneUnroll = EMDB_LANE_UNROLL;
 
 // reference thresholds (kernels.py:81-85, 814, 1069): the first five are
@@ -187,21 +157,17 @@ constexpr size_t kRedBytes = kRedDoubles * sizeof(real);
 
 // Extrema-scan slots of a CTA of NT threads: one contiguous range of 32-sample
 // chunks per slot, scanned by one warp and filled into knots by one warp.
-// The wide instances that overlap the scan with the lane sums scan with the
-// warps past the first four, so they have NT/32 - 4 slots.
 template <int NT>
 __host__ __device__ constexpr int scan_slots() {
-  return (NT > kThreads && EMDB_WIDE_OVERLAP) ? NT / 32 - kWarps : NT / 32;
+  return NT / 32;
 }
-// first warp that scans
-template <int NT>
-__host__ __device__ constexpr int scan_warp0() { return NT / 32 - scan_slots<NT>(); }
 
-// Per-warp scan counts (maxima, minima, sign changes, zero-run ends, fallback
-// trigger) live right after the control block: 5 x (warps per CTA) ints.
+// Per-warp scan counts live right after the control block, one 16-byte word a
+// warp: maxima | minima << 16, sign changes, zero-run ends, fallback trigger
+// (room for 5 ints a warp).
 struct SmemLayout {
   Ctl* ctl;
-  int* wc;            // [5][NW]: w_max | w_min | w_zc | w_zre | w_trig
+  uint4* wc;          // [NW]
   real* red;        // [6][128] between passes (= arena start)
   real* imf;        // [N]
   uint2* mm;          // [nch] ballot masks of the last extrema scan: maxima, minima
@@ -232,7 +198,7 @@ __device__ __forceinline__ SmemLayout carve(char* base, int N, int arena_total,
   size_t nch = (size_t)(N + 31) / 32;
   char* p = base;
   L.ctl = reinterpret_cast<Ctl*>(p); p += align16(sizeof(Ctl));
-  L.wc = reinterpret_cast<int*>(p); p += align16(5 * (NT / 32) * sizeof(int));
+  L.wc = reinterpret_cast<uint4*>(p); p += align16(5 * (NT / 32) * sizeof(int));
   L.mm = reinterpret_cast<uint2*>(p); p += align16(nch * 4) * 2;
   L.pp = reinterpret_cast<uint32_t*>(p); p += align16(nch * 2) * 2;
   // the proto-IMF directly ahead of the arena: the borrow placement uses both
@@ -631,66 +597,72 @@ struct TimeAxis {
 // with the serial scan's plateau rule, kernels.py:157-200).
 // ---------------------------------------------------------------------------
 // NS slots; `slot` is the calling warp's slot.
+//
+// The common chunk has no flat step, no exact zero and no underflowing product
+// in it or just before it; there an extremum is dp*dn < 0, its kind the sign
+// bit of dp, and a crossing v*vn < 0, four compares of doubles a sample in all
+// (all the reference's tests, kernels.py:157-200, took ten).  Any sample that
+// could be otherwise (a product that is zero or NaN) sends its chunk, and the
+// next one, whose first sample looks back at it, through those tests.
+// Neighbours come straight from shared memory (conflict-free consecutive
+// words): no shuffles, iterations independent.  Two chunks a trip where one
+// trace has an SM to itself, one where four share it (16,384 x 2048 seismic
+// 71.9 ms at one, 73.8 at two; 256 x 8192 65.0 and 64.6).
 template <int NS>
 __device__ __forceinline__ void extrema_count(const SmemLayout& L, int N, int slot, int lane) {
   const real* imf = L.imf;
-  int nch = (N + 31) >> 5;
-  int c0 = (slot * nch) / NS, c1 = ((slot + 1) * nch) / NS;
-  int rmax = 0, rmin = 0, zc = 0, zre = 0;
+  const int nch = (N + 31) >> 5;
+  const int c0 = (slot * nch) / NS, c1 = ((slot + 1) * nch) / NS;
+  uint32_t run = 0;              // maxima | minima << 16 of the slot so far
+  int zc = 0, zre = 0;
   bool trig = false;
-  // neighbours straight from shared memory (conflict-free consecutive
-  // doubles): no shuffles, no divergent edge loads; iterations independent
-#pragma unroll kScanUnroll
+  bool careful = c0 > 0 && c0 < c1 && imf[(c0 << 5) - 1] == real(0);
+#pragma unroll (NS == kWarps ? 1 : 2)
   for (int c = c0; c < c1; ++c) {
-    int i = (c << 5) + lane;
-    real v = (i < N) ? imf[i] : 0.0;
-    real vp = (i >= 1 && i - 1 < N) ? imf[i - 1] : 0.0;
-    real vn = (i + 1 < N) ? imf[i + 1] : 0.0;
-    bool interior = (i >= 1) && (i <= N - 2);
-    real dp = v - vp, dn = vn - v;
-    bool strict = interior && (dp * dn < 0.0);
-    bool ismin = strict && (dp < 0.0);
-    bool ismax = strict && !(dp < 0.0);
-    const bool flat = interior && dn == 0.0 && dp != 0.0;
-    if (__any_sync(kFull, flat)) {
-      // rare: true left edge of a flat run, classified by the slopes around it
-      if (flat) {
+    const int i = (c << 5) + lane;
+    const real v = imf[min(i, N - 1)], vp = imf[max(min(i, N) - 1, 0)], vn = imf[min(i + 1, N - 1)];
+    const bool interior = i >= 1 && i <= N - 2, left = i <= N - 2;
+    const real dp = v - vp, dn = vn - v;
+    const real turn = dp * dn, cross = v * vn;
+    const bool strict = interior && turn < real(0);
+    bool ismin = strict && dp < real(0);
+    bool ismax = strict && !(dp < real(0));
+    const bool sc = left && cross < real(0);
+    const bool odd = (interior && !(fabs(turn) > real(0))) || !(fabs(cross) > real(0));
+    const bool any_odd = __any_sync(kFull, odd);
+    if (any_odd || careful) {
+      if (interior && dn == real(0) && dp != real(0)) {
+        // rare: true left edge of a flat run, classified by the slopes around it
         int j = i;
         while (j + 1 < N && imf[j + 1] == v) ++j;
         if (j + 1 < N) {
-          real da = imf[j + 1] - imf[j];
-          if (dp > 0.0 && da < 0.0) ismax = true;
-          else if (dp < 0.0 && da > 0.0) ismin = true;
+          const real da = imf[j + 1] - imf[j];
+          if (dp > real(0) && da < real(0)) ismax = true;
+          else if (dp < real(0) && da > real(0)) ismin = true;
         }
       }
+      trig |= interior && (dp == real(0) || dn == real(0) || v == real(0));
+      const bool zr = i >= 1 && i < N && v != real(0) && vp == real(0);
+      zre += __popc(__ballot_sync(kFull, zr));
     }
-    trig |= interior && (dp == 0.0 || dn == 0.0 || v == 0.0);
-    bool sc = (i <= N - 2) && (v != 0.0) && (v * vn < 0.0);
-    bool zr = (i >= 1) && (i < N) && (v != 0.0) && (vp == 0.0);
-    uint32_t bmax = __ballot_sync(kFull, ismax);
-    uint32_t bmin = __ballot_sync(kFull, ismin);
+    careful = any_odd;
+    const uint32_t bmax = __ballot_sync(kFull, ismax);
+    const uint32_t bmin = __ballot_sync(kFull, ismin);
     if (lane == 0) {
       L.mm[c] = make_uint2(bmax, bmin);
-      L.pp[c] = (uint32_t)rmax | ((uint32_t)rmin << 16);
+      L.pp[c] = run;
     }
-    rmax += __popc(bmax);
-    rmin += __popc(bmin);
+    run += (uint32_t)__popc(bmax) + ((uint32_t)__popc(bmin) << 16);
     zc += __popc(__ballot_sync(kFull, sc));
-    zre += __popc(__ballot_sync(kFull, zr));
   }
   trig = __any_sync(kFull, trig);
-  if (lane == 0) {
-    int* w = L.wc;
-    w[slot] = rmax; w[NS + slot] = rmin;
-    w[2 * NS + slot] = zc; w[3 * NS + slot] = zre; w[4 * NS + slot] = trig ? 1 : 0;
-  }
+  if (lane == 0) L.wc[slot] = make_uint4(run, (uint32_t)zc, (uint32_t)zre, trig ? 1u : 0u);
 }
 
 struct ExtInfo {
-  int tot_max, tot_min;   // true counts
   int n_max, n_min;       // stored (capped) counts
   int n_zer;
-  int off_max, off_min;   // this warp's rank offsets
+  uint32_t off;           // this warp's rank offsets: maxima | minima << 16
   bool overflow;
   bool trig;              // serial-fallback trigger (exact zeros / flat runs)
 };
@@ -699,31 +671,24 @@ struct ExtInfo {
 // find_extrema_parallel: without a fallback trigger the zero-crossing count is
 // sign changes only; with one, the serial count adds one per zero run that
 // ends before N (kernels.py:123-143, 273-276).
-// `slot`: the caller's fill slot (its warp, if the warp fills), for its rank offsets
+// One lane reads one warp's word; a warp then sums them (the counts of a kind
+// are below 2^16 for the longest trace).  `warp`: the caller's, for its rank
+// offsets.
 template <int NS>
-__device__ __forceinline__ ExtInfo extrema_totals(const SmemLayout& L, int slot, int max_extrema) {
-  constexpr int NW = NS;
-  const int warp = slot;
-  const Ctl& C = *L.ctl;
-  const int* wc = L.wc;
+__device__ __forceinline__ ExtInfo extrema_totals(const SmemLayout& L, int warp, int lane,
+                                                  int max_extrema) {
+  const uint4 w = lane < NS ? L.wc[lane] : make_uint4(0u, 0u, 0u, 0u);
+  const uint32_t tot = __reduce_add_sync(kFull, w.x);
+  const uint32_t zc = __reduce_add_sync(kFull, w.y);
   ExtInfo e;
-  e.tot_max = e.tot_min = 0;
-  int zc = 0, zre = 0;
-  bool trig = false;
-  e.off_max = e.off_min = 0;
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    if (w < warp) { e.off_max += wc[w]; e.off_min += wc[NW + w]; }
-    e.tot_max += wc[w]; e.tot_min += wc[NW + w];
-    zc += wc[2 * NW + w]; zre += wc[3 * NW + w];
-    trig |= wc[4 * NW + w] != 0;
-  }
-  e.trig = trig;
-  if (!trig && C.chunk_bad) trig = true;
-  e.n_zer = zc + (trig ? zre : 0);
-  e.n_max = min(e.tot_max, max_extrema);
-  e.n_min = min(e.tot_min, max_extrema);
-  e.overflow = (e.tot_max >= max_extrema) || (e.tot_min >= max_extrema);
+  e.off = __reduce_add_sync(kFull, lane < warp ? w.x : 0u);
+  e.trig = __any_sync(kFull, w.w != 0u);
+  e.n_zer = (int)zc;
+  if (e.trig || L.ctl->chunk_bad) e.n_zer += (int)__reduce_add_sync(kFull, w.z);
+  const int tot_max = (int)(tot & 0xffffu), tot_min = (int)(tot >> 16);
+  e.n_max = min(tot_max, max_extrema);
+  e.n_min = min(tot_min, max_extrema);
+  e.overflow = tot_max >= max_extrema || tot_min >= max_extrema;
   return e;
 }
 
@@ -748,32 +713,22 @@ __device__ void chunk_fallback_check(const SmemLayout& L, int N, int tid) {
   __syncthreads();
 }
 
-// One extrema scan = count pass + totals.  Ends after a barrier with every
-// thread holding the same totals.
-// The totals of a finished count pass (after its barrier), and the
-// reference's rare chunk fallback.  Every thread gets the totals; a warp that
-// fills gets its slot's rank offsets.
-template <int NT>
-__device__ __forceinline__ ExtInfo extrema_finish(const SmemLayout& L, int N, int tid, int warp,
-                                                  int max_extrema) {
-  constexpr int NS = scan_slots<NT>();
-  const int slot = warp < NS ? warp : 0;
-  ExtInfo e = extrema_totals<NS>(L, slot, max_extrema);
-  if (N > kThreads * 128 && L.imf[0] == 0.0 && !e.trig) {
-    chunk_fallback_check(L, N, tid);
-    e = extrema_totals<NS>(L, slot, max_extrema);
-  }
-  return e;
-}
-
+// One extrema scan = count pass + totals, and the reference's rare chunk
+// fallback.  Ends after a barrier with every thread holding the same totals
+// and its warp's rank offsets.
 template <int NT>
 __device__ __forceinline__ ExtInfo extrema_scan(const SmemLayout& L, int N, int tid, int warp,
                                                 int lane, int max_extrema) {
-  constexpr int W0 = scan_warp0<NT>();
-  if (W0 == 0 || warp >= W0) extrema_count<scan_slots<NT>()>(L, N, warp - W0, lane);
+  constexpr int NS = scan_slots<NT>();
+  extrema_count<NS>(L, N, warp, lane);
   if (tid == 0) L.ctl->chunk_bad = 0;
   __syncthreads();
-  return extrema_finish<NT>(L, N, tid, warp, max_extrema);
+  ExtInfo e = extrema_totals<NS>(L, warp, lane, max_extrema);
+  if (N > kThreads * 128 && L.imf[0] == 0.0 && !e.trig) {
+    chunk_fallback_check(L, N, tid);
+    e = extrema_totals<NS>(L, warp, lane, max_extrema);
+  }
+  return e;
 }
 
 // ---------------------------------------------------------------------------
@@ -791,12 +746,12 @@ __device__ __forceinline__ bool fill_true_knots(const SmemLayout& L, const Knots
   int c0 = (warp * nch) / NS, c1 = ((warp + 1) * nch) / NS;
   unsigned lt = (1u << lane) - 1u;
   bool bad = false;
+  const int off_max = (int)(e.off & 0xffffu), off_min = (int)(e.off >> 16);
   // one extremum lane: rank it, write its knot, note head / tail indices
   auto put = [&](uint32_t bm, uint32_t bn, int pm, int pn, int ii, real v) {
     const bool ismax = (bm >> lane) & 1u;
     int q = ismax ? 0 : 1;
-    int rank = q == 0 ? e.off_max + pm + __popc(bm & lt)
-                      : e.off_min + pn + __popc(bn & lt);
+    int rank = q == 0 ? off_max + pm + __popc(bm & lt) : off_min + pn + __popc(bn & lt);
     int nq = q == 0 ? e.n_max : e.n_min;
     if (rank < nq) {
       (q == 0 ? K.XY[0] : K.XY[1])[NB + rank] = real2{T(ii), v};
@@ -808,7 +763,7 @@ __device__ __forceinline__ bool fill_true_knots(const SmemLayout& L, const Knots
   };
   if (!e.trig) {
     // no exact zeros or flat runs in this proto-IMF: every extremum is strict
-#pragma unroll kFillUnroll
+#pragma unroll (NS == kWarps ? 1 : 2)
     for (int c = c0; c < c1; ++c) {
       const uint32_t bm = L.mm[c].x, bn = L.mm[c].y;
       const int pm = L.pp[c] & 0xffff, pn = L.pp[c] >> 16;
@@ -838,8 +793,7 @@ __device__ __forceinline__ bool fill_true_knots(const SmemLayout& L, const Knots
   // the chunks' prefixes become global (warp offset added) for the evaluation
   // pass's segment counts, once every lane has taken its ranks
   __syncwarp();
-  const uint32_t off = (uint32_t)e.off_max | ((uint32_t)e.off_min << 16);
-  for (int c = c0 + lane; c < c1; c += 32) L.pp[c] += off;
+  for (int c = c0 + lane; c < c1; c += 32) L.pp[c] += e.off;
   return bad;
 }
 
@@ -1505,9 +1459,7 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
                                     : place_knots(slab, kc0, kc1);
   PassSums ps;
   EMDB_PH(&C, 9);
-  constexpr int NS = scan_slots<NT>();
-  bool bad = false;
-  if (NS == NT / 32 || warp < NS) bad = fill_true_knots<NS>(L, K, e, N, NB, T, warp, lane);
+  bool bad = fill_true_knots<scan_slots<NT>()>(L, K, e, N, NB, T, warp, lane);
   bad = __syncthreads_or(bad);
   EMDB_PH(&C, 0);
   bool mbad = false;
@@ -1572,39 +1524,16 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
   }
   // per-lane partial sums, then the reference's 128-lane trees on warp 0
   real* red = kPlace == kPlaceSlab ? L.red : K.red;
-  if constexpr (kWide && !EMDB_WIDE_OVERLAP) {
+  if constexpr (kWide) {
     __syncthreads();
     EMDB_PH(&C, 5);
     if (sums) wide_lane_sums<NT>(red, oldv, imf, qbuf, N, tid);
-  } else if (kWide) {
-    // the reference's 128 lanes, each summing its samples in increasing order;
-    // meanwhile the other warps run the next pass's extrema count on the
-    // updated proto-IMF (both only read it)
-    __syncthreads();
-    EMDB_PH(&C, 5);
-    if (tid < kThreads) {
-      for (int i = tid; i < N; i += kThreads) {
-        const real old = oldv[i], nw = imf[i], qd = qbuf[i];
-        const real diff = nw - old;
-        ps.sq += nw * nw;
-        ps.dsq += diff * diff;
-        ps.osq += old * old;
-        ps.std_ += qd * qd;
-        ps.omax = fmax(ps.omax, old);
-        ps.omin = fmin(ps.omin, old);
-      }
-    } else if (EMDB_WIDE_OVERLAP) {
-      extrema_count<scan_slots<NT>()>(L, N, warp - scan_warp0<NT>(), lane);
-    }
-    if (EMDB_WIDE_OVERLAP && tid == 0) C.chunk_bad = 0;
-  }
-  if (sums && (!kWide || (EMDB_WIDE_OVERLAP && tid < kThreads))) {
+  } else if (sums) {
     red[tid] = ps.sq; red[128 + tid] = ps.dsq; red[256 + tid] = ps.osq;
     red[384 + tid] = ps.std_; red[512 + tid] = ps.omax; red[640 + tid] = ps.omin;
   }
   __syncthreads();
   EMDB_PH(&C, kWide ? 6 : 5);
-#if EMDB_TREE_SPLIT
   // the six trees spread over the warps (warp w: sum w; warps 0/1 also the
   // max / min tree); the next extrema scan's barrier publishes C.sums
   if (sums && (!kWide || warp < kWarps)) {
@@ -1615,22 +1544,6 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
       if (lane == 0) C.sums[4 + warp] = b;
     }
   }
-  // overlapped scan: this barrier publishes C.sums (the scan's would have)
-  if (kWide && EMDB_WIDE_OVERLAP) __syncthreads();
-#else
-  if (warp == 0) {
-    real a0 = lane_tree(red, lane, 0);
-    real a1 = lane_tree(red + 128, lane, 0);
-    real a2 = lane_tree(red + 256, lane, 0);
-    real a3 = lane_tree(red + 384, lane, 0);
-    real a4 = lane_tree(red + 512, lane, 1);
-    real a5 = lane_tree(red + 640, lane, 2);
-    if (lane == 0) {
-      C.sums[0] = a0; C.sums[1] = a1; C.sums[2] = a2;
-      C.sums[3] = a3; C.sums[4] = a4; C.sums[5] = a5;
-    }
-  }
-#endif
   return (ps.bad ? 1 : 0) | (oor ? 2 : 0);
 }
 
@@ -1766,18 +1679,41 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
     bool finished = false;
     int extNo_last = rec ? rec->extNo_last : -1;
     bool stale = rec ? rec->stale != 0 : false;
-    int n_resume = rec ? rec->n : 0;
+    const int n_resume = rec ? rec->n : 0;
     bool yielded = false;
     int n_yield = 0;
     unsigned long long passes = 0, spilled = 0;
 
-    ExtInfo e = extrema_scan<NT>(L, N, tid, warp, lane, p.max_extrema);
-    ovf |= e.overflow;
-
-    while (!finished && imf_count < MAXI - 1) {
-      int n = n_resume;
-      n_resume = 0;
-      for (;;) {
+    // One loop over scans: each sift pass and each emitted IMF row ends in an
+    // extrema scan of the proto-IMF it leaves, which is also the next pass's
+    // (the reference scans the same data twice, kernels.py:930 vs 965).  One
+    // copy of the scan, the pass and the emission keeps the loop small.
+    int n = n_resume;
+    bool post = false;          // the scan follows a sift pass
+    bool pass_bad = false;
+    for (;;) {
+      const ExtInfo e = extrema_scan<NT>(L, N, tid, warp, lane, p.max_extrema);
+      EMDB_PH(&C, 7);
+      ovf |= e.overflow;
+      const int extNo = e.n_max + e.n_min;
+      bool emit = false;
+      if (post) {
+        extNo_last = extNo;
+        if (!pass_bad && abs(extNo - e.n_zer) < 2) {
+          const real sum_new_sq = C.sums[0], diff_sq = C.sums[1], old_sq = C.sums[2];
+          const real std_sum = C.sums[3], omax = C.sums[4], omin = C.sums[5];
+          bool f1 = false;
+          if (sum_new_sq < kSumNewSqMin) f1 = false;
+          else if (diff_sq / (omax - omin) < kSvarThr) f1 = true;
+          else if (std_sum < kStdThr) f1 = true;
+          else if (diff_sq / old_sq < kEnergyRatioThr) f1 = true;
+          if (f1) {
+            if (tid == 0) { C.dbg_n[imf_count] = n; C.dbg_e[imf_count] = extNo; C.dbg_z[imf_count] = e.n_zer; }
+            emit = true;
+          }
+        }
+      }
+      if (!emit) {
         if (migrate && (n & 3) == 0) {
           // every trace has started and few remain: hand this one to the
           // 512-thread instance at this pass boundary (checked every fourth
@@ -1796,103 +1732,50 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
         if (n >= p.max_iteration) {
           ovf = true;
           if (tid == 0) { C.dbg_n[imf_count] = n; C.dbg_e[imf_count] = -1; C.dbg_z[imf_count] = -1; }
-          break;
-        }
-        const int extNo = e.n_max + e.n_min;
-        if (!(extNo > 2 && e.n_max >= 1 && e.n_min >= 1)) {
+          emit = true;
+        } else if (!(extNo > 2 && e.n_max >= 1 && e.n_min >= 1)) {
           extNo_last = extNo;
           finished = true;
-          break;
-        }
-        const int kc0 = e.n_max + 2 * NB + 2, kc1 = e.n_min + 2 * NB + 2;
-        int flags;
-#if EMDB_MERGED_PLACE
-        {
-          // the wide instance's stride also holds the parked proto-IMF and the
-          // quotients: its knots may use only the part before them
-          const int place = choose_place(N, L.arena_bytes, kWide ? p.park_off : p.slab_stride,
-                                         kc0, kc1, kGImf);
-          if (EMDB_MERGED_PLACE == 2)
-            flags = sift_pass<NT, kAnyPlace, kInt>(L, slab, e, N, NB, T, tid, warp, lane, place,
-                                                   park_old, qbuf);
-          else if (place == kPlaceSmem || place == kPlaceBorrow || place == kPlaceBorrow2)
-            flags = sift_pass<NT, kOnChip, kInt>(L, slab, e, N, NB, T, tid, warp, lane, place,
-                                                 park_old, qbuf);
-          else
-            flags = sift_pass<NT, kOffChip, kInt>(L, slab, e, N, NB, T, tid, warp, lane, place,
-                                                  park_old, qbuf);
-          spilled += place != kPlaceSmem;
-        }
-#else
-        {
-          const int place = choose_place(N, L.arena_bytes, kWide ? p.park_off : p.slab_stride,
-                                         kc0, kc1, kGImf);
-          if (place == kPlaceSmem)
-            flags = sift_pass<NT, kPlaceSmem, kInt>(L, slab, e, N, NB, T, tid, warp, lane,
-                                                    place, park_old, qbuf);
-          else if (place == kPlaceBorrow)
-            flags = sift_pass<NT, kPlaceBorrow, kInt>(L, slab, e, N, NB, T, tid, warp, lane,
-                                                      place, park_old, qbuf);
-          else if (place == kPlaceBorrow2)
-            flags = sift_pass<NT, kPlaceBorrow2, kInt>(L, slab, e, N, NB, T, tid, warp, lane,
-                                                       place, park_old, qbuf);
-          else if (place == kPlaceSplit)
-            flags = sift_pass<NT, kPlaceSplit, kInt>(L, slab, e, N, NB, T, tid, warp, lane,
-                                                     place, park_old, qbuf);
-          else if (place == kPlacePark)
-            flags = sift_pass<NT, kPlacePark, kInt>(L, slab, e, N, NB, T, tid, warp, lane,
-                                                    place, park_old, qbuf);
-          else
-            flags = sift_pass<NT, kPlaceSlab, kInt>(L, slab, e, N, NB, T, tid, warp, lane,
-                                                    place, park_old, qbuf);
-          spilled += place != kPlaceSmem;
-        }
-#endif
-        ++passes;
-        const bool pass_bad = (flags & 1) != 0;
-        stale |= (flags & 2) != 0;
-        // ---- post-update extrema scan (also next pass's pre-scan); the
-        // wide instances ran its count inside the pass ----
-        if (kWide && EMDB_WIDE_OVERLAP) e = extrema_finish<NT>(L, N, tid, warp, p.max_extrema);
-        else e = extrema_scan<NT>(L, N, tid, warp, lane, p.max_extrema);
-        EMDB_PH(&C, 7);
-        ovf |= e.overflow;
-        const int extNo2 = e.n_max + e.n_min;
-        const int nzm2 = e.n_zer;
-        const bool f2 = abs(extNo2 - nzm2) < 2;
-        bool f1 = false;
-        if (!pass_bad) {
-          real sum_new_sq = C.sums[0], diff_sq = C.sums[1], old_sq = C.sums[2];
-          real std_sum = C.sums[3], omax = C.sums[4], omin = C.sums[5];
-          if (sum_new_sq < kSumNewSqMin) f1 = false;
-          else if (diff_sq / (omax - omin) < kSvarThr) f1 = true;
-          else if (std_sum < kStdThr) f1 = true;
-          else if (diff_sq / old_sq < kEnergyRatioThr) f1 = true;
-        }
-        extNo_last = extNo2;
-        if (f1 && f2) {
-          if (tid == 0) { C.dbg_n[imf_count] = n; C.dbg_e[imf_count] = extNo2; C.dbg_z[imf_count] = nzm2; }
-          break;
+          emit = true;
         }
       }
-      if (yielded) break;
-      // ---- emit IMF row, running residue into the next row, end condition ----
-      EMDB_PH(&C, 9);
-      {
+      if (emit) {
+        // ---- emit IMF row, running residue into the next row and imf[], end
+        // condition ----
+        EMDB_PH(&C, 9);
         const real* rsrc = imf_count == 0 ? S : out + (int64_t)imf_count * N;
         real* row = out + (int64_t)imf_count * N;
         real* rnext = out + (int64_t)(imf_count + 1) * N;
         real gmax = -1e30, gmin = 1e30, gabs = 0.0;
-        // the reference's 128 lanes (a wider CTA's other threads wait: once per IMF)
-        for (int i = tid; i < (!kWide || tid < kThreads ? N : 0); i += kThreads) {
-          real r = rsrc[i];
-          real v = imf[i];
-          row[i] = v;
-          real rn = r - v;
-          rnext[i] = rn;
+        auto note = [&](real rn) {
           gmax = fmax(gmax, rn);
           gmin = fmin(gmin, rn);
           gabs += fabs(rn);
+        };
+        // four samples' residues in flight (the rows may alias as far as the
+        // compiler knows, so it does not hoist loads over stores itself)
+        for (int i0 = tid; i0 < N; i0 += 4 * NT) {
+          real r[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) r[q] = rsrc[min(i0 + q * NT, N - 1)];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int i = i0 + q * NT;
+            if (i < N) {
+              const real v = imf[i];
+              const real rn = r[q] - v;
+              row[i] = v;
+              rnext[i] = rn;
+              imf[i] = rn;
+              if (!kWide) note(rn);
+            }
+          }
+        }
+        if (kWide) {
+          // the reference's 128 lanes
+          __syncthreads();
+          if (tid < kThreads)
+            for (int i = tid; i < N; i += kThreads) note(imf[i]);
         }
         real* red = L.red;
         if (!kWide || tid < kThreads) { red[tid] = gmax; red[128 + tid] = gmin; red[256 + tid] = gabs; }
@@ -1906,15 +1789,29 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
         __syncthreads();
         ++imf_count;
         if (C.sums[6] < kRangeThr || C.sums[7] < kTotalPowerThr) finished = true;
+        EMDB_PH(&C, 8);
+        if (finished || imf_count >= MAXI - 1) break;
+        n = 0;
+        post = false;
+        continue;
       }
-      if (!finished && imf_count < MAXI - 1) {
-        const real* rsrc = out + (int64_t)imf_count * N;
-        for (int i = tid; i < N; i += NT) imf[i] = rsrc[i];
-        __syncthreads();
-        e = extrema_scan<NT>(L, N, tid, warp, lane, p.max_extrema);
-        ovf |= e.overflow;
-      }
-      EMDB_PH(&C, 8);
+      // the wide instance's stride also holds the parked proto-IMF and the
+      // quotients: its knots may use only the part before them
+      const int kc0 = e.n_max + 2 * NB + 2, kc1 = e.n_min + 2 * NB + 2;
+      const int place = choose_place(N, L.arena_bytes, kWide ? p.park_off : p.slab_stride,
+                                     kc0, kc1, kGImf);
+      int flags;
+      if (place == kPlaceSmem || place == kPlaceBorrow || place == kPlaceBorrow2)
+        flags = sift_pass<NT, kOnChip, kInt>(L, slab, e, N, NB, T, tid, warp, lane, place,
+                                             park_old, qbuf);
+      else
+        flags = sift_pass<NT, kOffChip, kInt>(L, slab, e, N, NB, T, tid, warp, lane, place,
+                                              park_old, qbuf);
+      spilled += place != kPlaceSmem;
+      ++passes;
+      pass_bad = (flags & 1) != 0;
+      stale |= (flags & 2) != 0;
+      post = true;
     }
 
     if (yielded) {
@@ -1951,10 +1848,12 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
     const bool trend = extNo_last <= 2 && imf_count > 0;
     if (trend) imf_count -= 1;
     const real* rres = last_row == 0 ? S : out + (int64_t)last_row * N;
+    // the last proto-IMF (imf[] holds the residue): the row before the residue's
+    const real* vlast = out + (int64_t)max(last_row - 1, 0) * N;
     real amax = 0.0;
     for (int i = tid; i < (!kWide || tid < kThreads ? N : 0); i += kThreads) {
       real r = rres[i];
-      if (trend) r = r + imf[i];
+      if (trend) r = r + vlast[i];
       amax = fmax(amax, fabs(r));
     }
     real* red = L.red;
@@ -1969,7 +1868,7 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
     const int nim = rzero ? imf_count : imf_count + 1;
     for (int i = tid; i < N; i += NT) {
       if (trend) {
-        real r = rres[i] + imf[i];
+        real r = rres[i] + vlast[i];
         if (!rzero) out[(int64_t)imf_count * N + i] = r;
         out[(int64_t)last_row * N + i] = 0.0;
       } else {
