@@ -135,8 +135,8 @@ struct Ctl {
   int job;
   int head[2][kMaxNbsym + 1];  // first NB+1 extrema indices per side (0 = max, 1 = min)
   int tail[2][kMaxNbsym + 1];  // tail[q][k] = index of extremum n_q-1-k
-  int mlist[4][kMaxNbsym + 1]; // mirrored index lists: lmax, lmin, rmax, rmin
-  int mcnt[4];                 // entries per list; [0], [1] hold a range during the solve
+  unsigned range[2];           // largest / smallest right-hand side during the solve
+  int unused[38];              // keeps the block's size: it decides the longest trace a CTA takes
   int lsym, rsym;
   int kbase[2], kcnt[2];
   int dbg_n[kMaxImfsCap], dbg_e[kMaxImfsCap], dbg_z[kMaxImfsCap];
@@ -799,8 +799,13 @@ __device__ __forceinline__ bool fill_true_knots(const SmemLayout& L, const Knots
 
 // ---------------------------------------------------------------------------
 // Boundary mirroring (mirror_one_side, kernels.py:360-558) for both sides.
-// Lane 0 of warp 0 makes the O(nbsym) decisions into shared lists; the warp
-// then writes the mirrored knots.  Knot positions are strictly increasing
+// Every lane of warp 0 makes the same O(1) decisions (which extremum comes
+// first and last, whether the end sample lies beyond its neighbour, whether
+// the mirrored knots reach the end) and then writes its own mirrored knots: a
+// list is a run of extremum ranks plus possibly the end sample, so entry j
+// needs no list in memory.  The chain is five dependent shared-memory reads;
+// with the lists built by one lane, entry by entry, it was three to four times
+// as long.  Knot positions are strictly increasing
 // whenever T is (the host checks T), so the reference's adjacent-duplicate
 // removal never drops a knot and is not needed here.
 // ---------------------------------------------------------------------------
@@ -808,104 +813,82 @@ __device__ __forceinline__ int ind_of(const Ctl& C, int q, int n, int NB, int k)
   return k <= NB ? C.head[q][k] : C.tail[q][n - 1 - k];
 }
 
+// Ranks hi, hi-1, ..., lo of one kind of extremum; `end`: and the trace's end
+// sample (on the left after them, on the right before them, the ranks then
+// ascending).
+struct MirrorList {
+  int hi, lo, end;
+  __device__ __forceinline__ int count() const { return max(hi - lo + 1, 0) + end; }
+};
+
 __device__ __forceinline__ bool mirror_both(const SmemLayout& L, const Knots& K, const ExtInfo& e,
                                             int N, int NB, const TimeAxis& T, int lane) {
   Ctl& C = *L.ctl;
   const real* S = L.imf;
   const int nM = e.n_max, nm = e.n_min;
+  const int im0 = C.head[0][0], in0 = C.head[1][0], imL = C.tail[0][0], inL = C.tail[1][0];
+  const real s0 = S[0], sN = S[N - 1];
+  MirrorList l0, l1, r0, r1;
+  int lsym, rsym;
+  // ---- left bound: kernels.py:383-413 ----
+  {
+    const bool mf = im0 < in0;                       // a maximum comes first
+    const real so = S[mf ? in0 : im0];
+    const bool over = mf ? s0 > so : s0 < so;
+    const int nf = mf ? nM : nm, no = mf ? nm : nM;
+    const MirrorList f{min(nf, over ? NB + 1 : NB) - 1, over ? 1 : 0, 0};
+    const MirrorList o{min(no, over ? NB : NB - 1) - 1, 0, over ? 0 : 1};
+    l0 = mf ? f : o;
+    l1 = mf ? o : f;
+    lsym = over ? (mf ? im0 : in0) : 0;
+  }
+  // ---- right bound: kernels.py:415-454 ----
+  {
+    const bool mf = imL > inL;                       // a maximum comes last
+    const real so = S[mf ? inL : imL];
+    const bool over = mf ? sN > so : sN < so;
+    const int nf = mf ? nM : nm, no = mf ? nm : nM;
+    const MirrorList f{over ? nf - 2 : nf - 1, max(over ? nf - NB - 1 : nf - NB, 0), 0};
+    const MirrorList o{no - 1, max(over ? no - NB : no - NB + 1, 0), over ? 0 : 1};
+    r0 = mf ? f : o;
+    r1 = mf ? o : f;
+    rsym = over ? (mf ? imL : inL) : N - 1;
+  }
+  // An empty list falls back to the whole index list (kernels.py:456-459,
+  // 523-531); that only happens when the side has exactly one extremum,
+  // so the whole list is that one index.
+  if (l0.count() == 0) l0 = MirrorList{0, 0, 0};
+  if (l1.count() == 0) l1 = MirrorList{0, 0, 0};
+  if (r0.count() == 0) r0 = MirrorList{nM - 1, nM - 1, 0};
+  if (r1.count() == 0) r1 = MirrorList{nm - 1, nm - 1, 0};
+  // sample index of entry j
+  auto left_at = [&](const MirrorList& l, int q, int n, int j) {
+    return l.hi - j >= l.lo ? ind_of(C, q, n, NB, l.hi - j) : 0;
+  };
+  auto right_at = [&](const MirrorList& l, int q, int n, int j) {
+    if (l.end) return j == 0 ? N - 1 : ind_of(C, q, n, NB, l.lo + j - 1);
+    return ind_of(C, q, n, NB, l.hi - j);
+  };
+  // ---- mirrored point does not reach the boundary (kernels.py:469-503) ----
+  const real T0 = T(0), TN = T(N - 1);
+  const real tl = T(lsym), tr = T(rsym);
+  // the mirrored positions are stored as REAL_T before the compares
+  // (kernels.py:471-472, 488-489): in the FP32 build that rounds them
+  const real tl1 = 2.0 * tl - T(left_at(l1, 1, nm, 0)), tl0 = 2.0 * tl - T(left_at(l0, 0, nM, 0));
+  if (tl1 > T0 || tl0 > T0) {
+    if (lsym == im0) l0 = MirrorList{min(nM, NB) - 1, 0, 0};
+    else l1 = MirrorList{min(nm, NB) - 1, 0, 0};
+    lsym = 0;
+  }
+  const real tr1 = 2.0 * tr - T(right_at(r1, 1, nm, r1.count() - 1));
+  const real tr0 = 2.0 * tr - T(right_at(r0, 0, nM, r0.count() - 1));
+  if (tr1 < TN || tr0 < TN) {
+    if (rsym == imL) r0 = MirrorList{nM - 1, max(nM - NB, 0), 0};
+    else r1 = MirrorList{nm - 1, max(nm - NB, 0), 0};
+    rsym = N - 1;
+  }
+  const int c0 = l0.count(), c1 = l1.count(), c2 = r0.count(), c3 = r1.count();
   if (lane == 0) {
-    int* l0 = C.mlist[0];
-    int* l1 = C.mlist[1];
-    int* r0 = C.mlist[2];
-    int* r1 = C.mlist[3];
-    int c0 = 0, c1 = 0, c2 = 0, c3 = 0;
-    int lsym, rsym;
-    const int im0 = ind_of(C, 0, nM, NB, 0), in0 = ind_of(C, 1, nm, NB, 0);
-    const int imL = ind_of(C, 0, nM, NB, nM - 1), inL = ind_of(C, 1, nm, NB, nm - 1);
-    // ---- left bound ----
-    if (im0 < in0) {
-      if (S[0] > S[in0]) {
-        for (int k = min(nM, NB + 1) - 1; k >= 1; --k) l0[c0++] = ind_of(C, 0, nM, NB, k);
-        for (int k = min(nm, NB) - 1; k >= 0; --k) l1[c1++] = ind_of(C, 1, nm, NB, k);
-        lsym = im0;
-      } else {
-        for (int k = min(nM, NB) - 1; k >= 0; --k) l0[c0++] = ind_of(C, 0, nM, NB, k);
-        for (int k = min(nm, NB - 1) - 1; k >= 0; --k) l1[c1++] = ind_of(C, 1, nm, NB, k);
-        l1[c1++] = 0;
-        lsym = 0;
-      }
-    } else {
-      if (S[0] < S[im0]) {
-        for (int k = min(nM, NB) - 1; k >= 0; --k) l0[c0++] = ind_of(C, 0, nM, NB, k);
-        for (int k = min(nm, NB + 1) - 1; k >= 1; --k) l1[c1++] = ind_of(C, 1, nm, NB, k);
-        lsym = in0;
-      } else {
-        for (int k = min(nM, NB - 1) - 1; k >= 0; --k) l0[c0++] = ind_of(C, 0, nM, NB, k);
-        l0[c0++] = 0;
-        for (int k = min(nm, NB) - 1; k >= 0; --k) l1[c1++] = ind_of(C, 1, nm, NB, k);
-        lsym = 0;
-      }
-    }
-    // ---- right bound ----
-    if (imL < inL) {
-      if (S[N - 1] < S[imL]) {
-        for (int k = nM - 1; k >= max(nM - NB, 0); --k) r0[c2++] = ind_of(C, 0, nM, NB, k);
-        for (int k = nm - 2; k >= max(nm - NB - 1, 0); --k) r1[c3++] = ind_of(C, 1, nm, NB, k);
-        rsym = inL;
-      } else {
-        r0[c2++] = N - 1;
-        for (int k = max(nM - NB + 1, 0); k < nM; ++k) r0[c2++] = ind_of(C, 0, nM, NB, k);
-        for (int k = nm - 1; k >= max(nm - NB, 0); --k) r1[c3++] = ind_of(C, 1, nm, NB, k);
-        rsym = N - 1;
-      }
-    } else {
-      if (S[N - 1] > S[inL]) {
-        for (int k = nM - 2; k >= max(nM - NB - 1, 0); --k) r0[c2++] = ind_of(C, 0, nM, NB, k);
-        for (int k = nm - 1; k >= max(nm - NB, 0); --k) r1[c3++] = ind_of(C, 1, nm, NB, k);
-        rsym = imL;
-      } else {
-        for (int k = nM - 1; k >= max(nM - NB, 0); --k) r0[c2++] = ind_of(C, 0, nM, NB, k);
-        r1[c3++] = N - 1;
-        for (int k = max(nm - NB + 1, 0); k < nm; ++k) r1[c3++] = ind_of(C, 1, nm, NB, k);
-        rsym = N - 1;
-      }
-    }
-    // An empty list falls back to the whole index list (kernels.py:456-459,
-    // 523-531); that only happens when the side has exactly one extremum,
-    // so the whole list is that one index.
-    if (c0 == 0) l0[c0++] = im0;
-    if (c1 == 0) l1[c1++] = in0;
-    if (c2 == 0) r0[c2++] = imL;
-    if (c3 == 0) r1[c3++] = inL;
-    // ---- mirrored point does not reach the boundary (kernels.py:469-503) ----
-    const real T0 = T(0), TN = T(N - 1);
-    real tl = T(lsym);
-    // the mirrored positions are stored as REAL_T before the compares
-    // (kernels.py:471-472, 488-489): in the FP32 build that rounds them
-    const real tl1 = 2.0 * tl - T(l1[0]), tl0 = 2.0 * tl - T(l0[0]);
-    if (tl1 > T0 || tl0 > T0) {
-      if (lsym == im0) {
-        c0 = 0;
-        for (int k = min(nM, NB) - 1; k >= 0; --k) l0[c0++] = ind_of(C, 0, nM, NB, k);
-      } else {
-        c1 = 0;
-        for (int k = min(nm, NB) - 1; k >= 0; --k) l1[c1++] = ind_of(C, 1, nm, NB, k);
-      }
-      lsym = 0;
-    }
-    real tr = T(rsym);
-    const real tr1 = 2.0 * tr - T(r1[c3 - 1]), tr0 = 2.0 * tr - T(r0[c2 - 1]);
-    if (tr1 < TN || tr0 < TN) {
-      if (rsym == imL) {
-        c2 = 0;
-        for (int k = nM - 1; k >= max(nM - NB, 0); --k) r0[c2++] = ind_of(C, 0, nM, NB, k);
-      } else {
-        c3 = 0;
-        for (int k = nm - 1; k >= max(nm - NB, 0); --k) r1[c3++] = ind_of(C, 1, nm, NB, k);
-      }
-      rsym = N - 1;
-    }
-    C.mcnt[0] = c0; C.mcnt[1] = c1; C.mcnt[2] = c2; C.mcnt[3] = c3;
     C.lsym = lsym;
     C.rsym = rsym;
     C.kbase[0] = NB - c0;
@@ -913,21 +896,19 @@ __device__ __forceinline__ bool mirror_both(const SmemLayout& L, const Knots& K,
     C.kcnt[0] = c0 + nM + c2;
     C.kcnt[1] = c1 + nm + c3;
   }
-  __syncwarp();
-  // lanes write the mirrored knots: entry j of list q (0 lmax, 1 lmin, 2 rmax, 3 rmin)
+  // eight lanes a list write its knots: left maxima, left minima, right ones
+  const int q = lane >> 3, side = q & 1;
+  const bool left = q < 2;
+  const MirrorList l = left ? (side == 0 ? l0 : l1) : (side == 0 ? r0 : r1);
+  const int n = side == 0 ? nM : nm, cnt = l.count();
+  const real sym = T(left ? lsym : rsym);
+  real2* xy = (side == 0 ? K.XY[0] : K.XY[1]) + (left ? NB - cnt : NB + n);
   bool bad = false;
-  for (int ent = lane; ent < 4 * (kMaxNbsym + 1); ent += 32) {
-    int q = ent / (kMaxNbsym + 1), j = ent % (kMaxNbsym + 1);
-    int cq = C.mcnt[q];
-    if (j >= cq) continue;
-    int idx = C.mlist[q][j];
-    int side = q & 1;
-    bool left = q < 2;
-    real pos = 2.0 * T(left ? C.lsym : C.rsym) - T(idx);
-    real val = S[idx];
-    int nside = side == 0 ? nM : nm;
-    int slot = left ? (NB - cq + j) : (NB + nside + j);
-    (side == 0 ? K.XY[0] : K.XY[1])[slot] = real2{pos, val};
+  for (int j = lane & 7; j < cnt; j += 8) {
+    const int idx = left ? left_at(l, side, n, j) : right_at(l, side, n, j);
+    const real val = S[idx];
+    const real pos = 2.0 * sym - T(idx);
+    xy[j] = real2{pos, val};
     bad |= side == 0 ? (val < 0.0) : (val > 0.0);
   }
   return bad;
@@ -936,7 +917,7 @@ __device__ __forceinline__ bool mirror_both(const SmemLayout& L, const Knots& K,
 // ---------------------------------------------------------------------------
 // Not-a-knot spline: reduced system + PCR + moments (kernels.py:607-697).
 // ---------------------------------------------------------------------------
-// the two halves of a pair array
+// position of a knot of a pair array
 struct PairX {
   const real2* p;
   __device__ __forceinline__ real operator[](int i) const { return p[i].x; }
@@ -945,26 +926,6 @@ struct PairY {
   const real2* p;
   __device__ __forceinline__ real operator[](int i) const { return p[i].y; }
 };
-
-__device__ __forceinline__ void setup_row(const real2* xy, int n, int k, int m,
-                                          real& a, real& b, real& c, real& d) {
-  const PairX x{xy};
-  const PairY y{xy};
-  if (k == 0) {
-    real h0 = x[1] - x[0], h1 = x[2] - x[1];
-    real rhs1 = 6.0 * ((y[2] - y[1]) / h1 - (y[1] - y[0]) / h0);
-    a = 0.0; b = h0 + 2.0 * h1; c = h1 - h0; d = h1 * rhs1 / (h0 + h1);
-  } else if (k == m - 1) {
-    real hnm3 = x[n - 2] - x[n - 3], hnm2 = x[n - 1] - x[n - 2];
-    real rhs = 6.0 * ((y[n - 1] - y[n - 2]) / hnm2 - (y[n - 2] - y[n - 3]) / hnm3);
-    a = hnm3 - hnm2; b = 2.0 * hnm3 + hnm2; c = 0.0; d = hnm3 * rhs / (hnm3 + hnm2);
-  } else {
-    int i = k + 1;
-    real h_im1 = x[i] - x[i - 1], h_i = x[i + 1] - x[i];
-    a = h_im1; b = 2.0 * (h_im1 + h_i); c = h_i;
-    d = 6.0 * ((y[i + 1] - y[i]) / h_i - (y[i] - y[i - 1]) / h_im1);
-  }
-}
 
 // One PCR row update (kernels.py:651-668), in the reference's operation order;
 // returns the larger magnitude word of its two multipliers.
@@ -1050,19 +1011,46 @@ __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kb
   const int mt = m0 + m1;
   const real2* xy0 = K.XY[0] + kbase0;
   const real2* xy1 = K.XY[1] + kbase1;
-  unsigned* const range = reinterpret_cast<unsigned*>(C.mcnt);   // free until the next mirroring
+  unsigned* const range = C.range;
   if (tid == 0) {
     range[0] = 0u;
     range[1] = 0xffffffffu;
   }
+  // Rows (kernels.py:613-636): row k has the segments k and k+1 around it, and
+  // each segment's slope serves two rows.  A lane forms one slope and takes
+  // its left neighbour's from the lane below, so a warp's 32 segments give 31
+  // rows and the next 32 start one back: one division a row instead of two.
+  // The end rows have the same right-hand side up to the factor h/(h0+h1).
+  const int z0 = m0 > 0 ? m0 + 1 : 0, zt = z0 + (m1 > 0 ? m1 + 1 : 0);
 #pragma unroll 1
-  for (int r = tid; r < mt; r += NT) {
-    const bool s0 = r < m0;
-    const int k = s0 ? r : r - m0;
-    real a, b, c, d;
-    setup_row(s0 ? xy0 : xy1, s0 ? kcnt0 : kcnt1, k, s0 ? m0 : m1, a, b, c, d);
-    K.ac(0)[r] = real2{a, c};
-    K.bd(0)[r] = real2{b, d};
+  for (int zb = (tid >> 5) * 31; zb < zt; zb += (NT / 32) * 31) {
+    const int z = zb + (tid & 31);
+    const bool s0 = z < z0;
+    const int g = s0 ? z : z - z0, m = s0 ? m0 : m1;          // segment g of a system of m rows
+    real h = real(1), sl = real(0);
+    if (z < zt) {
+      const real2* xy = (s0 ? xy0 : xy1) + g;
+      const real2 p0 = xy[0], p1 = xy[1];
+      h = p1.x - p0.x;
+      const real dy = p1.y - p0.y;
+      bool slow = false;
+      sl = div_nb(dy, h, slow);
+      if (slow) sl = EMDB_DIV_RARE(dy, h);
+    }
+    const real hm = __shfl_up_sync(kFull, h, 1), sm = __shfl_up_sync(kFull, sl, 1);
+    if (z < zt && (tid & 31) != 0 && g > 0) {
+      const int k = g - 1, r = (s0 ? 0 : m0) + k;
+      real a = hm, b = 2.0 * (hm + h), c = h, d = 6.0 * (sl - sm);
+      if (k == 0) {
+        a = 0.0; b = hm + 2.0 * h; c = h - hm;
+        d = EMDB_DIV_RARE(h * d, hm + h);
+      } else if (k == m - 1) {
+        a = hm - h; b = 2.0 * hm + h; c = 0.0;
+        d = EMDB_DIV_RARE(hm * d, hm + h);
+      }
+      K.ac(0)[r] = real2{a, c};
+      K.bd(0)[r] = real2{b, d};
+    }
   }
   __syncthreads();
   EMDB_PH(&C, 2);

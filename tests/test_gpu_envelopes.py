@@ -109,3 +109,23 @@ def test_spacing_past_the_reciprocal_table():
     got = EMDKernelConfig(**cfg).build().run(torch.from_numpy(x[None]).cuda(), None)
     r = O.emd_signal(x, t, O.OracleConfig(**cfg))
     assert got[0][0].cpu().numpy().tobytes() == r.imfs.tobytes()
+
+
+@pytest.mark.parametrize("nbsym", [1, 2, 3, 7, 8])
+@pytest.mark.parametrize("n", [7, 12, 33, 40])
+def test_mirroring_of_few_extrema_equals_the_oracle(n, nbsym):
+    """A handful of extrema per side, fewer and more than nbsym, every order of
+    first and last kind and both sides of the end-sample tests."""
+    import torch
+    from cuda_emd import EMDKernelConfig
+    from oracle import emd_oracle as O
+    rng = np.random.default_rng(100 * n + nbsym)
+    X = rng.normal(size=(120, n))
+    X[::2] = np.cumsum(X[::2], axis=1)               # smoother: fewer extrema
+    X[::5, [0, -1]] *= 8.0                            # end samples beyond their neighbours
+    T = np.arange(n, dtype=np.float64)
+    got = EMDKernelConfig(nbsym=nbsym).build().run_envelope_only(torch.from_numpy(X).cuda(), None)
+    upper, lower = got[0].cpu().numpy(), got[1].cpu().numpy()
+    for i in range(X.shape[0]):
+        u, d = _envelopes(O, X[i], T, nbsym)
+        assert upper[i].tobytes() == u.tobytes() and lower[i].tobytes() == d.tobytes(), i
