@@ -932,18 +932,18 @@ struct PairY {
 __device__ __forceinline__ unsigned pcr_row(const real2* __restrict__ ac,
                                             const real2* __restrict__ bd,
                                             real2* __restrict__ acn, real2* __restrict__ bdn,
-                                            int r, int k, int s, int mq) {
+                                            int r, int k, int s, int mq, int guard) {
   const bool hl = k >= s, hr = k + s < mq;
-  const real2 zero{real(0), real(0)}, one{real(1), real(0)};
+  const int rl = hl ? r - s : guard, rr = hr ? r + s : guard;
   const real2 o = ac[r], p = bd[r];
-  const real2 pl = hl ? bd[r - s] : one, pr = hr ? bd[r + s] : one;
-  const real2 ol = hl ? ac[r - s] : zero, orr = hr ? ac[r + s] : zero;
+  const real2 pl = bd[rl], pr = bd[rr];
+  const real2 ol = ac[rl], orr = ac[rr];
   bool sl = false, sr = false;
   const real ql = div_nb(o.x, pl.x, sl);
   const real qr = div_nb(o.y, pr.x, sr);
   real alpha = hl ? ql : real(0);
   real beta = hr ? qr : real(0);
-  if ((hl && sl) || (hr && sr)) {
+  if (sl || sr) {
     alpha = hl ? EMDB_DIV_RARE(o.x, pl.x) : real(0);
     beta = hr ? EMDB_DIV_RARE(o.y, pr.x) : real(0);
   }
@@ -1015,6 +1015,8 @@ __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kb
   if (tid == 0) {
     range[0] = 0u;
     range[1] = 0xffffffffu;
+    K.ac(0)[mt] = K.ac(1)[mt] = real2{real(0), real(0)};
+    K.bd(0)[mt] = K.bd(1)[mt] = real2{real(1), real(0)};
   }
   // Rows (kernels.py:613-636): row k has the segments k and k+1 around it, and
   // each segment's slope serves two rows.  A lane forms one slope and takes
@@ -1071,7 +1073,7 @@ __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kb
     for (int r = tid; r < mt; r += NT) {
       const bool s0 = r < m0;
       mult = max(mult, pcr_row(K.ac(cur), K.bd(cur), K.ac(cur ^ 1), K.bd(cur ^ 1), r,
-                               s0 ? r : r - m0, s, s0 ? m0 : m1));
+                               s0 ? r : r - m0, s, s0 ? m0 : m1, mt));
       if (vote) {
         const real2 p = K.bd(cur ^ 1)[r];
         dmax = max(dmax, mag(p.y));
