@@ -25,12 +25,17 @@
 //    strided lanes + halving tree) and this file is compiled with
 //    -fmad=false, so every value equals the reference algorithm's FP64
 //    result bit for bit (the CPU oracle checks this);
-//  * every quotient is the IEEE one, but most are formed without the
-//    hardware division's slow-path branch: Markstein corrections from a
-//    reciprocal (RN(1/h) from a compile-time table on the integer time axis,
-//    where one correction is exact for integer operands), and for the PCR
-//    rows a branch-free division from the approximate reciprocal; each
-//    redoes its operation with the division outside the exact ranges.
+//  * every quotient is the IEEE one, but those of the hot loops are formed
+//    without the division's slow-path branch, by Markstein corrections from a
+//    reciprocal (one correction is exact for the integer operands of the
+//    integer time axis) or the approximate one (the PCR rows); a vote per
+//    pass makes sure that their operands are in the exact ranges, and other
+//    passes divide;
+//  * one trace's pass is a chain of short phases between barriers, four
+//    traces share an SM, and the code of a pass is as large as the 32 KB
+//    instruction cache (straight-line code past 2048 instructions runs at half
+//    the rate here with 16 warps): loops are kept rolled, rare paths are out
+//    of line with one call site each, and range tests are taken out of loops.
 //
 // Per-pass knot/PCR storage is placed by size: all in the CTA's shared-
 // memory arena; "borrow" (the proto-IMF parked in the per-CTA global slab
@@ -45,9 +50,6 @@
 #include "emdb_internal.cuh"
 
 // Tuning knobs (compile-time; results are identical for every setting):
-//  EMDB_OUTLINE    rarely taken paths as calls instead of inline copies:
-//                  1 the general evaluation and the binary segment search,
-//                  2 also the IEEE-division fallbacks of the PCR and setup rows
 // Settled: one sift-pass instance for the on-chip placements and one for the
 // off-chip ones (16,384 x 2048 seismic 208.4k signals/s; one instance for all
 // 195.6k, one per placement 184.9k), the six end-of-pass trees spread over the
@@ -61,9 +63,6 @@
 //                  on the first 128 threads only (no split): 293.0 / 46.7.
 #ifndef EMDB_LANE_UNROLL
 #define EMDB_LANE_UNROLL 16
-#endif
-#ifndef EMDB_OUTLINE
-#define EMDB_OUTLINE 2
 #endif
 //  EMDB_LOAD_CLOCKS  instrumented build: thread 0 of each CTA adds the clock64
 //                  cycles of every trace's load into shared memory, of the
@@ -94,10 +93,10 @@ constexpr int kPhases = 10;
 // the sift computes is a `real`; the reference kernel's double literals keep
 // their C++ meaning, so float expressions that mix them are evaluated in
 // double and rounded once, as in the reference source compiled with REAL_T =
-// float.  The FP64 build's branch-free quotients have float counterparts
-// (div_q from an IEEE reciprocal for the segment quotients, div_nb for the PCR
-// rows), self-tested against the float division by emdb_check_division modes 3
-// and 4; the one double quotient per envelope sample (the reference's "/ 6.0")
+// float.  The segment quotients have a float counterpart of the FP64 ones (div_q
+// from an IEEE reciprocal), self-tested against the float division by
+// emdb_check_division mode 3 (mode 4: div_nb, for which the PCR rows no longer
+// have a use); the one double quotient per envelope sample (the reference's "/ 6.0")
 // is formed from RN(1/6) and its residual (div6), which equals the double
 // division.
 #ifndef EMDB_F32
@@ -135,8 +134,7 @@ struct Ctl {
   int job;
   int head[2][kMaxNbsym + 1];  // first NB+1 extrema indices per side (0 = max, 1 = min)
   int tail[2][kMaxNbsym + 1];  // tail[q][k] = index of extremum n_q-1-k
-  unsigned range[2];           // largest / smallest right-hand side during the solve
-  int unused[38];              // keeps the block's size: it decides the longest trace a CTA takes
+  int unused[40];              // keeps the block's size: it decides the longest trace a CTA takes
   int lsym, rsym;
   int kbase[2], kcnt[2];
   int dbg_n[kMaxImfsCap], dbg_e[kMaxImfsCap], dbg_z[kMaxImfsCap];
@@ -177,16 +175,23 @@ struct SmemLayout {
   int arena_bytes;    // bytes left for the knot arena
 };
 
-__host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
+// sizes: size_t on the host (a query must not wrap for any int input), 32 bits
+// in the kernel, where the launch has checked that they fit
+#ifdef __CUDA_ARCH__
+using usize = unsigned;
+#else
+using usize = size_t;
+#endif
+__host__ __device__ inline usize align16(usize x) { return (x + 15) & ~usize(15); }
 
 // NT: threads per CTA (128, or 512 for the wide instance).  kGImf: the
 // proto-IMF lives in the CTA's global slab instead of shared memory (traces
 // longer than shared memory holds); it then takes no shared memory.
 template <int NT = kThreads, bool kGImf = false>
-__host__ __device__ inline size_t fixed_bytes(int N) {
-  size_t nch = (size_t)(N + 31) / 32;
-  size_t b = align16(sizeof(Ctl)) + align16(5 * (NT / 32) * sizeof(int));
-  if (!kGImf) b += align16((size_t)N * sizeof(real));
+__host__ __device__ inline usize fixed_bytes(int N) {
+  usize nch = (usize)(N + 31) / 32;
+  usize b = align16(sizeof(Ctl)) + align16(5 * (NT / 32) * sizeof(int));
+  if (!kGImf) b += align16((usize)N * sizeof(real));
   b += align16(nch * 4) * 2 + align16(nch * 2) * 2;
   return b;
 }
@@ -195,7 +200,7 @@ template <int NT = kThreads, bool kGImf = false>
 __device__ __forceinline__ SmemLayout carve(char* base, int N, int arena_total,
                                             real* gimf = nullptr) {
   SmemLayout L;
-  size_t nch = (size_t)(N + 31) / 32;
+  usize nch = (usize)(N + 31) / 32;
   char* p = base;
   L.ctl = reinterpret_cast<Ctl*>(p); p += align16(sizeof(Ctl));
   L.wc = reinterpret_cast<uint4*>(p); p += align16(5 * (NT / 32) * sizeof(int));
@@ -206,7 +211,7 @@ __device__ __forceinline__ SmemLayout carve(char* base, int N, int arena_total,
   if (kGImf) {
     L.imf = gimf;
   } else {
-    L.imf = reinterpret_cast<real*>(p); p += align16((size_t)N * sizeof(real));
+    L.imf = reinterpret_cast<real*>(p); p += align16((usize)N * sizeof(real));
   }
   L.arena = p;
   L.red = reinterpret_cast<real*>(p);
@@ -215,25 +220,28 @@ __device__ __forceinline__ SmemLayout carve(char* base, int N, int arena_total,
 }
 
 // Knot / PCR storage for one sift pass (both envelopes).  A PCR buffer holds
-// each row's off-diagonals as (a, c) pairs, then its (b, d) pairs, one 16-byte
-// word each.  The spline moments M take the place of buffer 0's (a, c) pairs,
-// which nothing reads any more by then.
+// blocks of eight rows: their (a, c) pairs, then their (b, d) pairs, so one
+// address serves both halves of a row and eight consecutive rows of either
+// half cover all banks once.  It has room for `cap` rows; the two systems take
+// at most cap - 8 (an envelope has at most its extrema plus 2 nbsym knots),
+// which leaves a row for the neighbour of rows that have none and the last
+// block's padding.  The spline moments M take the place of buffer 0, whose
+// rows nothing reads any more by then.
 struct Knots {
   real2* XY[2]; // (position, value) of each knot
   real* M[2];
-  real* P[2];   // ping-pong PCR buffers: (a, c) | (b, d), each `cap` rows
+  real* P[2];   // ping-pong PCR buffers, each `cap` rows
   real* red;    // reduction lanes after the solve: buffer 1, or just past it
   int cap;
-  __device__ __forceinline__ real2* ac(int q) const { return reinterpret_cast<real2*>(P[q]); }
-  __device__ __forceinline__ real2* bd(int q) const {
-    return reinterpret_cast<real2*>(P[q] + 2 * cap);
+  __device__ __forceinline__ char* rows(int q) const {
+    return reinterpret_cast<char*>(q ? P[1] : P[0]);
   }
 };
 
-__host__ __device__ inline size_t knot_bytes(int kc0, int kc1) {
-  // size_t throughout: a host-side size query must not wrap for any int input
-  const size_t cap = (size_t)kc0 + (size_t)kc1;
-  const size_t red_extra = (4 * cap >= (size_t)kRedDoubles) ? 0 : kRedBytes;
+__host__ __device__ inline usize knot_bytes(int kc0, int kc1) {
+  // usize throughout: a host-side size query must not wrap for any int input
+  const usize cap = (usize)kc0 + (usize)kc1;
+  const usize red_extra = (4 * cap >= (usize)kRedDoubles) ? 0 : kRedBytes;
   return (2 * cap + 8 * cap) * sizeof(real) + red_extra;
 }
 
@@ -256,8 +264,8 @@ __device__ __forceinline__ Knots place_knots(char* base, int kc0, int kc1) {
 // second PCR buffer: knots X | Y and PCR buffer 0 (which ends up holding the
 // moments) in the arena, buffer 1 in the per-CTA global slab.  Evaluation then
 // reads shared memory only, and half of the PCR levels read the slab.
-__host__ __device__ inline size_t split_bytes(int kc0, int kc1) {
-  return 6 * ((size_t)kc0 + (size_t)kc1) * sizeof(real);
+__host__ __device__ inline usize split_bytes(int kc0, int kc1) {
+  return 6 * ((usize)kc0 + (usize)kc1) * sizeof(real);
 }
 
 __device__ __forceinline__ Knots place_knots_split(char* sbase, int sbytes, char* gbase, int kc0,
@@ -274,7 +282,7 @@ __device__ __forceinline__ Knots place_knots_split(char* sbase, int sbytes, char
   K.M[1] = K.P[0] + kc0;
   // reduction lanes: shared memory past buffer 0 when they fit, else the slab
   // (buffer 1 is dead after the solve; the slab holds knot_bytes of the largest pass)
-  if (split_bytes(kc0, kc1) + kRedBytes <= (size_t)sbytes) K.red = p;
+  if (split_bytes(kc0, kc1) + kRedBytes <= (usize)sbytes) K.red = p;
   else K.red = (4 * K.cap >= kRedDoubles) ? K.P[1] : K.P[1] + 4 * K.cap;
   return K;
 }
@@ -285,13 +293,13 @@ __device__ __forceinline__ Knots place_knots_split(char* sbase, int sbytes, char
 // ahead of the knots), and X | Y | buffer 0 sit at the end of the arena, clear
 // of the proto-IMF that the knot fill reads.  Evaluation reads the old sample
 // values back from the slab; the reduction lanes go to the slab after them.
-__host__ __device__ inline bool borrow_fits(int N, int arena_bytes, size_t slab_stride, int kc0,
+__host__ __device__ inline bool borrow_fits(int N, int arena_bytes, usize slab_stride, int kc0,
                                             int kc1) {
-  const size_t cap = (size_t)kc0 + (size_t)kc1;
-  const size_t region = align16((size_t)N * sizeof(real)) + (size_t)arena_bytes;
-  return 6 * cap * sizeof(real) <= (size_t)arena_bytes &&
+  const usize cap = (usize)kc0 + (usize)kc1;
+  const usize region = align16((usize)N * sizeof(real)) + (usize)arena_bytes;
+  return 6 * cap * sizeof(real) <= (usize)arena_bytes &&
          10 * cap * sizeof(real) <= region &&
-         (align16((size_t)N * sizeof(real)) + kRedBytes) <= slab_stride;
+         (align16((usize)N * sizeof(real)) + kRedBytes) <= slab_stride;
 }
 
 __device__ __forceinline__ real* borrow_save(char* slab) { return reinterpret_cast<real*>(slab); }
@@ -308,7 +316,7 @@ __device__ __forceinline__ Knots place_knots_borrow(real* imf, char* arena, int 
   K.P[1] = imf;
   K.M[0] = K.P[0];
   K.M[1] = K.P[0] + kc0;
-  K.red = reinterpret_cast<real*>(slab + align16((size_t)N * sizeof(real)));
+  K.red = reinterpret_cast<real*>(slab + align16((usize)N * sizeof(real)));
   return K;
 }
 
@@ -319,13 +327,13 @@ __device__ __forceinline__ Knots place_knots_borrow(real* imf, char* arena, int 
 // (parked in the slab, as for the borrow placement).  Everything stays
 // on-chip; the arena needs 3 doubles per knot slot instead of 6, the region
 // 11 instead of 10.
-__host__ __device__ inline bool borrow2_fits(int N, int arena_bytes, size_t slab_stride, int kc0,
+__host__ __device__ inline bool borrow2_fits(int N, int arena_bytes, usize slab_stride, int kc0,
                                              int kc1) {
-  const size_t cap = (size_t)kc0 + (size_t)kc1;
-  const size_t region = align16((size_t)N * sizeof(real)) + (size_t)arena_bytes;
-  return 3 * cap * sizeof(real) <= (size_t)arena_bytes &&
+  const usize cap = (usize)kc0 + (usize)kc1;
+  const usize region = align16((usize)N * sizeof(real)) + (usize)arena_bytes;
+  return 3 * cap * sizeof(real) <= (usize)arena_bytes &&
          11 * cap * sizeof(real) <= region &&
-         (align16((size_t)N * sizeof(real)) + kRedBytes) <= slab_stride;
+         (align16((usize)N * sizeof(real)) + kRedBytes) <= slab_stride;
 }
 
 __device__ __forceinline__ Knots place_knots_borrow2(real* imf, char* arena, int arena_bytes,
@@ -340,7 +348,7 @@ __device__ __forceinline__ Knots place_knots_borrow2(real* imf, char* arena, int
   K.XY[1] = K.XY[0] + kc0;
   K.P[0] = imf;
   K.P[1] = imf + 4 * K.cap;
-  K.red = reinterpret_cast<real*>(slab + align16((size_t)N * sizeof(real)));
+  K.red = reinterpret_cast<real*>(slab + align16((usize)N * sizeof(real)));
   return K;
 }
 
@@ -352,11 +360,11 @@ __device__ __forceinline__ Knots place_knots_borrow2(real* imf, char* arena, int
 // then read shared memory; the evaluation reads the knots and the old samples
 // from the slab.  The reduction lanes use the arena start, free after the
 // solve.
-__host__ __device__ inline bool park_fits(int N, int arena_bytes, size_t slab_stride, int kc0,
+__host__ __device__ inline bool park_fits(int N, int arena_bytes, usize slab_stride, int kc0,
                                           int kc1) {
-  const size_t cap = (size_t)kc0 + (size_t)kc1;
-  const size_t imfb = align16((size_t)N * sizeof(real));
-  return 4 * cap * sizeof(real) <= imfb + (size_t)arena_bytes &&
+  const usize cap = (usize)kc0 + (usize)kc1;
+  const usize imfb = align16((usize)N * sizeof(real));
+  return 4 * cap * sizeof(real) <= imfb + (usize)arena_bytes &&
          imfb + 6 * cap * sizeof(real) <= slab_stride;
 }
 
@@ -364,7 +372,7 @@ __device__ __forceinline__ Knots place_knots_park(real* imf, char* slab, int N, 
                                                   real* red) {
   Knots K;
   K.cap = kc0 + kc1;
-  real* p = reinterpret_cast<real*>(slab + align16((size_t)N * sizeof(real)));
+  real* p = reinterpret_cast<real*>(slab + align16((usize)N * sizeof(real)));
   K.XY[0] = reinterpret_cast<real2*>(p);
   K.XY[1] = K.XY[0] + kc0;
   p += 2 * (kc0 + kc1);
@@ -384,18 +392,18 @@ enum : int { kOnChip = -1, kOffChip = -2, kAnyPlace = -3 };
 // that fits, the on-chip ones first (shared, borrow, compact borrow), then
 // split, park, slab.  `arena_bytes` is the knot arena left after the fixed
 // part (control block, scan masks, proto-IMF); the slab always fits.
-__host__ __device__ inline int choose_place(int N, int arena_bytes, size_t slab_stride, int kc0,
+__host__ __device__ inline int choose_place(int N, int arena_bytes, usize slab_stride, int kc0,
                                             int kc1, bool imf_global = false) {
   // a proto-IMF in global memory has no shared-memory region to lend: only
   // the placements that leave it alone
   if (imf_global)
-    return knot_bytes(kc0, kc1) <= (size_t)arena_bytes ? kPlaceSmem
-         : split_bytes(kc0, kc1) <= (size_t)arena_bytes ? kPlaceSplit
+    return knot_bytes(kc0, kc1) <= (usize)arena_bytes ? kPlaceSmem
+         : split_bytes(kc0, kc1) <= (usize)arena_bytes ? kPlaceSplit
                                                         : kPlaceSlab;
-  return knot_bytes(kc0, kc1) <= (size_t)arena_bytes ? kPlaceSmem
+  return knot_bytes(kc0, kc1) <= (usize)arena_bytes ? kPlaceSmem
        : borrow_fits(N, arena_bytes, slab_stride, kc0, kc1) ? kPlaceBorrow
        : borrow2_fits(N, arena_bytes, slab_stride, kc0, kc1) ? kPlaceBorrow2
-       : split_bytes(kc0, kc1) <= (size_t)arena_bytes ? kPlaceSplit
+       : split_bytes(kc0, kc1) <= (usize)arena_bytes ? kPlaceSplit
        : park_fits(N, arena_bytes, slab_stride, kc0, kc1) ? kPlacePark
                                                           : kPlaceSlab;
 }
@@ -412,9 +420,6 @@ __host__ __device__ inline int choose_place(int N, int arena_bytes, size_t slab_
 // infinite or NaN, as a/b would be).  Checked bit for bit against the hardware
 // division by emdb_check_division.
 //
-// div_q returns the quotient without branching and sets `slow` for operands
-// outside that range, so a caller can redo a whole sample with the division
-// once instead of branching on every quotient.
 __device__ __noinline__ double div_slow(double a, double b) { return a / b; }
 
 #if EMDB_F32
@@ -461,35 +466,12 @@ __device__ __forceinline__ float div_nb(float a, float b, bool& slow) {
 }
 #endif
 
-// Rarely taken paths of the hot loops (fewer than 4 knots, operands outside
-// the fast quotients' range, knot lists that are not strictly increasing) as
-// calls to one out-of-line body each, instead of an inline copy per call site:
-// keeps the hot loops' code small.  Defined after eval_seg / search_seg.
-__device__ __noinline__ real eval_seg_cold(const real2* xy, const real* M, int n, real t, int lo);
-__device__ __noinline__ int search_seg_cold(const real2* xy, int n, real t);
-#if EMDB_OUTLINE >= 1
-#define EMDB_EVAL_RARE(sv, t, lo) eval_seg_cold((sv).xy, (sv).M, (sv).n, (t), (lo))
-#define EMDB_SEARCH_RARE(sv, t) search_seg_cold((sv).xy, (sv).n, (t))
-#else
-#define EMDB_EVAL_RARE(sv, t, lo) eval_seg((sv), (t), (lo))
-#define EMDB_SEARCH_RARE(sv, t) search_seg((sv), (t))
-#endif
-#if EMDB_OUTLINE >= 2
-#define EMDB_DIV_RARE(a, b) div_slow((a), (b))
-#else
-#define EMDB_DIV_RARE(a, b) ((a) / (b))
-#endif
-
-__device__ __forceinline__ double div_q(double a, double b, double y, bool& slow) {
-  const double q0 = a * y;
-  const double e0 = fma(-q0, b, a);
-  const double q1 = fma(e0, y, q0);
-  const double e1 = fma(-q1, b, a);
-  const double q2 = fma(e1, y, q1);
-  const double aa = fabs(a), qa = fabs(q0);
-  const bool zero = a == 0.0;
-  slow |= !(zero || (aa > 0x1p-900 && aa < 0x1p+900 && qa > 0x1p-900 && qa < 0x1p+900));
-  return zero ? q0 : q2;
+// The two corrections without the tests, for a numerator of zero or in range
+// (a negative zero gives +0).
+__device__ __forceinline__ double quot(double a, double b, double y) {
+  double q = a * y;
+  q = fma(fma(-q, b, a), y, q);
+  return fma(fma(-q, b, a), y, q);
 }
 
 #if !EMDB_F32
@@ -507,17 +489,31 @@ __device__ __forceinline__ double div_q(double a, double b, double y, bool& slow
 // 2^-53 / m_b ulp(q) to a rounding boundary without lying on it, and never
 // lies on it, so the last FMA rounds as the division does.
 //
-// `slow` is set unless |a|, |b| and |q| are in [2^-511, 2^512), where no step
-// underflows or overflows: exponent fields 512..1535 are those whose two top
-// bits differ, i.e. whose high word plus 2^29 has bit 30 set.  A zero
-// numerator gives q0 = a*y, the correctly signed zero, and needs only b.
-// 10 FP64 operations and integer checks; the form before it (two linear
-// steps, a neighbour choice by two exact remainders and range compares on the
-// doubles) took 8 and 11 compares, which cost as much as arithmetic.
+// div_nb, the form that emdb_check_division tests, sets `slow` unless |a|, |b|
+// and |q| are in [2^-511, 2^512), where no step underflows or overflows:
+// exponent fields 512..1535 are those whose two top bits differ, i.e. whose
+// high word plus 2^29 has bit 30 set.  The PCR rows make sure of their
+// operands beforehand (solve_splines).
+// 10 FP64 operations; the form before it (two linear steps, a neighbour choice
+// by two exact remainders and range compares on the doubles) took 8 and 11
+// compares, which cost as much as arithmetic.
 __device__ __forceinline__ unsigned range_bits(double x) {
   return (unsigned)__double2hiint(x) + 0x20000000u;
 }
-__device__ __forceinline__ double div_nb(double a, double b, bool& slow) {
+// 1/b to within (1/2 + 2^-51) ulp; RN(1/b) for an integer b up to 65536, which
+// is never that close to the middle of two doubles (checked for each by
+// emdb_check_division mode 0).
+__device__ __forceinline__ double recip(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  double e = fma(-b, y, 1.0);
+  e = fma(e, e, e);
+  y = fma(e, y, y);
+  e = fma(-b, y, 1.0);
+  return fma(e, y, y);
+}
+// The quotient without its range checks (+0 for any zero numerator).
+__device__ __forceinline__ double div_core(double a, double b) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
   double e = fma(-b, y, 1.0);
@@ -529,11 +525,12 @@ __device__ __forceinline__ double div_nb(double a, double b, bool& slow) {
   const double r0 = fma(-q0, b, a);
   const double q1 = fma(r0, y, q0);
   const double r1 = fma(-q1, b, a);
-  const double q2 = fma(r1, y, q1);
-  const bool zero = a == 0.0;
-  const unsigned aq = range_bits(a) & range_bits(q2);
-  slow |= !(range_bits(b) & (zero ? 0x40000000u : aq) & 0x40000000u);
-  return zero ? q0 : q2;
+  return fma(r1, y, q1);
+}
+__device__ __forceinline__ double div_nb(double a, double b, bool& slow) {
+  const double q = div_core(a, b);
+  slow |= !(range_bits(a) & range_bits(b) & range_bits(q) & 0x40000000u);
+  return q;
 }
 #endif
 // high word of |x|: orders magnitudes, and (as a fixed-point number with 20
@@ -546,10 +543,12 @@ __device__ __forceinline__ unsigned mag(float x) {
 }
 
 #if !EMDB_F32
+// with the tests, for emdb_check_division
 __device__ __forceinline__ double div_rn(double a, double b, double y) {
-  bool slow = false;
-  const double q = div_q(a, b, y, slow);
-  return slow ? div_slow(a, b) : q;
+  const double q = quot(a, b, y), aa = fabs(a), qa = fabs(q);
+  if (a == 0.0) return a * y;
+  const bool in = aa > 0x1p-900 && aa < 0x1p+900 && qa > 0x1p-900 && qa < 0x1p+900;
+  return in ? q : div_slow(a, b);
 }
 #endif
 
@@ -569,22 +568,19 @@ __device__ __forceinline__ bool odd_range(double x) {
   // exponents [-900, 900): biased 123..1922
   return (v - (123u << 20)) >= (1800u << 20) && (v | (unsigned)__double2loint(x)) != 0u;
 }
+__device__ __forceinline__ double div6(double x) { return fma(x, kInv6, x * kInv6Lo); }
 __device__ __forceinline__ double div6(double x, bool& slow) {
   slow |= odd_range(x);
-  return fma(x, kInv6, x * kInv6Lo);
+  return div6(x);
+}
+// a moment that is neither zero nor in [2^-700, 2^900) (biased exponents 323..1922)
+__device__ __forceinline__ bool odd_moment(double m) {
+  const unsigned v = (unsigned)__double2hiint(m) & 0x7fffffffu;
+  return v - (323u << 20) >= (1600u << 20) && (v | (unsigned)__double2loint(m)) != 0u;
 }
 
-// RN(1/h) for integer h in [1, kRcpTab], built at compile time by IEEE
-// division and shipped initialised in the module.
-constexpr int kRcpTab = 16384;
-struct RcpTab { double v[kRcpTab + 1]; };
-constexpr RcpTab make_rcp_tab() {
-  RcpTab t{};
-  for (int h = 1; h <= kRcpTab; ++h) t.v[h] = 1.0 / (double)h;
-  return t;
-}
-__device__ const RcpTab g_rcp = make_rcp_tab();
-
+// longest integer segment that eval_seg_int takes
+constexpr int kMaxIntSeg = 65536;
 
 struct TimeAxis {
   const real* T;
@@ -634,6 +630,7 @@ __device__ __forceinline__ void extrema_count(const SmemLayout& L, int N, int sl
       if (interior && dn == real(0) && dp != real(0)) {
         // rare: true left edge of a flat run, classified by the slopes around it
         int j = i;
+#pragma unroll 1
         while (j + 1 < N && imf[j + 1] == v) ++j;
         if (j + 1 < N) {
           const real da = imf[j + 1] - imf[j];
@@ -704,6 +701,7 @@ __device__ void chunk_fallback_check(const SmemLayout& L, int N, int tid) {
   int start = tid * cs, end = min(start + cs, N);
   int lo = max(start, 1), hi = min(end, N - 1);
   int nmx = 0, nmn = 0;
+#pragma unroll 1
   for (int i = lo; i < hi; ++i) {
     real dp = s[i] - s[i - 1], dn = s[i + 1] - s[i];
     if (dp * dn < 0.0) { if (dp < 0.0) ++nmn; else ++nmx; }
@@ -761,38 +759,32 @@ __device__ __forceinline__ bool fill_true_knots(const SmemLayout& L, const Knots
       if (fe <= NB) C.tail[q][fe] = ii;
     }
   };
-  if (!e.trig) {
-    // no exact zeros or flat runs in this proto-IMF: every extremum is strict
 #pragma unroll (NS == kWarps ? 1 : 2)
-    for (int c = c0; c < c1; ++c) {
-      const uint32_t bm = L.mm[c].x, bn = L.mm[c].y;
-      const int pm = L.pp[c] & 0xffff, pn = L.pp[c] >> 16;
-      if (((bm | bn) >> lane) & 1u) {
-        const int i = (c << 5) + lane;
-        put(bm, bn, pm, pn, i, imf[i]);
+  for (int c = c0; c < c1; ++c) {
+    const uint2 m = L.mm[c];
+    const uint32_t pp = L.pp[c];
+    if (((m.x | m.y) >> lane) & 1u) {
+      int ii = (c << 5) + lane;
+      real v = imf[ii];
+      if (e.trig) {
+        // a proto-IMF with exact zeros or flat runs: a plateau extremum reports
+        // the run's midpoint
+        const real dp = v - imf[ii - 1], dn = imf[ii + 1] - v;
+        if (!(dp * dn < 0.0)) {
+          int j = ii;
+#pragma unroll 1
+          while (j + 1 < N && imf[j + 1] == v) ++j;
+          ii = (ii + j) / 2;
+          v = imf[ii];
+        }
       }
-    }
-  } else {
-    for (int c = c0; c < c1; ++c) {
-      const uint32_t bm = L.mm[c].x, bn = L.mm[c].y;
-      const int pm = L.pp[c] & 0xffff, pn = L.pp[c] >> 16;
-      if (!(((bm | bn) >> lane) & 1u)) continue;
-      int i = (c << 5) + lane;
-      int ii = i;
-      real v = imf[i];
-      real dp = v - imf[i - 1], dn = imf[i + 1] - v;
-      if (!(dp * dn < 0.0)) {       // plateau extremum: report the run's midpoint
-        int j = i;
-        while (j + 1 < N && imf[j + 1] == v) ++j;
-        ii = (i + j) / 2;
-        v = imf[ii];
-      }
-      put(bm, bn, pm, pn, ii, v);
+      put(m.x, m.y, pp & 0xffff, pp >> 16, ii, v);
     }
   }
   // the chunks' prefixes become global (warp offset added) for the evaluation
   // pass's segment counts, once every lane has taken its ranks
   __syncwarp();
+#pragma unroll 1
   for (int c = c0 + lane; c < c1; c += 32) L.pp[c] += e.off;
   return bad;
 }
@@ -904,6 +896,7 @@ __device__ __forceinline__ bool mirror_both(const SmemLayout& L, const Knots& K,
   const real sym = T(left ? lsym : rsym);
   real2* xy = (side == 0 ? K.XY[0] : K.XY[1]) + (left ? NB - cnt : NB + n);
   bool bad = false;
+#pragma unroll 1
   for (int j = lane & 7; j < cnt; j += 8) {
     const int idx = left ? left_at(l, side, n, j) : right_at(l, side, n, j);
     const real val = S[idx];
@@ -927,51 +920,81 @@ struct PairY {
   __device__ __forceinline__ real operator[](int i) const { return p[i].y; }
 };
 
-// One PCR row update (kernels.py:651-668), in the reference's operation order;
-// returns the larger magnitude word of its two multipliers.
-__device__ __forceinline__ unsigned pcr_row(const real2* __restrict__ ac,
-                                            const real2* __restrict__ bd,
-                                            real2* __restrict__ acn, real2* __restrict__ bdn,
-                                            int r, int k, int s, int mq, int guard) {
-  const bool hl = k >= s, hr = k + s < mq;
-  const int rl = hl ? r - s : guard, rr = hr ? r + s : guard;
-  const real2 o = ac[r], p = bd[r];
-  const real2 pl = bd[rl], pr = bd[rr];
-  const real2 ol = ac[rl], orr = ac[rr];
-  bool sl = false, sr = false;
-  const real ql = div_nb(o.x, pl.x, sl);
-  const real qr = div_nb(o.y, pr.x, sr);
-  real alpha = hl ? ql : real(0);
-  real beta = hr ? qr : real(0);
-  if (sl || sr) {
-    alpha = hl ? EMDB_DIV_RARE(o.x, pl.x) : real(0);
-    beta = hr ? EMDB_DIV_RARE(o.y, pr.x) : real(0);
+// Row r of a PCR buffer: byte offset of its (a, c) pair; its (b, d) pair
+// follows kBD bytes on.
+constexpr int kRow = (int)sizeof(real2), kBD = 8 * kRow;
+__device__ __forceinline__ int row_at(int r) { return (r >> 3) * (2 * kBD) + (r & 7) * kRow; }
+// Byte distance to the row `s` below / above a row that is number r & 7 of its block
+__device__ __forceinline__ int row_below(int r, int s) {
+  return s < 8 ? s * kRow + ((r & 7) < s ? kBD : 0) : 2 * s * kRow;
+}
+__device__ __forceinline__ int row_above(int r, int s) {
+  return s < 8 ? s * kRow + ((r & 7) + s >= 8 ? kBD : 0) : 2 * s * kRow;
+}
+__device__ __forceinline__ real2& pair_at(char* p) { return *reinterpret_cast<real2*>(p); }
+__device__ __forceinline__ const real2& pair_at(const char* p) {
+  return *reinterpret_cast<const real2*>(p);
+}
+
+// The PCR levels from stride s on with the division itself, rows of two systems
+// in buffer `cur` (kernels.py:651-668, in the reference's operation order);
+// the result ends up in buffer 1.  The whole CTA calls it, for the systems that
+// the levels in solve_splines do not cover.
+template <int NT>
+__device__ __noinline__ void pcr_levels_any(char* b0, char* b1, int m0, int m1, int s, int cur) {
+  const int tid = threadIdx.x, mt = m0 + m1, guard = row_at(mt);
+#pragma unroll 1
+  for (; s < max(m0, m1); s *= 2) {
+    const char* src = cur ? b1 : b0;
+    char* dst = cur ? b0 : b1;
+#pragma unroll 1
+    for (int r = tid; r < mt; r += NT) {
+      const bool s0 = r < m0;
+      const bool hl = (s0 && r >= s) || r >= m0 + s;
+      const bool hr = r < m0 - s || (!s0 && r < mt - s);
+      const char* own = src + row_at(r);
+      const char* l = src + (hl ? row_at(r - s) : guard);
+      const char* rr = src + (hr ? row_at(r + s) : guard);
+      const real2 o = pair_at(own), p = pair_at(own + kBD);
+      const real2 ol = pair_at(l), pl = pair_at(l + kBD);
+      const real2 orr = pair_at(rr), pr = pair_at(rr + kBD);
+      const real alpha = hl ? o.x / pl.x : real(0);
+      const real beta = hr ? o.y / pr.x : real(0);
+      char* to = dst + row_at(r);
+      pair_at(to) = real2{-alpha * ol.x, -beta * orr.y};
+      pair_at(to + kBD) = real2{p.x - alpha * ol.y - beta * orr.x,
+                                p.y - alpha * pl.y - beta * pr.y};
+    }
+    cur ^= 1;
+    __syncthreads();
   }
-  acn[r] = real2{-alpha * ol.x, -beta * orr.y};
-  bdn[r] = real2{p.x - alpha * ol.y - beta * orr.x, p.y - alpha * pl.y - beta * pr.y};
-  return max(mag(alpha), mag(beta));
+  if (cur == 0) {
+#pragma unroll 1
+    for (int r = tid; r < mt; r += NT) {
+      const int at = row_at(r);
+      pair_at(b1 + at + kBD) = pair_at(b0 + at + kBD);
+    }
+    __syncthreads();
+  }
 }
 
 // The last PCR level of a system whose multipliers have died out (see
-// solve_splines), for row k (index r): the right-hand side after it, d.  The
-// diagonal stays as it is.  A neighbour's term is formed only where it can
+// solve_splines): the right-hand side after it, d.  The diagonal stays as it
+// is.  A neighbour's term is formed only where it can
 // reach the rounding of d: RN(d - x) = d for |x| below a quarter ulp, and the
 // magnitude words bound |a d_l| against |d b_l| from both sides (each is at
 // most 0.0861 below its logarithm).
-__device__ __forceinline__ real pcr_last(const real2* ac, const real2* bd, int r, int k, int s,
-                                         int mq) {
+__device__ __forceinline__ real pcr_last(const char* own, const char* l, const char* r, bool hl,
+                                         bool hr) {
   constexpr int kFrac = sizeof(real) == 8 ? 20 : 23;
   constexpr int kGap = ((sizeof(real) == 8 ? 55 : 26) << kFrac) + (1 << kFrac) / 4;
-  const real2 o = ac[r];
-  const bool hl = k >= s, hr = k + s < mq;
-  const real2 pl = hl ? bd[r - s] : real2{real(1), real(0)};
-  const real2 pr = hr ? bd[r + s] : real2{real(1), real(0)};
-  real d = bd[r].y;
+  const real2 o = pair_at(own), pl = pair_at(l + kBD), pr = pair_at(r + kBD);
+  real d = pair_at(own + kBD).y;
   const int dm = (int)mag(d);
-  const bool l = hl && dm - (int)mag(o.x) <= (int)mag(pl.y) - (int)mag(pl.x) + kGap;
-  const bool rr = hr && dm - (int)mag(o.y) <= (int)mag(pr.y) - (int)mag(pr.x) + kGap;
-  if (l) d -= EMDB_DIV_RARE(o.x, pl.x) * pl.y;
-  if (rr) d -= EMDB_DIV_RARE(o.y, pr.x) * pr.y;
+  if (hl && dm - (int)mag(o.x) <= (int)mag(pl.y) - (int)mag(pl.x) + kGap)
+    d -= o.x / pl.x * pl.y;
+  if (hr && dm - (int)mag(o.y) <= (int)mag(pr.y) - (int)mag(pr.x) + kGap)
+    d -= o.y / pr.x * pr.y;
   return d;
 }
 
@@ -996,27 +1019,57 @@ __device__ __forceinline__ real pcr_last(const real2* ac, const real2* bd, int r
 // round away too (pcr_last), and the division by the diagonal, fused.  One
 // vote decides for both systems; systems for which it fails (and those of at
 // most 32 rows) run every level.
-// Bound by FP64 issue and latency: per row and level two quotients (20 FP64
-// operations) and 8 more, six 16-byte loads.  On 2048-sample seismic traces
-// the row-levels fall from 4.25 to 3.0 million per 24 traces, at 8192 samples
-// from 16.4 to 9.7; no pass of those needed a seventh level.  B200, all levels
-// with the former quotients / as here: 16,384 x 2048 seismic 84.8 / 72.7 ms,
-// 1,024 x 4096 64.0 / 41.1, 256 x 8192 89.0 / 66.9; envelopes alone, 4,096 x
-// 2048: 0.53 / 0.38 ms.
-template <int NT>
-__device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kbase1, int kcnt0,
+// Bound by FP64 latency and instruction supply: per row and level two
+// quotients (20 FP64 operations), 8 more and about 45 others, six 16-byte
+// loads.  On 2048-sample seismic traces the row-levels fall from 4.25 to 3.0
+// million per 24 traces, at 8192 samples from 16.4 to 9.7; no pass of those
+// needed a seventh level.  B200, all levels with the former quotients / cut
+// short, 16-byte rows / blocks of rows, no operand tests, votes without
+// reductions, plain divisions where a lane has one: 16,384 x 2048 seismic 84.8 /
+// 72.7 / 54.2 ms (the last with the other changes since), 256 x 8192 89.0 / 66.9
+// / 50.8, 96 x 1501 1.75 / 1.60 / 1.15; envelopes alone, 4,096 x 2048: 0.53 / 0.38
+// / 0.35 ms.
+//
+// Quotients without range checks or zero tests.  Suppose the spacings are
+// positive, within [2^-100, 2^100) and within 2^24 of each other, and no
+// right-hand side is -0.  The rows stay diagonally dominant
+// (|a| + |c| <= b/2; rows without a left or right neighbour <= b), so b loses
+// at most half a level and stays within 2^-5 and 2^6 of the spacings; each
+// level squares the couplings relative to it, so the non-zero ones entering
+// the fifth level are at least 2^-52 (2^-30)^16 2^-100 = 2^-632 (2^-52: the
+// end rows' h1 - h0), and their quotients' last remainders at least 2^-870:
+// nothing underflows.  A zero coupling gives the multiplier +0 where the
+// division may give -0, and a row without a neighbour multiplies a row (0, 1,
+// 0, 0) by its zero coupling instead of by +0; either changes no b, and no d
+// except -0 - (-0), which cannot arise from right-hand sides other than -0.
+// Each row checks its spacing -- on the integer axis to be in [1, kMaxIntSeg],
+// else within 2^12 of the first one -- and one vote decides; the others take
+// pcr_levels_any, and so do the levels past the fifth where the vote on those
+// fails (its window for d is 2^23 either way of the middle row's).
+// Returns (the same in every thread) whether the evaluation needs no test of
+// spacings and moments: the condition on spacings above and every moment zero
+// or in [2^-700, 2^900).  The FP32 build divides, tests its quotients, and
+// gets true.
+template <int NT, bool kInt>
+__device__ __forceinline__ bool solve_splines(const Knots& K, int kbase0, int kbase1, int kcnt0,
                                               int kcnt1, int tid, Ctl& C) {
+  constexpr bool kDouble = sizeof(real) == 8;
+  constexpr int kLast = 32;                     // stride of the fused level
+  constexpr int kFrac = kDouble ? 20 : 23, kBias = kDouble ? 1023 : 127;   // of magnitude words
   const int m0 = kcnt0 >= 4 ? kcnt0 - 2 : 0;
   const int m1 = kcnt1 >= 4 ? kcnt1 - 2 : 0;
-  const int mt = m0 + m1;
+  const int mt = m0 + m1, mmax = max(m0, m1);
   const real2* xy0 = K.XY[0] + kbase0;
   const real2* xy1 = K.XY[1] + kbase1;
-  unsigned* const range = C.range;
-  if (tid == 0) {
-    range[0] = 0u;
-    range[1] = 0xffffffffu;
-    K.ac(0)[mt] = K.ac(1)[mt] = real2{real(0), real(0)};
-    K.bd(0)[mt] = K.bd(1)[mt] = real2{real(1), real(0)};
+  const bool deep = mmax > kLast;
+  // levels alternate buffers and have to end in buffer 1 (M goes to buffer 0):
+  // five of them, or ceil(log2 mmax)
+  int cur = deep || mmax < 2 ? 0 : 1 ^ (1 & (32 - __clz(mmax - 1)));
+  const int guard = row_at(mt);
+  if (tid < 2) {
+    // the neighbour of rows that have none
+    pair_at(K.rows(tid) + guard) = real2{real(0), real(0)};
+    pair_at(K.rows(tid) + guard + kBD) = real2{real(1), real(0)};
   }
   // Rows (kernels.py:613-636): row k has the segments k and k+1 around it, and
   // each segment's slope serves two rows.  A lane forms one slope and takes
@@ -1024,6 +1077,8 @@ __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kb
   // rows and the next 32 start one back: one division a row instead of two.
   // The end rows have the same right-hand side up to the factor h/(h0+h1).
   const int z0 = m0 > 0 ? m0 + 1 : 0, zt = z0 + (m1 > 0 ? m1 + 1 : 0);
+  const unsigned href = kInt ? 0u : mag(xy0[1].x - xy0[0].x) - (12u << kFrac);
+  bool odd = false;
 #pragma unroll 1
   for (int zb = (tid >> 5) * 31; zb < zt; zb += (NT / 32) * 31) {
     const int z = zb + (tid & 31);
@@ -1034,93 +1089,95 @@ __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kb
       const real2* xy = (s0 ? xy0 : xy1) + g;
       const real2 p0 = xy[0], p1 = xy[1];
       h = p1.x - p0.x;
-      const real dy = p1.y - p0.y;
-      bool slow = false;
-      sl = div_nb(dy, h, slow);
-      if (slow) sl = EMDB_DIV_RARE(dy, h);
+      sl = (p1.y - p0.y) / h;
+      if (kDouble && kInt) odd |= !(h >= real(1) && h <= real(kMaxIntSeg));
+      else if (kDouble) odd |= !(h > real(0)) || mag(h) - href >= (24u << kFrac);
     }
     const real hm = __shfl_up_sync(kFull, h, 1), sm = __shfl_up_sync(kFull, sl, 1);
     if (z < zt && (tid & 31) != 0 && g > 0) {
       const int k = g - 1, r = (s0 ? 0 : m0) + k;
       real a = hm, b = 2.0 * (hm + h), c = h, d = 6.0 * (sl - sm);
-      if (k == 0) {
-        a = 0.0; b = hm + 2.0 * h; c = h - hm;
-        d = EMDB_DIV_RARE(h * d, hm + h);
-      } else if (k == m - 1) {
-        a = hm - h; b = 2.0 * hm + h; c = 0.0;
-        d = EMDB_DIV_RARE(hm * d, hm + h);
+      if (k == 0 || k == m - 1) {
+        const real dh = k == 0 ? h * d : hm * d;
+        d = dh / (hm + h);
+        a = k == 0 ? real(0) : hm - h;
+        b = k == 0 ? hm + 2.0 * h : 2.0 * hm + h;
+        c = k == 0 ? h - hm : real(0);
       }
-      K.ac(0)[r] = real2{a, c};
-      K.bd(0)[r] = real2{b, d};
+      char* to = K.rows(cur) + row_at(r);
+      pair_at(to) = real2{a, c};
+      pair_at(to + kBD) = real2{b, d};
+      if (kDouble) odd |= d == real(0) && signbit(d);
     }
   }
-  __syncthreads();
+  if (!kInt && kDouble) odd |= href - ((kBias - 100u) << kFrac) >= (176u << kFrac);
+  const bool plain = !__syncthreads_or(odd);
+  odd = !plain;
   EMDB_PH(&C, 2);
-  constexpr int kLast = 32;                     // stride of the fused level
-  constexpr unsigned kSmall = (sizeof(real) == 8 ? (1023u - 26u) << 20 : (127u - 26u) << 23);
-  constexpr unsigned kNormal = sizeof(real) == 8 ? 1u << 20 : 1u << 23;
-  constexpr unsigned kRange = 46u * kNormal;
-  constexpr unsigned kInfMag = sizeof(real) == 8 ? 0x7ff00000u : 0x7f800000u;
-  const int mmax = max(m0, m1);
-  int cur = 0;
   bool fused = false;
+  int s = 1;
+  if (plain) {
 #pragma unroll 1
-  for (int s = 1; s < mmax; s *= 2) {
-    // the level whose multipliers and right-hand sides are looked at
-    const bool vote = 2 * s == kLast && mmax > kLast;
-    unsigned mult = 0u, dmax = 0u, dmin = 0xffffffffu;
+    for (; s < min(mmax, kLast); s *= 2) {
+      const int below = row_below(tid, s), above = row_above(tid, s);
+      const char* src = K.rows(cur);
+      char* dst = K.rows(cur ^ 1);
+      // the level whose multipliers and right-hand sides are looked at
+      const bool vote = 2 * s == kLast && deep;
+      const unsigned dref =
+          mag(pair_at(src + row_at(mt >> 1) + kBD).y) - (23u << kFrac);
+      bool no = dref - (1u << kFrac) >= unsigned(2 * kBias - 50) << kFrac;
+      int at = row_at(tid);
 #pragma unroll 1
-    for (int r = tid; r < mt; r += NT) {
-      const bool s0 = r < m0;
-      mult = max(mult, pcr_row(K.ac(cur), K.bd(cur), K.ac(cur ^ 1), K.bd(cur ^ 1), r,
-                               s0 ? r : r - m0, s, s0 ? m0 : m1, mt));
-      if (vote) {
-        const real2 p = K.bd(cur ^ 1)[r];
-        dmax = max(dmax, mag(p.y));
-        dmin = min(dmin, mag(p.y));
-        if (mag(p.x) < kNormal) mult = 0xffffffffu;
+      for (int r = tid; r < mt; r += NT, at += NT * 2 * kRow) {
+        const bool s0 = r < m0;
+        const bool hl = (s0 && r >= s) || r >= m0 + s;
+        const bool hr = r < m0 - s || (!s0 && r < mt - s);
+        const char* own = src + at;
+        const char* l = hl ? own - below : src + guard;
+        const char* rr = hr ? own + above : src + guard;
+        const real2 o = pair_at(own), p = pair_at(own + kBD);
+        const real2 ol = pair_at(l), pl = pair_at(l + kBD);
+        const real2 orr = pair_at(rr), pr = pair_at(rr + kBD);
+#if !EMDB_F32
+        const real alpha = div_core(o.x, pl.x), beta = div_core(o.y, pr.x);
+#else
+        const real alpha = hl ? o.x / pl.x : real(0), beta = hr ? o.y / pr.x : real(0);
+#endif
+        const real2 p2{p.x - alpha * ol.y - beta * orr.x, p.y - alpha * pl.y - beta * pr.y};
+        pair_at(dst + at) = real2{-alpha * ol.x, -beta * orr.y};
+        pair_at(dst + at + kBD) = p2;
+        if (vote)
+          no |= max(mag(alpha), mag(beta)) > (kBias - 26u) << kFrac ||
+                mag(p2.y) - dref >= (46u << kFrac) || (!kDouble && mag(p2.x) < (1u << kFrac));
       }
-    }
-    cur ^= 1;
-    if (vote) {
-      dmax = __reduce_max_sync(kFull, dmax);
-      dmin = __reduce_min_sync(kFull, dmin);
-      if ((tid & 31) == 0) {
-        atomicMax(range, dmax);
-        atomicMin(range + 1, dmin);
-      }
-      const int bad = __syncthreads_or(mult > kSmall);
-      const unsigned hi = range[0], lo = range[1];
-      if (!bad && hi < kInfMag && lo >= kNormal && hi - lo < kRange) {
-        fused = true;
-        break;
-      }
-    } else if (s < NT || 2 * s >= mmax) {
-      // Rows are owned by thread r mod NT, so a level with stride >= NT reads
-      // and writes only the calling thread's rows: no barrier is needed before
-      // the next such level.  Earlier levels read other threads' rows, and the
-      // solve below does too, so those transitions keep the barrier.
-      __syncthreads();
+      cur ^= 1;
+      if (vote) fused = !__syncthreads_or(no);
+      else __syncthreads();
     }
   }
+  if (!fused && s < mmax) pcr_levels_any<NT>(K.rows(0), K.rows(1), m0, m1, s, cur);
   EMDB_PH(&C, 3);
-  // diagonal solve + end-moment recovery (M[0], M[n-1] by the owners of the end rows)
-  const real2* ac = K.ac(cur);
-  const real2* bd = K.bd(cur);
-  auto moment = [&](int r, int k, int mq) {
-    const real d = fused ? pcr_last(ac, bd, r, k, kLast, mq) : bd[r].y;
-    const real b = bd[r].x;
-    bool slow = false;
-    const real q = div_nb(d, b, slow);
-    return slow ? EMDB_DIV_RARE(d, b) : q;
-  };
+  // diagonal solve
+  {
+    const char* src = K.rows(1);
+    int at = row_at(tid);
 #pragma unroll 1
-  for (int r = tid; r < mt; r += NT) {
-    const bool s0 = r < m0;
-    const int k = s0 ? r : r - m0;
-    const int mq = s0 ? m0 : m1;
-    const real Mk1 = moment(r, k, mq);
-    (s0 ? K.M[0] : K.M[1])[k + 1] = Mk1;
+    for (int r = tid; r < mt; r += NT, at += NT * 2 * kRow) {
+      const bool s0 = r < m0;
+      const char* own = src + at;
+      const real2 p = pair_at(own + kBD);
+      real d = p.y;
+      if (fused) {
+        const bool hl = (s0 && r >= kLast) || r >= m0 + kLast;
+        const bool hr = r < m0 - kLast || (!s0 && r < mt - kLast);
+        d = pcr_last(own, hl ? own - 2 * kLast * kRow : own, hr ? own + 2 * kLast * kRow : own,
+                     hl, hr);
+      }
+      const real q = d / p.x;
+      (s0 ? K.M[0] : K.M[1])[s0 ? r + 1 : r - m0 + 1] = q;
+      if (kDouble) odd |= odd_moment(q);
+    }
   }
   __syncthreads();
   // end moments from the first and last two (the reference forms the same
@@ -1131,17 +1188,19 @@ __device__ __forceinline__ void solve_splines(const Knots& K, int kbase0, int kb
     if (n >= 4) {
       const PairX x{q == 0 ? xy0 : xy1};
       real* M = q == 0 ? K.M[0] : K.M[1];
-      if ((tid & 1) == 0) {
-        const real h0 = x[1] - x[0], h1 = x[2] - x[1];
-        M[0] = ((h0 + h1) * M[1] - h0 * M[2]) / h1;
-      } else {
-        const real hnm3 = x[n - 2] - x[n - 3], hnm2 = x[n - 1] - x[n - 2];
-        M[n - 1] = ((hnm3 + hnm2) * M[n - 2] - hnm2 * M[n - 3]) / hnm3;
-      }
+      const bool left = (tid & 1) == 0;
+      const int i = left ? 0 : n - 3;
+      const real ha = x[i + 1] - x[i], hb = x[i + 2] - x[i + 1];
+      // M[0] = ((h0+h1) M[1] - h0 M[2]) / h1, M[n-1] the same from the other end
+      const real ho = left ? ha : hb, hi = left ? hb : ha;
+      const real m = ((ha + hb) * M[left ? 1 : n - 2] - ho * M[left ? 2 : n - 3]) / hi;
+      M[left ? 0 : n - 1] = m;
+      if (kDouble) odd |= odd_moment(m);
     }
   }
-  __syncthreads();
+  const int any_odd = __syncthreads_or(odd);
   EMDB_PH(&C, 4);
+  return !any_odd;
 }
 
 // One envelope's spline: knots, moments, knot count, mirrored-left and true knots.
@@ -1178,15 +1237,23 @@ __device__ __forceinline__ real eval_seg(const SideView& s, real t, int lo) {
 // eval_seg for n >= 4 knots with the quotients formed without the division's
 // slow-path branch, in the same operation order; sets `slow` for operands
 // outside the exact range, and the caller then re-evaluates the sample with
-// eval_seg.
+// eval_seg.  (FP64: spacings in [2^-100, 2^100), see EnvEval; the numerators'
+// quotients as in div_nb from one reciprocal.)
 __device__ __forceinline__ real eval_seg_q(const real2* xy, const real* M, real t, int lo,
                                            bool& slow) {
   const real2 p0 = xy[lo], p1 = xy[lo + 1];
   const real M0 = M[lo], M1 = M[lo + 1];
   const real h = p1.x - p0.x;
+#if EMDB_F32
   const real rh = real(1) / h;
   const real A = div_q(p1.x - t, h, rh, slow);
   const real B = div_q(t - p0.x, h, rh, slow);
+#else
+  const real a = p1.x - t, b = t - p0.x;
+  const real y = recip(h);
+  const real A = quot(a, h, y), B = quot(b, h, y);
+  slow |= odd_range(a) || odd_range(b);
+#endif
   const real num = ((A * A * A - A) * M0 + (B * B * B - B) * M1) * (h * h);
   return (A * p0.y + B * p1.y) + div6(num, slow);
 }
@@ -1194,6 +1261,7 @@ __device__ __forceinline__ real eval_seg_q(const real2* xy, const real* M, real 
 // The reference's per-sample binary search (kernels.py:722-726).
 __device__ __forceinline__ int search_seg(const SideView& s, real t) {
   int lo = 0, hi = s.n - 2;
+#pragma unroll 1
   while (lo < hi) {
     int mid = (lo + hi + 1) >> 1;
     if (s.xy[mid].x <= t) lo = mid; else hi = mid - 1;
@@ -1201,12 +1269,14 @@ __device__ __forceinline__ int search_seg(const SideView& s, real t) {
   return lo;
 }
 
-// Out-of-line bodies of the rare paths declared with div_slow.
-__device__ __noinline__ real eval_seg_cold(const real2* xy, const real* M, int n, real t, int lo) {
-  return eval_seg(SideView{xy, M, n, 0, 0}, t, lo);
-}
-__device__ __noinline__ int search_seg_cold(const real2* xy, int n, real t) {
-  return search_seg(SideView{xy, nullptr, n, 0, 0}, t);
+// Both envelopes at t by search and division, out of line: the rare passes'
+// evaluation (fewer than 4 knots, knot lists that are not strictly increasing,
+// operands outside the quotients' range), one call site a loop.
+__device__ __noinline__ real2 eval_any(const real2* xy0, const real* M0, int n0,
+                                       const real2* xy1, const real* M1, int n1, real t) {
+  const SideView s0{xy0, M0, n0, 0, 0}, s1{xy1, M1, n1, 0, 0};
+  return real2{eval_seg(s0, t, n0 >= 4 ? search_seg(s0, t) : 0),
+               eval_seg(s1, t, n1 >= 4 ? search_seg(s1, t) : 0)};
 }
 
 // 128-lane tree of the reference (kernels.py:794-804), on warp 0, for a value
@@ -1312,25 +1382,27 @@ __device__ __forceinline__ void wide_lane_sums(real* red, const real* __restrict
 // sample times are integers, so A = (x1-t)/h and B = (t-x0)/h are quotients of
 // integers 0 <= a <= h.  For those, q0 = RN(a*y) with y = RN(1/h) and one
 // correction RN(q0 + (a - h*q0)*y) equal RN(a/h): checked exhaustively for
-// every pair with h <= 65536 (2.1e9 pairs).  A spacing past the table sets
-// `slow`, and the caller redoes the sample with eval_seg.  h + 2^52 holds the
-// integer h in its low word (no conversion instruction).
+// every pair with h <= 65536 (2.1e9 pairs).
+//
+// No operand is tested.  With h <= kMaxIntSeg and every moment zero or in
+// [2^-700, 2^900) (EnvEval): A is 0, 1 or in [1/h, 1 - 1/h], so A^3 - A is 0 or
+// at least 2^-18 and at most 1/2, its product with a moment 0 or a normal
+// number of at least 2^-718, the sum of two such products a multiple of 2^-771
+// below 2^900, and h^2 in [1, 2^32]: num is 0 or in [2^-771, 2^932), inside
+// div6's range.
 #if !EMDB_F32
-__device__ __forceinline__ real eval_seg_int(const real2* xy, const real* M, real t, int lo,
-                                             bool& slow) {
+__device__ __forceinline__ real eval_seg_int(const real2* xy, const real* M, real t, int lo) {
   const real2 p0 = xy[lo], p1 = xy[lo + 1];
   const real M0 = M[lo], M1 = M[lo + 1];
   const real h = p1.x - p0.x;
   const real a = p1.x - t, b = t - p0.x;
-  const unsigned hi = (unsigned)__double2loint(h + 0x1p52);
-  slow |= hi > (unsigned)kRcpTab;
-  const real r = g_rcp.v[min(hi, (unsigned)kRcpTab)];
+  const real r = recip(h);
   real A = a * r;
   A = fma(fma(-A, h, a), r, A);
   real B = b * r;
   B = fma(fma(-B, h, b), r, B);
   const real num = ((A * A * A - A) * M0 + (B * B * B - B) * M1) * (h * h);
-  return (A * p0.y + B * p1.y) + div6(num, slow);
+  return (A * p0.y + B * p1.y) + div6(num);
 }
 #endif
 
@@ -1346,52 +1418,67 @@ __device__ __forceinline__ real eval_seg_int(const real2* xy, const real* M, rea
 // the chunks outside [lsym, rsym) compare them one by one; inside, with at
 // least one mirrored knot at each end, no clamp is needed either.
 //
-// A sample takes 27 FP64 operations per envelope on the integer axis; with the
-// range tests as compares of doubles, the two-step quotient by 6 and the
-// mirrored knots' compares in every chunk it took about 45.  The loop over
-// samples is kept rolled: the pass is bound by instruction supply as much as
-// by FP64 latency (unrolled by the compiler 93.5 ms, rolled 85.1 ms, 16,384 x
-// 2048 seismic).
+// `hot`, one value for the pass: the segments are O(1) and the quotients need
+// no test (solve_splines' answer), so that a chunk runs straight through; a
+// pass with exact zeros or flat runs, nbsym > 2, fewer than four knots or
+// operands of unusual magnitude searches and divides sample by sample.
+//
+// A sample takes 31 FP64 operations per envelope on the integer axis.  The loop
+// over chunks is kept rolled and two chunks a trip are slower: the pass is
+// bound by instruction supply and issue more than by FP64 latency.  Operand
+// tests and cold paths in the loop, RN(1/h) from a table / as here: 8 x 30011
+// 2.82 / 2.43 ms, 2,048 x 2048 from host memory 14.6 / 13.6, 16,384 x 2048 seismic
+// 60.1 / 58.2.
 template <bool kInt>
 struct EnvEval {
   const SideView s0, s1;
-  const bool fast;
-  const int iL, iR;
+  const bool hot;
+  const int cL, cR;              // chunks that need no compare with mirrored knots
   const unsigned incl;
-  __device__ __forceinline__ EnvEval(const SmemLayout& L, const Knots& K, const SideView& a,
-                                     const SideView& b, int NB, bool trig, int lane)
-      : s0(a), s1(b), fast(NB <= 2 && !trig && a.n >= 4 && b.n >= 4), iL(L.ctl->lsym),
-        iR(L.ctl->rsym), incl(lane == 31 ? kFull : ((2u << lane) - 1u)) {}
-  // segment of t, counted from the last left-mirrored knot, near the ends
-  static __device__ __forceinline__ int edge_seg(const SideView& s, int k, real t) {
-#pragma unroll 1
-    for (int j = 0; j < s.nl; ++j) k += s.xy[j].x <= t;
-#pragma unroll 1
-    for (int j = s.nl + s.nt; j < s.n; ++j) k += s.xy[j].x <= t;
-    return min(max(k - 1, 0), s.n - 2) - (s.nl - 1);
-  }
-  __device__ __forceinline__ void operator()(const SmemLayout& L, int i, real t, real& emax,
+  __device__ __forceinline__ EnvEval(const SmemLayout& L, const SideView& a, const SideView& b,
+                                     int NB, bool trig, bool plain, int lane)
+      : s0(a), s1(b), hot(NB <= 2 && !trig && a.n >= 4 && b.n >= 4 && plain),
+        cL((L.ctl->lsym + 31) >> 5), cR(L.ctl->rsym >> 5),
+        incl(lane == 31 ? kFull : ((2u << lane) - 1u)) {}
+  // chunk c, this lane's sample time t
+  __device__ __forceinline__ void operator()(const SmemLayout& L, int c, real t, real& emax,
                                              real& emin) const {
-    bool slow = !fast;
-    int lo0 = 0, lo1 = 0;
-    if (fast) {
-      const int c = i >> 5;
+    bool slow = !hot;
+    if (hot) {
       const uint2 m = L.mm[c];
       const uint32_t pp = L.pp[c];
-      lo0 = min((int)(pp & 0xffffu) + __popc(m.x & incl), s0.nt);
-      lo1 = min((int)(pp >> 16) + __popc(m.y & incl), s1.nt);
-      if ((c << 5) < iL || (c << 5) + 31 >= iR) {
-        lo0 = edge_seg(s0, lo0, t);
-        lo1 = edge_seg(s1, lo1, t);
+      int lo0 = min((int)(pp & 0xffffu) + __popc(m.x & incl), s0.nt);
+      int lo1 = min((int)(pp >> 16) + __popc(m.y & incl), s1.nt);
+      if (c < cL || c >= cR) {
+        // mirrored knots at or left of t
+        int k0 = -1, k1 = -1;
+#pragma unroll 1
+        for (int j = 0; j < s0.nl + s1.nl; ++j) {
+          const bool f = j < s0.nl;
+          const bool in = (f ? s0.xy[j].x : s1.xy[j - s0.nl].x) <= t;
+          k0 += f && in;
+          k1 += !f && in;
+        }
+        const int e0 = s0.nl + s0.nt, e1 = s1.nl + s1.nt;
+#pragma unroll 1
+        for (int j = 0; j < (s0.n - e0) + (s1.n - e1); ++j) {
+          const bool f = j < s0.n - e0;
+          const bool in = (f ? s0.xy[e0 + j].x : s1.xy[e1 + j - (s0.n - e0)].x) <= t;
+          k0 += f && in;
+          k1 += !f && in;
+        }
+        lo0 = min(max(lo0 + k0, 0), s0.n - 2);
+        lo1 = min(max(lo1 + k1, 0), s1.n - 2);
+      } else {
+        lo0 += s0.nl - 1;
+        lo1 += s1.nl - 1;
       }
-      lo0 += s0.nl - 1;
-      lo1 += s1.nl - 1;
 #if !EMDB_F32
       // (the FP32 build has no integer-axis shortcut: a float quotient formed
-      // in double from the table's RN(1/h) would be rounded twice)
+      // in double from RN(1/h) would be rounded twice)
       if (kInt) {
-        emax = eval_seg_int(s0.xy, s0.M, t, lo0, slow);
-        emin = eval_seg_int(s1.xy, s1.M, t, lo1, slow);
+        emax = eval_seg_int(s0.xy, s0.M, t, lo0);
+        emin = eval_seg_int(s1.xy, s1.M, t, lo1);
       } else
 #endif
       {
@@ -1400,12 +1487,9 @@ struct EnvEval {
       }
     }
     if (slow) {
-      if (!fast) {
-        lo0 = s0.n >= 4 ? EMDB_SEARCH_RARE(s0, t) : 0;
-        lo1 = s1.n >= 4 ? EMDB_SEARCH_RARE(s1, t) : 0;
-      }
-      emax = EMDB_EVAL_RARE(s0, t, lo0);
-      emin = EMDB_EVAL_RARE(s1, t, lo1);
+      const real2 v = eval_any(s0.xy, s0.M, s0.n, s1.xy, s1.M, s1.n, t);
+      emax = v.x;
+      emin = v.y;
     }
   }
 };
@@ -1461,16 +1545,18 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
     mbad = mirror_both(L, K, e, N, NB, T, lane);
   } else if (kWide) {
     if (parked)
+#pragma unroll 1
       for (int i = tid - 32; i < N; i += NT - 32) park_old[i] = imf[i];
   } else if (lend) {
     // park the proto-IMF while warp 0 mirrors; the PCR buffers overwrite it
     real* save = borrow_save(slab);
+#pragma unroll 1
     for (int i = tid - 32; i < N; i += kThreads - 32) save[i] = imf[i];
   }
   ps.bad = __syncthreads_or(bad || mbad) != 0;
   EMDB_PH(&C, 1);
   const int kb0 = C.kbase[0], kb1 = C.kbase[1], kn0 = C.kcnt[0], kn1 = C.kcnt[1];
-  solve_splines<NT>(K, kb0, kb1, kn0, kn1, tid, C);
+  const bool plain = solve_splines<NT, kInt>(K, kb0, kb1, kn0, kn1, tid, C);
   const real* oldv = !parked ? imf : kWide ? park_old : borrow_save(slab);
   // A pass with a maximum below zero or a minimum above it is never the last
   // one of its IMF, whatever the stop tests say (the reference forms their
@@ -1487,7 +1573,7 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
   ps.omax = -1e30;
   ps.omin = 1e30;
   bool oor = false;
-  const EnvEval<kInt> eval(L, K, sv0, sv1, NB, e.trig, lane);
+  const EnvEval<kInt> eval(L, sv0, sv1, NB, e.trig, plain, lane);
   // T is strictly increasing, so the knot spans cover every sample iff they
   // cover the first and the last one
   if (N > 0) {
@@ -1495,21 +1581,26 @@ __device__ __forceinline__ int sift_pass(const SmemLayout& L, char* slab, const 
     oor = (t0 < sv0.xy[0].x) || (tN > sv0.xy[sv0.n - 1].x) || (t0 < sv1.xy[0].x) ||
           (tN > sv1.xy[sv1.n - 1].x);
   }
-  real ti = kInt ? (real)tid : real(0);
+  // one warp a chunk of 32 samples, every NT / 32-th chunk (thread tid has the
+  // samples tid, tid + NT, ...); lanes past the end compute the last sample again
+  real ti = (real)tid;
 #pragma unroll 1
-  for (int i = tid; i < N; i += NT) {
-    const real t = kInt ? ti : T(i);
+  for (int c = __shfl_sync(kFull, warp, 0); c << 5 < N; c += NT / 32) {
+    const int i = (c << 5) + lane;
+    const real t = kInt ? ti : T(min(i, N - 1));
     ti += (real)NT;
-    const real old = oldv[i];
+    const real old = oldv[min(i, N - 1)];
     real emax, emin;
-    eval(L, i, t, emax, emin);
+    eval(L, c, t, emax, emin);
     const real mean = 0.5 * (emax + emin);
     const real nw = old - mean;
-    imf[i] = nw;
-    if (sums) {
-      // the wide instances sum per reference lane after the update
-      if (kWide) qbuf[i] = (nw - old) / nw;
-      else accumulate(ps, old, nw);
+    if (i < N) {
+      imf[i] = nw;
+      if (sums) {
+        // the wide instances sum per reference lane after the update
+        if (kWide) qbuf[i] = (nw - old) / nw;
+        else accumulate(ps, old, nw);
+      }
     }
   }
   // per-lane partial sums, then the reference's 128-lane trees on warp 0
@@ -1918,25 +2009,29 @@ __device__ __forceinline__ void envelope_pass(const SmemLayout& L, char* slab, c
   if (warp == 0) mirror_both(L, K, e, N, NB, T, lane);
   __syncthreads();
   const int kb0 = C.kbase[0], kb1 = C.kbase[1], kn0 = C.kcnt[0], kn1 = C.kcnt[1];
-  solve_splines<kThreads>(K, kb0, kb1, kn0, kn1, tid, C);
+  const bool plain = solve_splines<kThreads, kInt>(K, kb0, kb1, kn0, kn1, tid, C);
   const SideView sv[2] = {{K.XY[0] + kb0, K.M[0], kn0, NB - kb0, e.n_max},
                           {K.XY[1] + kb1, K.M[1], kn1, NB - kb1, e.n_min}};
   nk[0] = kn0;
   nk[1] = kn1;
   const int kcnt[2] = {kn0, kn1};
   bool oor = false;
-  const EnvEval<kInt> eval(L, K, sv[0], sv[1], NB, e.trig, lane);
+  const EnvEval<kInt> eval(L, sv[0], sv[1], NB, e.trig, plain, lane);
 #pragma unroll 1
-  for (int i = tid; i < N; i += kThreads) {
-    real t = T(i);
+  for (int ch = __shfl_sync(kFull, warp, 0); ch << 5 < N; ch += kWarps) {
+    const int i = (ch << 5) + lane;
+    const real t = T(min(i, N - 1));
     if (kInt) {
       // arange: the knot span covers every sample (see the mirroring)
-      real a, c;
-      eval(L, i, t, a, c);
-      emax_out[i] = a;
-      emin_out[i] = c;
+      real a, b;
+      eval(L, ch, t, a, b);
+      if (i < N) {
+        emax_out[i] = a;
+        emin_out[i] = b;
+      }
       continue;
     }
+    if (i >= N) continue;
     int lo0 = sv[0].n >= 4 ? search_seg(sv[0], t) : 0;
     int lo1 = sv[1].n >= 4 ? search_seg(sv[1], t) : 0;
     bool r0 = !(t < sv[0].xy[0].x || t > sv[0].xy[sv[0].n - 1].x);
@@ -2041,6 +2136,7 @@ __global__ void div_check_kernel(int mode, long long n, unsigned long long seed,
     for (long long bb = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; bb <= n; bb += stride) {
       const double b = (double)bb;
       const double y = 1.0 / b;
+      if (recip(b) != y) ++bad1;
       for (long long aa = 0; aa <= bb; ++aa) {
         const double a = (double)aa;
         if (__double_as_longlong(div_rn(a, b, y)) != __double_as_longlong(a / b)) ++bad0;

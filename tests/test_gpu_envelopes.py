@@ -129,3 +129,33 @@ def test_mirroring_of_few_extrema_equals_the_oracle(n, nbsym):
     for i in range(X.shape[0]):
         u, d = _envelopes(O, X[i], T, nbsym)
         assert upper[i].tobytes() == u.tobytes() and lower[i].tobytes() == d.tobytes(), i
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-170, 1e150])
+def test_spacings_and_values_of_any_magnitude(scale):
+    """Operands that the quotients without range tests do not cover: spacings
+    over a range of 2^40, axes far from 1, moments far from 1, knots of -0 and
+    +0 side by side."""
+    import torch
+    from cuda_emd import EMDKernelConfig
+    from oracle import emd_oracle as O
+    rng = np.random.default_rng(31)
+    n = 700
+    X = [_zigzag(rng, n, k) * v for k in (9, 62, 66, 150) for v in (1.0, 1e-120, 1e120)]
+    z = _zigzag(rng, n, 150)
+    z[z > 0.0] = np.where(rng.random(int((z > 0.0).sum())) < 0.5, 0.0, -0.0)
+    X = np.stack(X + [z])
+    step = np.ones(n - 1)
+    step[300:320] = 2.0 ** rng.uniform(0, 40, size=20)
+    T = np.concatenate([[0.0], np.cumsum(step)]) * scale
+    L = EMDKernelConfig().build()
+    got = L.run_envelope_only(torch.from_numpy(X).cuda(), torch.from_numpy(T).cuda())
+    run = [o.cpu().numpy() for o in EMDKernelConfig(max_iteration=4, max_imfs=4).build().run(
+        torch.from_numpy(X).cuda(), torch.from_numpy(T).cuda())]
+    for i in range(X.shape[0]):
+        with np.errstate(all="ignore"):
+            u, d = _envelopes(O, X[i], T, 2)
+            r = O.emd_signal(X[i], T, O.OracleConfig(max_iteration=4, max_imfs=4))
+        for a, b in ((got[0][i].cpu().numpy(), u), (got[1][i].cpu().numpy(), d), (run[0][i], r.imfs)):
+            same = (a.view(np.int64) == b.view(np.int64)) | (np.isnan(a) & np.isnan(b))
+            assert same.all(), (i, int((~same).sum()))
