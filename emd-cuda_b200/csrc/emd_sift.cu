@@ -1681,8 +1681,8 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
   real* gimf = kGImf ? reinterpret_cast<real*>(slab + p.imf_off) : nullptr;
 
   // this launch may hand over its tail / resumes another launch's tail
-  const bool migrate = kTail && !kWide && p.cont_buf != nullptr;
-  const bool resume = kTail && kWide && p.resume != 0;
+  const bool migrate = kTail && NT != kWideThreads && p.cont_buf != nullptr;
+  const bool resume = kTail && NT == kWideThreads && p.resume != 0;
   for (;;) {
     if (tid == 0) Cs->job = atomicAdd(resume ? p.cont_ticket : p.queue, 1);
     __syncthreads();
@@ -2364,12 +2364,13 @@ cudaError_t sift_occupancy(int arena_bytes, int variant, int* ctas_per_sm, bool 
 }
 
 cudaError_t launch_sift(const SiftParams& p, int grid, cudaStream_t stream) {
-  // tail migration (p.cont_buf): the 128 x 4 build that hands over, the
-  // 512-thread build that resumes
+  // tail migration (p.cont_buf): the 128 x 4 and 256 x 2 builds that hand over,
+  // the 512-thread build that resumes
   if (p.cont_buf != nullptr) {
     switch (p.variant) {
       case 1: return launch_v<kWideThreads, 1, false, true>(p, grid, stream);
       case 4: return launch_v<kThreads, 4, false, true>(p, grid, stream);
+      case 2: return launch_v<kHalfWideThreads, 2, false, true>(p, grid, stream);
       default: return cudaErrorInvalidValue;
     }
   }

@@ -26,7 +26,7 @@ struct emdb_plan {
   int arena_override = 0;
   int variant = 0;            // kernel instance (register variant); 0 = by trace length
   int max_ctas = 0;           // cap on a launch's persistent grid (0 = resident CTAs)
-  int tail = -1;              // tail migration: 0 off, -1 below the SM count, > 0 that many
+  int tail = -1;              // tail migration: 0 off, -1 two or three per SM, > 0 that many
   int* d_tail = nullptr;      // [0] traces in flight, [1] resume tickets
   int* d_cont_valid = nullptr;
   int cont_valid_cap = 0;
@@ -375,9 +375,7 @@ int launch_common(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, 
   // tail migration: the traces still in flight when the queue runs dry move
   // to a second launch of the 512-thread instance (not for launches of that
   // instance already)
-  // (the 256-thread instance gains nothing from it: 2,048 x 4096 seismic
-  // 46.1 ms without, 47.4-47.9 ms with thresholds of 74-444 traces)
-  const bool tail = p->tail != 0 && sp.variant == 4;
+  const bool tail = p->tail != 0 && (sp.variant == 4 || sp.variant == 2);
   typename SiftKernels<R>::Params rp{};
   int rgrid = 0;
   size_t cont_stride = 0;
@@ -402,12 +400,13 @@ int launch_common(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, 
     if (e != cudaSuccess) return cuda_fail(e, "tail reset");
     sp.active = p->d_tail;
     sp.cont_ticket = p->d_tail + 1;
-    // automatic: three traces per SM -- the resume launch runs a trace
-    // ~2.5x faster on a whole SM than a 128-thread CTA does, so handing
-    // over pays once fewer than that remain (B200, cfg1 shape: 16,384
-    // traces 67.1 ms at 1 per SM, 66.7-66.9 at 3, 67.2 at 4; 4,096 traces
-    // 22.4 / 21.9 / 21.9 ms)
-    sp.yield_below = p->tail < 0 ? 3 * p->num_sms : p->tail;
+    // automatic: three traces per SM from the 128-thread instance, two from the
+    // 256-thread one.  B200, ms, off and thresholds of 1 / 2 / 3 / 4 per SM:
+    // 128 threads, 16,384 x 2048 seismic 54.0; 53.0 / 52.7 / 52.5 / 53.0, 2,048 x
+    // 2048 11.4; 9.0 / 8.8 / 8.6 / 8.9; 256 threads (1 / 1.5 / 2 per SM), 1,024 x
+    // 4096 35.5; 28.0 / 27.7 / 27.1, 6,000 x 4096 101.5; 96.8 / 96.3 / 95.6, 300 x
+    // 3000 9.8; 8.6 / 8.5 / 8.4.
+    sp.yield_below = p->tail < 0 ? (sp.variant == 4 ? 3 : 2) * p->num_sms : p->tail;
     sp.cont_buf = p->d_cont;
     sp.cont_stride = cont_stride;
     sp.cont_valid = p->d_cont_valid;

@@ -200,7 +200,7 @@ class Plan:
         check(self.L.emdb_plan_set_variant(self.handle, int(min_ctas_per_sm)), "emdb_plan_set_variant")
 
     def set_tail(self, yield_below: int) -> None:
-        """Tail migration (emdb_plan_set_tail): 0 off, -1 below the SM count,
+        """Tail migration (emdb_plan_set_tail): 0 off, -1 two or three per SM,
         > 0 below that many traces in flight."""
         check(self.L.emdb_plan_set_tail(self.handle, int(yield_below)), "emdb_plan_set_tail")
 

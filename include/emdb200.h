@@ -84,17 +84,17 @@ int emdb_plan_set_variant(emdb_plan* plan, int min_ctas_per_sm);
  * grid is one CTA per signal, kernels.py:1366-1367). */
 int emdb_plan_set_max_ctas(emdb_plan* plan, int max_ctas);
 /* Tail migration for the plan's dense and ragged launches of the 128-thread
- * instance (4 per SM; no reference counterpart: its launch is one CTA per
- * signal, kernels.py:1366-1367).  Once every trace of a launch has started
+ * and 256-thread instances (4 and 2 per SM; no reference counterpart: its
+ * launch is one CTA per signal, kernels.py:1366-1367).  Once every trace of a launch has started
  * and at most yield_below of them are still in flight, each stops at its
  * next sift-pass boundary, parks its proto-IMF and loop state in a
  * plan-owned record, and a second launch of the 512-thread instance finishes
  * them, one trace per SM -- the last traces of a batch then run on a whole
- * SM instead of a quarter of one.  Same results bit for bit.  yield_below:
- * -1 = three per SM of the device (the default), 0 = off, > 0 that many.
- * Measured on B200 (dense seismic, 2048 samples): 4,096 traces 25.9 -> 21.9
- * ms, 16,384 traces 68.0 -> 66.7 ms; in FP32, where a few traces sift to
- * the iteration cap, 16,384 traces 114.0 -> 77.0 ms. */
+ * SM instead of a quarter or half of one.  Same results bit for bit.
+ * yield_below: -1 = three per SM of the device from 128-thread CTAs, two from
+ * 256-thread ones (the default), 0 = off, > 0 that many.  Measured on B200
+ * (dense seismic): 2,048 x 2048 samples 11.4 -> 8.6 ms, 16,384 x 2048 54.0 ->
+ * 52.5 ms, 1,024 x 4096 35.5 -> 27.1 ms. */
 int emdb_plan_set_tail(emdb_plan* plan, int yield_below);
 /* Arena and CTAs/SM the plan would use for traces up to max_n. */
 int emdb_plan_query(emdb_plan* plan, int max_n, int* arena_bytes, int* ctas_per_sm,
