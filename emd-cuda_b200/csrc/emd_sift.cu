@@ -1729,7 +1729,10 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
     SmemLayout L = carve<NT, kGImf>(smem, N, p.arena_bytes, gimf);
     Ctl& C = *L.ctl;
     real* imf = L.imf;
-    if (migrate && tid == 0) atomicAdd(p.active, 1);
+    if (migrate && tid == 0) {
+      atomicAdd(p.active, 1);
+      atomicAdd(p.started, 1);
+    }
     for (int k = tid; k < MAXI; k += NT) {
       C.dbg_n[k] = rec ? rec->dbg[0][k] : -1;
       C.dbg_e[k] = rec ? rec->dbg[1][k] : -1;
@@ -1801,7 +1804,7 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
           // pass: the two L2 reads and the barrier cost ~1 % per pass)
           int want = 0;
           if (tid == 0)
-            want = *reinterpret_cast<volatile int*>(p.queue) >= p.batch &&
+            want = *reinterpret_cast<volatile int*>(p.started) >= p.total &&
                    *reinterpret_cast<volatile int*>(p.active) <= p.yield_below;
           if (__syncthreads_or(want)) {
             yielded = true;
@@ -1898,7 +1901,8 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
     if (yielded) {
       // continuation record in this CTA's slot (a CTA hands over at most one
       // trace: the queue is empty when it does)
-      ContHead* h = reinterpret_cast<ContHead*>(p.cont_buf + (size_t)blockIdx.x * p.cont_stride);
+      const int rec_id = p.cont_base + blockIdx.x;
+      ContHead* h = reinterpret_cast<ContHead*>(p.cont_buf + (size_t)rec_id * p.cont_stride);
       real* dst = reinterpret_cast<real*>(reinterpret_cast<char*>(h) + cont_data_off());
       for (int i = tid; i < N; i += NT) dst[i] = imf[i];
       for (int k = tid; k < kMaxImfsCap; k += NT) {
@@ -1907,13 +1911,13 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
         h->dbg[2][k] = C.dbg_z[k];
       }
       if (tid == 0) {
-        h->b = b;
+        h->b = p.trace0 + b;
         h->n = n_yield;
         h->imf_count = imf_count;
         h->extNo_last = extNo_last;
         h->ovf = ovf ? 1 : 0;
         h->stale = stale ? 1 : 0;
-        p.cont_valid[blockIdx.x] = 1;
+        p.cont_valid[rec_id] = 1;
         atomicSub(p.active, 1);
         if (p.counters) {
           atomicAdd(p.counters, passes);

@@ -27,11 +27,15 @@ struct emdb_plan {
   int variant = 0;            // kernel instance (register variant); 0 = by trace length
   int max_ctas = 0;           // cap on a launch's persistent grid (0 = resident CTAs)
   int tail = -1;              // tail migration: 0 off, -1 two or three per SM, > 0 that many
-  int* d_tail = nullptr;      // [0] traces in flight, [1] resume tickets
-  int* d_cont_valid = nullptr;
-  int cont_valid_cap = 0;
-  char* d_cont = nullptr;     // continuation records
-  size_t cont_bytes = 0;
+  // tail migration's counters and records, one set for device launches and one
+  // for the host pipeline (whose launches run on streams of their own)
+  struct Tail {
+    int* counters = nullptr;  // [0] traces in flight, [1] resume tickets, [2] traces started
+    int* valid = nullptr;
+    int valid_cap = 0;
+    char* cont = nullptr;     // continuation records
+    size_t cont_bytes = 0;
+  } tail_dev, tail_host;
   int* d_ctl = nullptr;       // [0] sift queue, [1] status, [2] envelope queue
   unsigned long long* d_cnt = nullptr;  // [0] sift passes, [1] spilled passes, [2] / [3]
                                         // load / trace cycles, [4..13] phase cycles
@@ -344,26 +348,69 @@ int prepare_sift(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, i
 
 // Device buffers of tail migration for `grid` CTAs and traces up to max_n.
 template <typename R>
-int ensure_tail(emdb_plan* p, int grid, int max_n, size_t* stride) {
+int ensure_tail(emdb_plan::Tail& t, int grid, int max_n, size_t* stride) {
   *stride = al256(emdb::cont_data_off() + (size_t)std::max(max_n, 1) * sizeof(R));
   cudaError_t e = cudaSuccess;
-  if (!p->d_tail) e = cudaMalloc(&p->d_tail, 2 * sizeof(int));
-  if (e == cudaSuccess && grid > p->cont_valid_cap) {
-    if (p->d_cont_valid) cudaFree(p->d_cont_valid);
-    p->d_cont_valid = nullptr;
-    p->cont_valid_cap = 0;
-    e = cudaMalloc(&p->d_cont_valid, (size_t)grid * sizeof(int));
-    if (e == cudaSuccess) p->cont_valid_cap = grid;
+  if (!t.counters) e = cudaMalloc(&t.counters, 3 * sizeof(int));
+  if (e == cudaSuccess && grid > t.valid_cap) {
+    if (t.valid) cudaFree(t.valid);
+    t.valid = nullptr;
+    t.valid_cap = 0;
+    e = cudaMalloc(&t.valid, (size_t)grid * sizeof(int));
+    if (e == cudaSuccess) t.valid_cap = grid;
   }
   const size_t bytes = *stride * (size_t)grid;
-  if (e == cudaSuccess && bytes > p->cont_bytes) {
-    if (p->d_cont) cudaFree(p->d_cont);
-    p->d_cont = nullptr;
-    p->cont_bytes = 0;
-    e = cudaMalloc(&p->d_cont, bytes);
-    if (e == cudaSuccess) p->cont_bytes = bytes;
+  if (e == cudaSuccess && bytes > t.cont_bytes) {
+    if (t.cont) cudaFree(t.cont);
+    t.cont = nullptr;
+    t.cont_bytes = 0;
+    e = cudaMalloc(&t.cont, bytes);
+    if (e == cudaSuccess) t.cont_bytes = bytes;
   }
   if (e != cudaSuccess) return cuda_fail(e, "allocating the tail-migration records");
+  return EMDB_OK;
+}
+
+// Whether a launch of this instance hands its last traces over to the
+// 512-thread instance (which has nobody to hand over to).
+bool hands_over(const emdb_plan* p, int variant) {
+  return p->tail != 0 && (variant == 4 || variant == 2);
+}
+
+// Tail migration for launches of `grid` CTAs in all over `total` traces: zeroes
+// the counters and records on `st`, sets sp's fields, and makes rp (a resume
+// launch's parameters, from prepare_sift) take the records.
+template <typename R>
+int set_up_tail(const emdb_plan* p, const emdb_plan::Tail& t, typename SiftKernels<R>::Params& sp,
+                typename SiftKernels<R>::Params& rp, int grid, int total, size_t cont_stride,
+                cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(t.counters, 0, 3 * sizeof(int), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(t.valid, 0, (size_t)grid * sizeof(int), st);
+  if (e != cudaSuccess) return cuda_fail(e, "tail reset");
+  sp.active = t.counters;
+  sp.started = t.counters + 2;
+  sp.total = total;
+  sp.trace0 = sp.cont_base = 0;
+  // automatic: three traces per SM from the 128-thread instance, two from the
+  // 256-thread one.  B200, ms, off and thresholds of 1 / 2 / 3 / 4 per SM:
+  // 128 threads, 16,384 x 2048 seismic 54.0; 53.0 / 52.7 / 52.5 / 53.0, 2,048 x
+  // 2048 11.4; 9.0 / 8.8 / 8.6 / 8.9; 256 threads (1 / 1.5 / 2 per SM), 1,024 x
+  // 4096 35.5; 28.0 / 27.7 / 27.1, 6,000 x 4096 101.5; 96.8 / 96.3 / 95.6, 300 x
+  // 3000 9.8; 8.6 / 8.5 / 8.4.
+  sp.yield_below = p->tail < 0 ? (sp.variant == 4 ? 3 : 2) * p->num_sms : p->tail;
+  sp.cont_buf = t.cont;
+  sp.cont_stride = cont_stride;
+  sp.cont_valid = t.valid;
+  sp.cont_cap = grid;
+  sp.cont_ticket = t.counters + 1;
+  sp.resume = 0;
+  rp.active = rp.started = nullptr;
+  rp.cont_buf = t.cont;
+  rp.cont_stride = cont_stride;
+  rp.cont_valid = t.valid;
+  rp.cont_cap = grid;
+  rp.cont_ticket = t.counters + 1;
+  rp.resume = 1;
   return EMDB_OK;
 }
 
@@ -373,9 +420,8 @@ int launch_common(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, 
   int rc = prepare_sift<R>(p, sp, max_n, &grid);
   if (rc) return rc;
   // tail migration: the traces still in flight when the queue runs dry move
-  // to a second launch of the 512-thread instance (not for launches of that
-  // instance already)
-  const bool tail = p->tail != 0 && (sp.variant == 4 || sp.variant == 2);
+  // to a second launch of the 512-thread instance
+  const bool tail = hands_over(p, sp.variant);
   typename SiftKernels<R>::Params rp{};
   int rgrid = 0;
   size_t cont_stride = 0;
@@ -384,47 +430,23 @@ int launch_common(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, 
     rc = prepare_sift<R>(p, rp, max_n, &rgrid, 1);
     if (rc) return rc;
     rgrid = std::min(rgrid, grid);
-    rc = ensure_tail<R>(p, grid, max_n, &cont_stride);
+    rc = ensure_tail<R>(p->tail_dev, grid, max_n, &cont_stride);
     if (rc) return rc;
   }
   rc = ensure_slab(p, std::max(sp.slab_stride * (size_t)grid,
                                tail ? rp.slab_stride * (size_t)rgrid : 0));
   if (rc) return rc;
-  sp.queue = p->d_ctl;
-  sp.slab = p->d_slab;
+  sp.queue = rp.queue = p->d_ctl;
+  sp.slab = rp.slab = p->d_slab;
   cudaError_t e = cudaMemsetAsync(p->d_ctl, 0, sizeof(int), st);
   if (e != cudaSuccess) return cuda_fail(e, "queue reset");
   if (tail) {
-    e = cudaMemsetAsync(p->d_tail, 0, 2 * sizeof(int), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p->d_cont_valid, 0, (size_t)grid * sizeof(int), st);
-    if (e != cudaSuccess) return cuda_fail(e, "tail reset");
-    sp.active = p->d_tail;
-    sp.cont_ticket = p->d_tail + 1;
-    // automatic: three traces per SM from the 128-thread instance, two from the
-    // 256-thread one.  B200, ms, off and thresholds of 1 / 2 / 3 / 4 per SM:
-    // 128 threads, 16,384 x 2048 seismic 54.0; 53.0 / 52.7 / 52.5 / 53.0, 2,048 x
-    // 2048 11.4; 9.0 / 8.8 / 8.6 / 8.9; 256 threads (1 / 1.5 / 2 per SM), 1,024 x
-    // 4096 35.5; 28.0 / 27.7 / 27.1, 6,000 x 4096 101.5; 96.8 / 96.3 / 95.6, 300 x
-    // 3000 9.8; 8.6 / 8.5 / 8.4.
-    sp.yield_below = p->tail < 0 ? (sp.variant == 4 ? 3 : 2) * p->num_sms : p->tail;
-    sp.cont_buf = p->d_cont;
-    sp.cont_stride = cont_stride;
-    sp.cont_valid = p->d_cont_valid;
-    sp.cont_cap = grid;
-    sp.resume = 0;
+    rc = set_up_tail<R>(p, p->tail_dev, sp, rp, grid, sp.batch, cont_stride, st);
+    if (rc) return rc;
   }
   e = SiftKernels<R>::launch(sp, grid, st);
   if (e != cudaSuccess) return cuda_fail(e, "sift launch");
   if (tail) {
-    rp.queue = p->d_ctl;
-    rp.slab = p->d_slab;
-    rp.active = nullptr;
-    rp.cont_ticket = p->d_tail + 1;
-    rp.cont_buf = p->d_cont;
-    rp.cont_stride = cont_stride;
-    rp.cont_valid = p->d_cont_valid;
-    rp.cont_cap = grid;
-    rp.resume = 1;
     e = SiftKernels<R>::launch(rp, rgrid, st);
     if (e != cudaSuccess) return cuda_fail(e, "tail launch");
   }
@@ -484,9 +506,11 @@ int emdb_plan_destroy(emdb_plan* p) {
   {
     DeviceGuard g(p->device);
     if (p->d_slab) cudaFree(p->d_slab);
-    if (p->d_tail) cudaFree(p->d_tail);
-    if (p->d_cont_valid) cudaFree(p->d_cont_valid);
-    if (p->d_cont) cudaFree(p->d_cont);
+    for (emdb_plan::Tail* t : {&p->tail_dev, &p->tail_host}) {
+      if (t->counters) cudaFree(t->counters);
+      if (t->valid) cudaFree(t->valid);
+      if (t->cont) cudaFree(t->cont);
+    }
     if (p->d_ctl) cudaFree(p->d_ctl);
     if (p->d_cnt) cudaFree(p->d_cnt);
     if (p->d_stage) cudaFree(p->d_stage);
@@ -678,7 +702,7 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
     if (e != cudaSuccess) return cuda_fail(e, "allocating host-pipeline staging");
     p->stage_bytes = total;
   }
-  constexpr int kMaxChunks = 256;
+  constexpr int kMaxChunks = 256, kMinChunk = 8;
   constexpr int kG = emdb_plan::kGroups;
   if (!p->copy_stream) {
     e = cudaStreamCreateWithFlags(&p->copy_stream, cudaStreamNonBlocking);
@@ -696,12 +720,15 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(&p->d_chunk_flag, p->h_chunk_flag, 0);
     if (e != cudaSuccess) return cuda_fail(e, "setting up the host pipeline");
   }
-  // chunks of >= 64 traces, at most kMaxChunks of them; groups are whole
-  // chunks (4 groups for large batches, so the first launch starts after a
-  // quarter of the input copy)
-  const int chunk = std::max(64, (batch + kMaxChunks - 1) / kMaxChunks);
+  // Chunks of >= 8 traces, at most kMaxChunks of them: a chunk's copy starts
+  // when its slowest trace is done, so few traces a chunk let most rows cross
+  // the bus during the sift (B200, 2,048 x 2048 seismic, chunks of 64 / 32 / 16 /
+  // 8 / 4 traces: 12.5 / 11.4 / 10.6 / 9.9 / 9.9 ms, with the hand-over below; 13.3
+  // and 10.0 without and with it at 8).  Groups are whole chunks (4 groups for
+  // large batches, so the first launch starts after a quarter of the input copy).
+  const int chunk = std::max(kMinChunk, (batch + kMaxChunks - 1) / kMaxChunks);
   const int nchunk = (batch + chunk - 1) / chunk;
-  const int ngroup = nchunk >= 4 * kG ? kG : 1;
+  const int ngroup = batch >= 1024 ? kG : 1;
   volatile unsigned* flag = p->h_chunk_flag;
   // the previous call on this plan has returned, so no kernel writes the flags now
   for (int c = 0; c < nchunk; ++c) flag[c] = 0u;
@@ -738,7 +765,25 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
     if (k == 0) base = sp;                     // arena and config fields are shared
   }
   size_t slab_need = 0;
-  for (int k = 0; k < ngroup; ++k) slab_need += (size_t)grid[k] * base.slab_stride;
+  int grid_all = 0;
+  for (int k = 0; k < ngroup; ++k) {
+    slab_need += (size_t)grid[k] * base.slab_stride;
+    grid_all += grid[k];
+  }
+  // the batch's last traces, whichever group they are in, move to a launch of
+  // the 512-thread instance after the groups' (tail migration over the groups)
+  const bool tail = hands_over(p, base.variant);
+  emdb::SiftParams rp = base;
+  int rgrid = 0;
+  size_t cont_stride = 0;
+  if (tail) {
+    rp.batch = batch;
+    int rc = prepare_sift<double>(p, rp, N, &rgrid, 1);
+    if (rc == EMDB_OK) rc = ensure_tail<double>(p->tail_host, grid_all, N, &cont_stride);
+    if (rc) return rc;
+    rgrid = std::min(rgrid, grid_all);
+    slab_need = std::max(slab_need, (size_t)rgrid * rp.slab_stride);
+  }
   if (slab_need > p->group_slab_bytes) {
     if (p->d_group_slab) cudaFree(p->d_group_slab);
     p->d_group_slab = nullptr;
@@ -755,6 +800,10 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
   if (e == cudaSuccess) e = cudaMemsetAsync(p->d_group_queue, 0, kG * sizeof(int), st);
   if (e == cudaSuccess && T) e = cudaMemcpyAsync(d_T, T, n * 8, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cuda_fail(e, "host-pipeline set-up");
+  if (tail) {
+    int rc = set_up_tail<double>(p, p->tail_host, base, rp, grid_all, batch, cont_stride, st);
+    if (rc) return rc;
+  }
   unsigned long long h2d = (unsigned long long)(B * n * 8 + (T ? n * 8 : 0)), d2h = 0;
   // on a failure after the first launch, let what was issued finish before
   // returning: the staging and slabs are reused by the next call
@@ -764,6 +813,7 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
     return cuda_fail(err, what);
   };
   size_t slab_off = 0;
+  int grid_off = 0;
   for (int k = 0; k < ngroup; ++k) {
     const size_t t0 = (size_t)gstart[k], cnt = (size_t)gcount[k];
     if (N > 0)
@@ -787,6 +837,9 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
     sp.chunk_rows = p->d_chunk_rows + gstart[k] / chunk;
     sp.chunk_flag = p->d_chunk_flag + gstart[k] / chunk;
     slab_off += (size_t)grid[k] * base.slab_stride;
+    sp.trace0 = gstart[k];
+    sp.cont_base = grid_off;
+    grid_off += grid[k];
     e = emdb::launch_sift(sp, grid[k], p->group_stream[k]);
     if (e == cudaSuccess) e = cudaEventRecord(p->ev_group[k], p->group_stream[k]);
     if (e != cudaSuccess) return drain(e, "sift launch");
@@ -794,7 +847,23 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
   // only now does the caller's stream wait for the kernels: waiting inside the
   // loop would hold the next group's input copy behind this group's kernel
   for (int k = 0; k < ngroup && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(st, p->ev_group[k], 0);
-  if (e == cudaSuccess) e = cudaEventRecord(p->ev_kernel, st);     // after every group's kernel
+  if (e == cudaSuccess && tail) {
+    rp.values = d_sig;
+    rp.imfs = d_imf;
+    rp.n_imfs = d_n;
+    rp.overflow = d_ov;
+    rp.dbg_n = d_dn;
+    rp.dbg_ext = d_de;
+    rp.dbg_nzm = d_dz;
+    rp.queue = p->d_group_queue;
+    rp.slab = p->d_group_slab;
+    rp.chunk_span = batch;
+    rp.chunk_count = p->d_chunk_count;
+    rp.chunk_rows = p->d_chunk_rows;
+    rp.chunk_flag = p->d_chunk_flag;
+    e = emdb::launch_sift(rp, rgrid, st);
+  }
+  if (e == cudaSuccess) e = cudaEventRecord(p->ev_kernel, st);     // after every kernel
   if (e != cudaSuccess) return drain(e, "host-pipeline event");
 
   NvtxRange nvtx_copyback("emdb_run_host copy-back");

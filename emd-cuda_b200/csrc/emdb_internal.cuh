@@ -75,11 +75,18 @@ struct SiftParamsT {
   // stops at its next sift-pass boundary and leaves a continuation record
   // (its proto-IMF and loop state) in the record of its CTA; a second launch
   // of the 512-thread instance with resume = 1 finishes them, one per SM.
-  int* active;                // traces in flight in this launch (zeroed before it)
+  // A batch run as several launches (the host pipeline's input groups) shares
+  // the counters and the records: each launch has its first trace's number in
+  // the batch and its first record.
+  int* active;                // traces in flight (zeroed before)
+  int* started;               // traces started so far (zeroed before), of `total`
+  int total;
+  int trace0;
+  int cont_base;
   int yield_below;
   char* cont_buf;             // cont_cap records of cont_stride bytes, one per CTA
   size_t cont_stride;
-  int* cont_valid;            // [cont_cap]: 1 = record holds a trace (zeroed before it)
+  int* cont_valid;            // [cont_cap]: 1 = record holds a trace (zeroed before)
   int cont_cap;
   int* cont_ticket;           // the resume launch's ticket counter (zeroed before it)
   int resume;
