@@ -63,6 +63,10 @@ struct emdb_plan {
   char* d_group_slab = nullptr;
   size_t group_slab_bytes = 0;
   unsigned long long host_h2d = 0, host_d2h = 0;   // bytes the last emdb_run_host moved
+  // CTAs per SM of the instances launched so far, by arena (the query costs
+  // more host time than the launch)
+  struct Occupancy { int arena, variant, per_sm; bool gimf, f32; };
+  std::vector<Occupancy> occupancy;
   std::mutex mu;
 };
 
@@ -295,6 +299,13 @@ int prepare_sift(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, i
     return fail(EMDB_ERR_UNSUPPORTED, "trace length " + std::to_string(max_n) +
                 " exceeds the longest supported trace (131072 samples)");
   // force_variant: that instance at its automatic arena (the tail's resume launch)
+  // A batch of at most one trace per SM goes to the 512-thread instance
+  // directly, where tail migration would move it anyway after a first launch
+  // that only starts it (B200, host clock, one 1024-sample
+  // trace: 233 / 223 us a call).
+  if (!force_variant && p->variant == 0 && p->arena_override == 0 && p->tail != 0 &&
+      sp.batch <= p->num_sms)
+    force_variant = 1;
   int variant = force_variant ? force_variant : effective_variant(p, max_n);
   int arena = force_variant ? auto_arena_for<R>(p->smem_optin, force_variant, p->cfg.nbsym, max_n)
                             : arena_for<R>(p, max_n);
@@ -315,8 +326,15 @@ int prepare_sift(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, i
     return fail(EMDB_ERR_UNSUPPORTED, "trace length " + std::to_string(max_n) +
                 " does not fit this device's shared memory");
   int per_sm = 0;
-  cudaError_t e = K::occupancy(arena, variant, &per_sm, gimf);
-  if (e != cudaSuccess) return cuda_fail(e, "occupancy query");
+  for (const auto& o : p->occupancy)
+    if (o.arena == arena && o.variant == variant && o.gimf == gimf && o.f32 == (sizeof(R) == 4))
+      per_sm = o.per_sm;
+  if (per_sm < 1) {
+    cudaError_t e = K::occupancy(arena, variant, &per_sm, gimf);
+    if (e != cudaSuccess) return cuda_fail(e, "occupancy query");
+    if (p->occupancy.size() >= 64) p->occupancy.clear();
+    p->occupancy.push_back({arena, variant, per_sm, gimf, sizeof(R) == 4});
+  }
   if (per_sm < 1) return fail(EMDB_ERR_UNSUPPORTED, "kernel cannot be resident with this arena");
   *grid = std::min(sp.batch, per_sm * p->num_sms);
   if (p->max_ctas > 0) *grid = std::min(*grid, p->max_ctas);
