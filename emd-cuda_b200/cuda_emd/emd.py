@@ -128,11 +128,15 @@ class GPUBatchEMD:
         return self._config
 
     def warmup(self, N: int = 64) -> None:
-        """One tiny real call (an all-zero trace, emd.py:58-64) so that plan
-        creation and first-launch costs land here, not in a timed call."""
+        """Tiny real calls (all-zero traces, emd.py:58-64) so that plan creation
+        and first-launch costs land here, not in a timed call: one with more
+        traces than SMs and one with a single trace, which take different kernel
+        instances."""
         import torch
         dt = torch.float32 if self._config.f32 else torch.float64
-        self(torch.zeros((1, N), dtype=dt, device="cuda"))
+        sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+        for batch in (sms + 1, 1):
+            self(torch.zeros((batch, N), dtype=dt, device="cuda"))
 
     def _get_launcher(self):
         if self._launcher is None:
