@@ -93,12 +93,11 @@ constexpr int kPhases = 10;
 // the sift computes is a `real`; the reference kernel's double literals keep
 // their C++ meaning, so float expressions that mix them are evaluated in
 // double and rounded once, as in the reference source compiled with REAL_T =
-// float.  The segment quotients have a float counterpart of the FP64 ones (div_q
-// from an IEEE reciprocal), self-tested against the float division by
-// emdb_check_division mode 3 (mode 4: div_nb, for which the PCR rows no longer
-// have a use); the one double quotient per envelope sample (the reference's "/ 6.0")
-// is formed from RN(1/6) and its residual (div6), which equals the double
-// division.
+// float.  Its quotients (div_q from an IEEE reciprocal; on the integer axis quot
+// and div_core from the approximate one) are self-tested against the float
+// division by emdb_check_division modes 3 and 4; the one double quotient per
+// envelope sample (the reference's "/ 6.0") is formed from RN(1/6) and its
+// residual (div6), which equals the double division.
 #ifndef EMDB_F32
 #define EMDB_F32 0
 #endif
@@ -423,13 +422,10 @@ __host__ __device__ inline int choose_place(int N, int arena_bytes, usize slab_s
 __device__ __noinline__ double div_slow(double a, double b) { return a / b; }
 
 #if EMDB_F32
-// Float counterparts (same methods, binary32 ranges): div_q is the two-step
-// Markstein quotient from y = RN(1/b); div_nb the branch-free quotient from
-// the approximate reciprocal (one Newton step reaches binary32 accuracy), a
-// faithful quotient and the exact-remainder choice of its neighbour (Muller
-// et al., Handbook of Floating-Point Arithmetic, ch. 4.9 / 5.3).  `slow` is
-// set outside the ranges where every step is exact: |a|, |q| in
-// (2^-100, 2^100), |b| in (2^-110, 2^110).
+// Float counterpart: div_q is the two-step Markstein quotient from y = RN(1/b)
+// (Muller et al., Handbook of Floating-Point Arithmetic, ch. 4.9 / 5.3).  `slow`
+// is set outside the ranges where every step is exact: |a|, |q| in
+// (2^-100, 2^100).
 __device__ __noinline__ float div_slow(float a, float b) { return a / b; }
 
 __device__ __forceinline__ float div_q(float a, float b, float y, bool& slow) {
@@ -444,25 +440,30 @@ __device__ __forceinline__ float div_q(float a, float b, float y, bool& slow) {
   return zero ? q0 : q2;
 }
 
-__device__ __forceinline__ float div_nb(float a, float b, bool& slow) {
+// 1/b within (1/2 + 2^-21) ulp, and a/b from it: the argument is the one at the
+// FP64 div_core, with 24 bits for 53.  y's relative error is at most
+// (1 + 2^-20) 2^-25 m_b (m_b in [1, 2) the significand of b) and the remainder
+// half an ulp of q, so the last step is off by less than the 2^-24 / m_b ulp(q)
+// that separate a quotient from a rounding boundary when m_b < 2 - 2^-18; the
+// 64 significands nearest 2 are checked with every numerator
+// (emdb_check_division mode 3, like all integer pairs up to 65536).  The
+// remainders are exact for |a| >= 2^-102 and |b| in [2^-5, 2^24), where q is
+// normal too.
+__device__ __forceinline__ float recip(float h) {
   float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-  const float e = fmaf(-b, y, 1.0f);
-  y = fmaf(y, e, y);
-  const float q0 = a * y;
-  const float r0 = fmaf(-q0, b, a);
-  const float q1 = fmaf(r0, y, q0);
-  const float r1 = fmaf(-q1, b, a);
-  const bool up = (r1 > 0.0f) == (b > 0.0f);
-  const int step = (up == (q1 > 0.0f)) ? 1 : -1;
-  const float qn = __int_as_float(__float_as_int(q1) + step);
-  const float rn = fmaf(-qn, b, a);
-  const float q = fabsf(rn) < fabsf(r1) ? qn : q1;
-  const float aa = fabsf(a), qa = fabsf(q1), ba = fabsf(b);
-  const bool bok = ba > 0x1p-110f && ba < 0x1p+110f;
-  const bool zero = a == 0.0f;
-  slow |= !bok || (!zero && !(aa > 0x1p-100f && aa < 0x1p+100f && qa > 0x1p-100f && qa < 0x1p+100f));
-  return zero ? q0 : q;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(h));
+  return fmaf(fmaf(-h, y, 1.0f), y, y);
+}
+__device__ __forceinline__ float quot(float a, float h, float y) {
+  float q = a * y;
+  q = fmaf(fmaf(-q, h, a), y, q);
+  return fmaf(fmaf(-q, h, a), y, q);
+}
+
+__device__ __forceinline__ float div_core(float a, float b) { return quot(a, b, recip(b)); }
+// neither zero nor at least 2^-80
+__device__ __forceinline__ bool tiny(float x) {
+  return (__float_as_uint(x) & 0x7fffffffu) - 1u < (47u << 23) - 1u;
 }
 #endif
 
@@ -1048,8 +1049,16 @@ __device__ __forceinline__ real pcr_last(const char* own, const char* l, const c
 // fails (its window for d is 2^23 either way of the middle row's).
 // Returns (the same in every thread) whether the evaluation needs no test of
 // spacings and moments: the condition on spacings above and every moment zero
-// or in [2^-700, 2^900).  The FP32 build divides, tests its quotients, and
-// gets true.
+// or in [2^-700, 2^900).
+// FP32: the same on the integer axis.  A coupling entering the fourth level is
+// a spacing times eight multipliers h_k / (2 (h_k + h_k+1)), each at least a
+// quarter, or a quarter of h_k / h_k+1 where spacings rise: with at most four
+// rises of 2^16 and one end row's factor it is at least 2^-96, and the
+// remainders are exact.  The fifth level divides where one is below 2^-80
+// (extrema in pairs thousands of samples apart).  Every float moment is in
+// div6's range.  On a given axis the FP32 build divides, tests its segment
+// quotients, and gets true.  B200, 4,096 x 1500 float seismic: 10.2 ms,
+// evaluation without tests 9.2, and the rows too 8.2.
 template <int NT, bool kInt>
 __device__ __forceinline__ bool solve_splines(const Knots& K, int kbase0, int kbase1, int kcnt0,
                                               int kcnt1, int tid, Ctl& C) {
@@ -1090,7 +1099,7 @@ __device__ __forceinline__ bool solve_splines(const Knots& K, int kbase0, int kb
       const real2 p0 = xy[0], p1 = xy[1];
       h = p1.x - p0.x;
       sl = (p1.y - p0.y) / h;
-      if (kDouble && kInt) odd |= !(h >= real(1) && h <= real(kMaxIntSeg));
+      if (kInt) odd |= !(h >= real(1) && h <= real(kMaxIntSeg));
       else if (kDouble) odd |= !(h > real(0)) || mag(h) - href >= (24u << kFrac);
     }
     const real hm = __shfl_up_sync(kFull, h, 1), sm = __shfl_up_sync(kFull, sl, 1);
@@ -1107,7 +1116,7 @@ __device__ __forceinline__ bool solve_splines(const Knots& K, int kbase0, int kb
       char* to = K.rows(cur) + row_at(r);
       pair_at(to) = real2{a, c};
       pair_at(to + kBD) = real2{b, d};
-      if (kDouble) odd |= d == real(0) && signbit(d);
+      if (kDouble || kInt) odd |= d == real(0) && signbit(d);
     }
   }
   if (!kInt && kDouble) odd |= href - ((kBias - 100u) << kFrac) >= (176u << kFrac);
@@ -1139,11 +1148,18 @@ __device__ __forceinline__ bool solve_splines(const Knots& K, int kbase0, int kb
         const real2 o = pair_at(own), p = pair_at(own + kBD);
         const real2 ol = pair_at(l), pl = pair_at(l + kBD);
         const real2 orr = pair_at(rr), pr = pair_at(rr + kBD);
-#if !EMDB_F32
-        const real alpha = div_core(o.x, pl.x), beta = div_core(o.y, pr.x);
-#else
-        const real alpha = hl ? o.x / pl.x : real(0), beta = hr ? o.y / pr.x : real(0);
+        real alpha, beta;
+        if (kDouble || kInt) {
+          alpha = div_core(o.x, pl.x), beta = div_core(o.y, pr.x);
+#if EMDB_F32
+          if (s == 16 && (tiny(o.x) || tiny(o.y))) {
+            alpha = div_slow(o.x, pl.x);
+            beta = div_slow(o.y, pr.x);
+          }
 #endif
+        } else {
+          alpha = hl ? o.x / pl.x : real(0), beta = hr ? o.y / pr.x : real(0);
+        }
         const real2 p2{p.x - alpha * ol.y - beta * orr.x, p.y - alpha * pl.y - beta * pr.y};
         pair_at(dst + at) = real2{-alpha * ol.x, -beta * orr.y};
         pair_at(dst + at + kBD) = p2;
@@ -1389,22 +1405,24 @@ __device__ __forceinline__ void wide_lane_sums(real* red, const real* __restrict
 // at least 2^-18 and at most 1/2, its product with a moment 0 or a normal
 // number of at least 2^-718, the sum of two such products a multiple of 2^-771
 // below 2^900, and h^2 in [1, 2^32]: num is 0 or in [2^-771, 2^932), inside
-// div6's range.
-#if !EMDB_F32
+// div6's range.  (FP32: every float is; its quotients take both corrections.)
 __device__ __forceinline__ real eval_seg_int(const real2* xy, const real* M, real t, int lo) {
   const real2 p0 = xy[lo], p1 = xy[lo + 1];
   const real M0 = M[lo], M1 = M[lo + 1];
   const real h = p1.x - p0.x;
   const real a = p1.x - t, b = t - p0.x;
   const real r = recip(h);
+#if EMDB_F32
+  const real A = quot(a, h, r), B = quot(b, h, r);
+#else
   real A = a * r;
   A = fma(fma(-A, h, a), r, A);
   real B = b * r;
   B = fma(fma(-B, h, b), r, B);
+#endif
   const real num = ((A * A * A - A) * M0 + (B * B * B - B) * M1) * (h * h);
   return (A * p0.y + B * p1.y) + div6(num);
 }
-#endif
 
 // Both envelopes at sample i (kernels.py:706-733).
 //
@@ -1473,15 +1491,10 @@ struct EnvEval {
         lo0 += s0.nl - 1;
         lo1 += s1.nl - 1;
       }
-#if !EMDB_F32
-      // (the FP32 build has no integer-axis shortcut: a float quotient formed
-      // in double from RN(1/h) would be rounded twice)
       if (kInt) {
         emax = eval_seg_int(s0.xy, s0.M, t, lo0);
         emin = eval_seg_int(s1.xy, s1.M, t, lo1);
-      } else
-#endif
-      {
+      } else {
         emax = eval_seg_q(s0.xy, s0.M, t, lo0, slow);
         emin = eval_seg_q(s1.xy, s1.M, t, lo1, slow);
       }
@@ -2212,13 +2225,13 @@ cudaError_t launch_div_check(int mode, long long n, unsigned long long seed,
 
 #if EMDB_F32
 // ---------------------------------------------------------------------------
-// Self-test of the float quotients (div_q, div_nb above) against the float
-// division.  mode 0: every integer pair 0 <= a <= b <= n through div_q with
-// y = RN(1/b) (the segment quotients on the default time axis); mode 1: n
-// pseudo-random pairs, [0] div_q with y = RN(1/b), significands random and
-// exponents in [-40, 40]; [1] div_nb with exponents in [-140, 140] (zeros,
-// subnormals and the range edges through the fallback); [2] div_nb on
-// PCR-like rows, |a| <= |b| within 2^+-40 of 1.  Counts mismatching bits.
+// Self-test of the float quotients above against the float division.  mode 0:
+// every integer pair 0 <= a <= b <= n through [0] div_q with y = RN(1/b) and [1]
+// quot with recip(b); [2] div_core, every numerator over the 64 significands
+// nearest 2.  mode 1: n pseudo-random pairs, [0] div_q with y = RN(1/b),
+// significands random and exponents in [-40, 40]; [1] div_core (the division for
+// `tiny` numerators) with exponents from -110 and of b in [-5, 23]; [2] div_core
+// on PCR-like rows, |a| <= |b|.  Counts mismatching bits.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t mix64f(uint64_t z) {
   z += 0x9e3779b97f4a7c15ull;
@@ -2237,20 +2250,30 @@ __global__ void div_check_f32_kernel(int mode, long long n, unsigned long long s
                                      unsigned long long* mismatches) {
   unsigned long long bad0 = 0, bad1 = 0, bad2 = 0;
   const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  auto wrong = [](float q, float a, float b) {
+    return __float_as_int(q) != __float_as_int(div_slow(a, b));
+  };
   if (mode == 0) {
-    for (long long bb = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; bb <= n; bb += stride) {
+    for (long long bb = 1 + first; bb <= n; bb += stride) {
       const float b = (float)bb;
-      const float y = 1.0f / b;
+      const float y = 1.0f / b, r = recip(b);
       for (long long aa = 0; aa <= bb; ++aa) {
         const float a = (float)aa;
         bool slow = false;
         float q = div_q(a, b, y, slow);
         if (slow) q = div_slow(a, b);
-        if (__float_as_int(q) != __float_as_int(div_slow(a, b))) ++bad0;
+        bad0 += wrong(q, a, b);
+        bad1 += wrong(quot(a, b, r), a, b);
       }
     }
+    for (long long i = first; i < 64ll << 23; i += stride) {
+      const float b = __int_as_float(0x3fffffff - (int)(i >> 23));             // 2 - (k + 1) 2^-23
+      const float a = __int_as_float(0x3f800000 | (int)(i & 0x7fffff));
+      bad2 += wrong(div_core(a, b), a, b);
+    }
   } else {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+    for (long long i = first; i < n; i += stride) {
       const uint64_t h1 = mix64f(seed ^ (uint64_t)i), h2 = mix64f(h1 ^ 0x5bd1e995ull);
       const uint64_t h3 = mix64f(h2 ^ 0x9e3779b9ull), h4 = mix64f(h3 ^ 0x7f4a7c15ull);
       {
@@ -2258,24 +2281,17 @@ __global__ void div_check_f32_kernel(int mode, long long n, unsigned long long s
         bool slow = false;
         float q = div_q(a, b, 1.0f / b, slow);
         if (slow) q = div_slow(a, b);
-        if (__float_as_int(q) != __float_as_int(div_slow(a, b))) ++bad0;
+        bad0 += wrong(q, a, b);
       }
       {
-        float a = rnd_float(h3, -140, 140), b = rnd_float(h4, -140, 140);
-        if ((h3 & 0xff) == 0) a = 0.0f;
-        bool slow = false;
-        float q = div_nb(a, b, slow);
-        if (slow) q = div_slow(a, b);
-        if (__float_as_int(q) != __float_as_int(div_slow(a, b))) ++bad1;
+        const float a = rnd_float(h3, -110, 23), b = rnd_float(h4, -5, 23);
+        bad1 += wrong(tiny(a) ? div_slow(a, b) : div_core(a, b), a, b);
       }
       {
-        const float b = rnd_float(h2 ^ h3, -40, 40);
+        const float b = rnd_float(h2 ^ h3, -5, 23);
         const float f = __int_as_float((int)((h4 >> 41) | 0x3f800000u)) - 1.0f;   // [0, 1)
         const float a = ((h1 & 2) ? -f : f) * b;
-        bool slow = false;
-        float q = div_nb(a, b, slow);
-        if (slow) q = div_slow(a, b);
-        if (__float_as_int(q) != __float_as_int(div_slow(a, b))) ++bad2;
+        bad2 += a != 0.0f && wrong(div_core(a, b), a, b);
       }
     }
   }
