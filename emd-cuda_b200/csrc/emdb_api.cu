@@ -180,19 +180,26 @@ int auto_arena_for(int smem_optin, int variant, int nbsym, int max_n) {
 // The plan's kernel instance for traces up to max_n.  Unless one was set
 // (or an arena, which is sized for the 128-thread instance): four 128-thread
 // CTAs per SM up to 2048 samples, two 256-thread CTAs per SM up to 4096, one
-// 512-thread CTA per SM beyond.  Measured on B200, dense seismic batches,
-// 128 / 256 / 512 threads: 16,384 x 2048 68 / 80 / 110 ms; 2,048 x 4096 72.1
-// / 46.3 / 51.6 ms; 1,024 x 8192 491.6 / 360.4 / 292.4 ms (three-tone and
-// chirp traces of 4096-8192 samples gain 1.6-2.9x on the wide instance).
+// 512-thread CTA per SM beyond.  B200, dense seismic batches, ms with 128 / 256 /
+// 512 threads, the first two handing their last traces over: 4,096 x 2300 23.9 /
+// 22.2 / 28.5; 2,048 x 4096 48.2 / 43.9 / 48.9; 1,024 x 6000 124.5 / 112.7 / 113.1;
+// 256 x 8192 54.6 / 54.6 / 56.8; 256 x 12000 - / 68.9 / 66.2.
+// FP32: knots take half the room, so the lines lie further out, and below the
+// first a fifth 128-thread CTA (102 registers) pays.  4 / 5 CTAs of 128, 256, 512
+// threads: 8,192 x 1000 6.4 / 6.1 / 9.0 / 13.8; 8,192 x 2048 22.5 / 21.3 / 27.4 / 37.6;
+// 4,096 x 3000 31.0 / 39.7 / 35.1 / 43.8; 2,048 x 4096 36.5 / 60.8 / 38.3 / 44.7; 1,024
+// x 7000 166 / - / 147 / 176; 300 x 16384 1100 / 1104 / 1013 / 1072.
+template <typename R>
 int effective_variant(const emdb_plan* p, int max_n) {
   if (p->variant != 0) return p->variant;
   if (p->arena_override > 0) return 4;
+  if (sizeof(R) == 4) return max_n > 16384 ? 1 : max_n > 4096 ? 2 : max_n > 2048 ? 4 : 5;
   return max_n > 4096 ? 1 : max_n > 2048 ? 2 : 4;
 }
 
 template <typename R = double>
 int auto_arena(const emdb_plan* p, int max_n) {
-  return auto_arena_for<R>(p->smem_optin, effective_variant(p, max_n), p->cfg.nbsym, max_n);
+  return auto_arena_for<R>(p->smem_optin, effective_variant<R>(p, max_n), p->cfg.nbsym, max_n);
 }
 
 template <typename R = double>
@@ -306,7 +313,7 @@ int prepare_sift(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, i
   if (!force_variant && p->variant == 0 && p->arena_override == 0 && p->tail != 0 &&
       sp.batch <= p->num_sms)
     force_variant = 1;
-  int variant = force_variant ? force_variant : effective_variant(p, max_n);
+  int variant = force_variant ? force_variant : effective_variant<R>(p, max_n);
   int arena = force_variant ? auto_arena_for<R>(p->smem_optin, force_variant, p->cfg.nbsym, max_n)
                             : arena_for<R>(p, max_n);
   bool gimf = false;
@@ -391,8 +398,9 @@ int ensure_tail(emdb_plan::Tail& t, int grid, int max_n, size_t* stride) {
 
 // Whether a launch of this instance hands its last traces over to the
 // 512-thread instance (which has nobody to hand over to).
+template <typename R>
 bool hands_over(const emdb_plan* p, int variant) {
-  return p->tail != 0 && (variant == 4 || variant == 2);
+  return p->tail != 0 && (variant == 4 || variant == 2 || (sizeof(R) == 4 && variant == 5));
 }
 
 // Tail migration for launches of `grid` CTAs in all over `total` traces: zeroes
@@ -415,7 +423,7 @@ int set_up_tail(const emdb_plan* p, const emdb_plan::Tail& t, typename SiftKerne
   // 2048 11.4; 9.0 / 8.8 / 8.6 / 8.9; 256 threads (1 / 1.5 / 2 per SM), 1,024 x
   // 4096 35.5; 28.0 / 27.7 / 27.1, 6,000 x 4096 101.5; 96.8 / 96.3 / 95.6, 300 x
   // 3000 9.8; 8.6 / 8.5 / 8.4.
-  sp.yield_below = p->tail < 0 ? (sp.variant == 4 ? 3 : 2) * p->num_sms : p->tail;
+  sp.yield_below = p->tail < 0 ? (sp.variant == 2 ? 2 : 3) * p->num_sms : p->tail;
   sp.cont_buf = t.cont;
   sp.cont_stride = cont_stride;
   sp.cont_valid = t.valid;
@@ -439,7 +447,7 @@ int launch_common(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, 
   if (rc) return rc;
   // tail migration: the traces still in flight when the queue runs dry move
   // to a second launch of the 512-thread instance
-  const bool tail = hands_over(p, sp.variant);
+  const bool tail = hands_over<R>(p, sp.variant);
   typename SiftKernels<R>::Params rp{};
   int rgrid = 0;
   size_t cont_stride = 0;
@@ -595,7 +603,7 @@ static int plan_query(emdb_plan* p, int max_n, int* arena_bytes, int* ctas_per_s
   int arena = arena_for<R>(p, max_n);
   int per_sm = 0;
   if (arena > 0) {
-    cudaError_t e = SiftKernels<R>::occupancy(arena, effective_variant(p, max_n), &per_sm);
+    cudaError_t e = SiftKernels<R>::occupancy(arena, effective_variant<R>(p, max_n), &per_sm);
     if (e != cudaSuccess) return cuda_fail(e, "occupancy query");
   }
   if (arena_bytes) *arena_bytes = arena;
@@ -790,7 +798,7 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
   }
   // the batch's last traces, whichever group they are in, move to a launch of
   // the 512-thread instance after the groups' (tail migration over the groups)
-  const bool tail = hands_over(p, base.variant);
+  const bool tail = hands_over<double>(p, base.variant);
   emdb::SiftParams rp = base;
   int rgrid = 0;
   size_t cont_stride = 0;

@@ -71,8 +71,9 @@ int emdb_plan_set_arena(emdb_plan* plan, int arena_bytes);
  * then targets that many CTAs; 1 = the wide instance, one 512-thread CTA per
  * SM working on one trace (long traces: 16 warps and the knots on-chip);
  * 2 = two 256-thread CTAs per SM; same results bit for bit; 0 (the default)
- * = by trace length: 4 up to 2048 samples, 2 up to 4096, 1 beyond (4 when
- * an arena was set).  The ragged autotuner sets one per tier.  A launch whose traces
+ * = by trace length: 4 up to 2048 samples, 2 up to 4096, 1 beyond; for float
+ * launches 5 up to 2048, 4 up to 4096, 2 up to 16384, 1 beyond (4 when an arena
+ * was set).  The ragged autotuner sets one per tier.  A launch whose traces
  * do not fit the plan's instance runs on the wide instance at the full
  * shared-memory arena, with the proto-IMF in global memory when shared
  * memory cannot hold it, so any trace length runs. */
@@ -84,7 +85,7 @@ int emdb_plan_set_variant(emdb_plan* plan, int min_ctas_per_sm);
  * grid is one CTA per signal, kernels.py:1366-1367). */
 int emdb_plan_set_max_ctas(emdb_plan* plan, int max_ctas);
 /* Tail migration for the plan's dense and ragged launches of the 128-thread
- * and 256-thread instances (4 and 2 per SM; no reference counterpart: its
+ * and 256-thread instances (4, for float launches also 5, and 2 per SM; no reference counterpart: its
  * launch is one CTA per signal, kernels.py:1366-1367).  Once every trace of a launch has started
  * and at most yield_below of them are still in flight, each stops at its
  * next sift-pass boundary, parks its proto-IMF and loop state in a
