@@ -545,9 +545,10 @@ def main():
             "e2e": e2e, "roofline": roofline, "cpu_baseline": cpu, "clocks": clk,
             "order": ordered,
             # each dense launch of the 128/256-thread instances is a pair
-            # (tail migration's resume launch); learned steps add the
+            # (tail migration's resume launch), one of at most a trace per SM
+            # is single; learned steps add the
             # feature and inference kernels
-            "gpu_launches": a.steps * ((2 if ctas_per_sm >= 2 else 1) + (2 if ordered else 0)),
+            "gpu_launches": a.steps * ((2 if ctas_per_sm >= 2 and B * ctas_per_sm > grid_max else 1) + (2 if ordered else 0)),
         }
         print(json.dumps(line), flush=True)
     R.finish(world)

@@ -3,7 +3,7 @@
 // Behaviour follows the reference's emd_batch_kernel (SeismicFlow/emd-cuda,
 // kernels.py:834-1080) and its device functions, re-built for B200:
 //
-//  * one 128-thread CTA per trace, persistent: CTAs pull trace tickets from an
+//  * one CTA (128, 256 or 512 threads) per trace, persistent: CTAs pull trace tickets from an
 //    atomic work queue (FIFO, or a caller-given order), so a long trace never
 //    holds a wave back and CSR batches of mixed length run in one launch;
 //  * the proto-IMF lives in shared memory for the whole decomposition; the
@@ -17,9 +17,10 @@
 //    kernels.py:722-726).  The post-update scan of pass n is reused as the
 //    pre-scan of pass n+1 (the reference scans the same data twice,
 //    kernels.py:930 vs 965);
-//  * boundary mirroring runs on one warp (decisions on one lane);
+//  * boundary mirroring runs on one warp, eight lanes to each mirrored end;
 //  * the upper and lower not-a-knot systems are solved concurrently by
-//    parallel cyclic reduction (ping-pong buffers, one barrier per level);
+//    parallel cyclic reduction (ping-pong buffers, one barrier per level), and
+//    levels that can no longer change a bit are left out;
 //  * envelope evaluation, the mean update and the six stop-test partial
 //    sums are one fused pass; sums are formed in the reference's order (128
 //    strided lanes + halving tree) and this file is compiled with
@@ -2330,7 +2331,7 @@ size_t sift_slab_bytes(int max_extrema, int nbsym) {
 
 namespace {
 // kInt: the kernel build for the integer time axis (T = arange), whose
-// segment quotients use the reciprocal table.
+// segment quotients are quotients of integers.
 template <int NT, int V, bool kInt, bool kG = false>
 cudaError_t occupancy_vt(int arena_bytes, int* ctas_per_sm) {
   cudaError_t e = cudaFuncSetAttribute(emd_sift_kernel<NT, V, kInt, kG>,
