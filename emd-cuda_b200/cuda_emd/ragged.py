@@ -273,15 +273,19 @@ class RaggedRunner:
 
     def split_heavy(self, tiers: list, heavy: np.ndarray, cost: np.ndarray | None) -> list:
         """The learned tier choice: the heavy traces of each long tier that
-        runs the 128-thread instance move to a launch of the wide instance
-        (one 512-thread CTA per SM, knots on-chip) capped at their share of
-        the SMs; the rest stay in the tuned launch.  Launched first, so their
-        CTAs take their SMs before the light launch fills the others."""
+        runs the 128- or 256-thread instance move to a launch of the wide
+        instance (one 512-thread CTA per SM, knots on-chip) capped at their
+        share of the SMs; the rest stay in the tuned launch.  Launched before
+        every other tier, so their CTAs take their SMs before the others fill
+        them: behind a tier of whole-SM CTAs the few heavy CTAs would start
+        when it ends and run on alone (65,536 traces of 256-8,192 samples on
+        one B200: 1,311 ms a step in tier order, 1,029 with the heavy
+        launches first, 1,032 without a split)."""
         import torch
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         c = np.ones(heavy.shape[0]) if cost is None else np.asarray(cost, dtype=np.float64)
         total = float(c.sum()) or 1.0
-        out = []
+        first, out = [], []
         for t in tiers:
             if t.edge < WIDE_FROM or t.variant == WIDE:
                 out.append(t)
@@ -299,12 +303,12 @@ class RaggedRunner:
             ht.max_n = t.max_n
             share = float(c[h].sum()) / total * self.heavy_boost
             ht.plan.set_max_ctas(int(min(max(1, round(share * sms)), h.size, sms)))
-            out.append(ht)
+            first.append(ht)
             light = t.idx[~heavy[t.idx]]
             if light.size:
                 t.idx = light
                 out.append(t)
-        return out
+        return first + out
 
     @staticmethod
     def _fill_orders(idx, orders, cost, device) -> None:
