@@ -161,7 +161,7 @@ __host__ __device__ constexpr int scan_slots() {
 }
 
 // Per-warp scan counts live right after the control block, one 16-byte word a
-// warp: maxima | minima << 16, sign changes, zero-run ends, fallback trigger
+// warp: maxima | minima << 16, sign changes, zero-run ends, flags (kScan*)
 // (room for 5 ints a warp).
 struct SmemLayout {
   Ctl* ctl;
@@ -594,6 +594,11 @@ struct TimeAxis {
 // Extrema: count pass (find_extrema_parallel semantics, kernels.py:231-349,
 // with the serial scan's plateau rule, kernels.py:157-200).
 // ---------------------------------------------------------------------------
+// Flags of a warp's scan word
+enum : uint32_t { kScanTrig = 1, kScanZeroFirst = 2 };
+// Longest trace whose zero-crossing count no chunk fallback can change
+constexpr int kFallbackFrom = kThreads * 128;
+
 // NS slots; `slot` is the calling warp's slot.
 //
 // The common chunk has no flat step, no exact zero and no underflowing product
@@ -655,7 +660,13 @@ __device__ __forceinline__ void extrema_count(const SmemLayout& L, int N, int sl
     zc += __popc(__ballot_sync(kFull, sc));
   }
   trig = __any_sync(kFull, trig);
-  if (lane == 0) L.wc[slot] = make_uint4(run, (uint32_t)zc, (uint32_t)zre, trig ? 1u : 0u);
+  if (lane == 0) {
+    // what extrema_scan decides by has to be read here: after its barrier
+    // other warps may be writing the residue into imf[] already
+    const bool zero_first = slot == 0 && N > kFallbackFrom && imf[0] == real(0);
+    L.wc[slot] = make_uint4(run, (uint32_t)zc, (uint32_t)zre,
+                            (trig ? kScanTrig : 0u) | (zero_first ? kScanZeroFirst : 0u));
+  }
 }
 
 struct ExtInfo {
@@ -664,6 +675,7 @@ struct ExtInfo {
   uint32_t off;           // this warp's rank offsets: maxima | minima << 16
   bool overflow;
   bool trig;              // serial-fallback trigger (exact zeros / flat runs)
+  bool zero_first;        // N > kFallbackFrom and the first sample is zero
 };
 
 // After the count pass + barrier.  Reproduces the parallel/serial split of
@@ -681,7 +693,8 @@ __device__ __forceinline__ ExtInfo extrema_totals(const SmemLayout& L, int warp,
   const uint32_t zc = __reduce_add_sync(kFull, w.y);
   ExtInfo e;
   e.off = __reduce_add_sync(kFull, lane < warp ? w.x : 0u);
-  e.trig = __any_sync(kFull, w.w != 0u);
+  e.trig = __any_sync(kFull, (w.w & kScanTrig) != 0u);
+  e.zero_first = __any_sync(kFull, (w.w & kScanZeroFirst) != 0u);
   e.n_zer = (int)zc;
   if (e.trig || L.ctl->chunk_bad) e.n_zer += (int)__reduce_add_sync(kFull, w.z);
   const int tot_max = (int)(tot & 0xffffu), tot_min = (int)(tot >> 16);
@@ -715,7 +728,10 @@ __device__ void chunk_fallback_check(const SmemLayout& L, int N, int tid) {
 
 // One extrema scan = count pass + totals, and the reference's rare chunk
 // fallback.  Ends after a barrier with every thread holding the same totals
-// and its warp's rank offsets.
+// and its warp's rank offsets.  Nothing here reads imf[] after the last
+// barrier: the caller may write it at once (the emission of a row does), and a
+// warp that came late to a test on imf[] would enter the fallback's barriers
+// alone.
 template <int NT>
 __device__ __forceinline__ ExtInfo extrema_scan(const SmemLayout& L, int N, int tid, int warp,
                                                 int lane, int max_extrema) {
@@ -724,7 +740,7 @@ __device__ __forceinline__ ExtInfo extrema_scan(const SmemLayout& L, int N, int 
   if (tid == 0) L.ctl->chunk_bad = 0;
   __syncthreads();
   ExtInfo e = extrema_totals<NS>(L, warp, lane, max_extrema);
-  if (N > kThreads * 128 && L.imf[0] == 0.0 && !e.trig) {
+  if (e.zero_first && !e.trig) {
     chunk_fallback_check(L, N, tid);
     e = extrema_totals<NS>(L, warp, lane, max_extrema);
   }
