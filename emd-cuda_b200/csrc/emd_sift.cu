@@ -1746,6 +1746,7 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
         atomicOr(p.status, kStatusTooLong);
         p.n_imfs[b] = 0;
         p.overflow[b] = 1;
+        if (migrate) atomicAdd(p.started, 1);   // the others wait for all to have started
       }
       for (int k = tid; k < MAXI; k += NT) {
         p.dbg_n[(int64_t)b * MAXI + k] = -1;
