@@ -78,6 +78,11 @@ def candidates(plan: _native.Plan, max_n: int) -> list[tuple[int, int]]:
     return out
 
 
+def _version(t):
+    """Counts torch's writes to a tensor (inference tensors have no counter)."""
+    return None if t.is_inference() else t._version
+
+
 class Tier:
     def __init__(self, edge: int, idx: np.ndarray, cfg: EMDKernelConfig, device: int):
         self.edge = edge
@@ -119,6 +124,11 @@ class RaggedRunner:
         self._heavy_tiers: dict[int, Tier] = {}
         self._graph = None
         self._graph_key = None
+        # the prepared batch: (key, tiers, indices, orders), its offsets and the
+        # tensor they came from
+        self._prep = None
+        self._prep_off = None
+        self._prep_src = None
         self._cache = self._load_cache()
 
     # -- autotune cache ----------------------------------------------------------
@@ -238,31 +248,47 @@ class RaggedRunner:
         """Host-side plan: tiers and per-tier queue orders (device int32).
 
         The tiers, their tuning and one persistent order buffer per tier are
-        cached for repeated calls on the same values / offsets tensors (a
-        captured graph reads those buffers); each call refills the buffers on
-        the current stream: FIFO, or longest `cost` first (cost: per-trace
-        work estimates, device tensor or host array).  ``offsets_host`` (the
-        same offsets in host memory) spares the device read-back.  ``heavy``
-        (host bool per trace, with ``cost_host``): those traces of each long
-        tier run in their own launch of the wide instance (split_heavy)."""
+        cached for repeated calls on batches of the same layout (a captured
+        graph reads those buffers); each call refills the buffers on the
+        current stream: FIFO, or longest `cost` first (cost: per-trace work
+        estimates, device tensor or host array).  What is cached is keyed by
+        the offsets' values: a buffer that is refilled, or freed and handed out
+        again for another batch, has other lengths at the same address.
+        ``offsets_host`` (the same offsets in host memory) spares the read-back
+        that takes.  ``heavy`` (host bool per trace, with ``cost_host``): those
+        traces of each long tier run in their own launch of the wide instance
+        (split_heavy)."""
         import hashlib
+        off_h = self._host_offsets(offsets, offsets_host)
         hkey = None if heavy is None else hashlib.sha1(np.packbits(heavy).tobytes()).hexdigest()
-        key = (offsets.data_ptr(), int(offsets.shape[0]), values.data_ptr(), hkey)
-        cached = getattr(self, "_prep", None)
-        if cached is None or cached[0] != key:
-            tiers, idx = self._prepare(values, offsets, offsets_host, heavy, cost_host)
+        key = (hkey, values.device)
+        if self._prep is None or self._prep[0] != key or not np.array_equal(self._prep_off, off_h):
+            self._prep = None
+            tiers, idx = self._prepare(values, offsets, off_h, heavy, cost_host)
             orders = [x.clone() for x in idx]
-            self._prep = cached = (key, tiers, idx, orders)
-        _, tiers, idx, orders = cached
+            self._prep = (key, tiers, idx, orders)
+            self._prep_off = np.array(off_h)
+        self._prep_src = (offsets, _version(offsets))
+        _, tiers, idx, orders = self._prep
         self._fill_orders(idx, orders, cost, values.device)
         return tiers, orders
 
-    def _prepare(self, values, offsets, offsets_host=None, heavy=None, cost_host=None):
+    def _host_offsets(self, offsets, offsets_host):
+        """The batch's offsets in host memory.  Nothing can be read back inside
+        a stream capture; there the plan made just before it stands for the
+        same tensor, if nothing has been written to it since."""
         import torch
         if offsets_host is not None:
-            off_h = np.asarray(offsets_host)
-        else:
-            off_h = offsets.cpu().numpy() if hasattr(offsets, "cpu") else np.asarray(offsets)
+            return np.asarray(offsets_host)
+        if offsets.is_cuda and torch.cuda.is_current_stream_capturing() and self._prep is not None:
+            src, version = self._prep_src
+            if (src.data_ptr() == offsets.data_ptr() and src.shape == offsets.shape
+                    and version == _version(offsets)):
+                return self._prep_off
+        return offsets.cpu().numpy()
+
+    def _prepare(self, values, offsets, off_h, heavy=None, cost_host=None):
+        import torch
         lengths = np.diff(off_h)
         tiers = self.tiers_for(lengths)
         self.tune(values, offsets, lengths, tiers)
@@ -418,11 +444,6 @@ class RaggedRunner:
             self._graph = self._graph_key = None
         v, o = st["v"], st["o"]
         off_np = offs_h.numpy()
-        if st.get("off_np") is None or not np.array_equal(st["off_np"], off_np):
-            # new batch layout in the same buffers: plan (tiers, orders, graph) again
-            st["off_np"] = off_np.copy()
-            self._prep = None
-            self._graph = self._graph_key = None
         v.copy_(vals_h, non_blocking=True)
         o.copy_(offs_h, non_blocking=True)
         if st["outs"] is None:
