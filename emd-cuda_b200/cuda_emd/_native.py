@@ -7,6 +7,8 @@ using the binding raises.  Build the library with
 from __future__ import annotations
 
 import ctypes
+import functools
+import hashlib
 import os
 import threading
 
@@ -52,6 +54,13 @@ _lock = threading.Lock()
 
 def lib_path() -> str:
     return LIB_PATH
+
+
+@functools.cache
+def build_digest() -> str:
+    """Identifies the library's build by its contents (read once)."""
+    with open(LIB_PATH, "rb") as f:
+        return hashlib.blake2b(f.read(), digest_size=8).hexdigest()
 
 
 def load() -> ctypes.CDLL:

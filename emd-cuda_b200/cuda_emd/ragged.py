@@ -17,7 +17,7 @@ The autotuner times every candidate (register-budget variant, arena) pair --
 the largest arena that keeps k = 6..1 CTAs per SM resident, with the kernel
 build compiled for max(k, 4) CTAs -- on a sample of each tier large enough to
 measure throughput (about 16 traces per CTA, or the whole tier) and caches
-the winner in a JSON file keyed by device, config and tier.
+the winner in a JSON file keyed by library build, device, config and tier.
 """
 from __future__ import annotations
 
@@ -136,9 +136,11 @@ class RaggedRunner:
         import torch
         name = torch.cuda.get_device_name(self.device)
         c = self.cfg
-        # "t3": entries timed on throughput-sized samples with the wide instance
-        # among the candidates (older ones are ignored)
-        return f"t3|{name}|{c.max_extrema},{c.nbsym},{c.max_iteration},{c.max_imfs}|{edge}"
+        # "t4": entries timed on throughput-sized samples with the wide instance
+        # among the candidates, by the kernels of this build of the library: the
+        # times of another build's say nothing about these
+        build = _native.build_digest() if self.cache_path else ""
+        return f"t4|{build}|{name}|{c.max_extrema},{c.nbsym},{c.max_iteration},{c.max_imfs}|{edge}"
 
     def _load_cache(self) -> dict:
         if self.cache_path and os.path.isfile(self.cache_path):
