@@ -190,6 +190,7 @@ class Plan:
         h = ctypes.c_void_p()
         check(self.L.emdb_plan_create(ctypes.byref(cfg), device, ctypes.byref(h)), "emdb_plan_create")
         self.handle = h
+        self._variant = self._arena = 0
 
     def close(self) -> None:
         if getattr(self, "handle", None) is not None and self.handle.value:
@@ -204,9 +205,15 @@ class Plan:
 
     def set_arena(self, arena_bytes: int) -> None:
         check(self.L.emdb_plan_set_arena(self.handle, int(arena_bytes)), "emdb_plan_set_arena")
+        self._arena = int(arena_bytes)
 
     def set_variant(self, min_ctas_per_sm: int) -> None:
         check(self.L.emdb_plan_set_variant(self.handle, int(min_ctas_per_sm)), "emdb_plan_set_variant")
+        self._variant = int(min_ctas_per_sm)
+
+    def by_length(self) -> bool:
+        """The plan picks its kernel instance itself (no variant or arena set)."""
+        return self._variant == 0 and self._arena == 0
 
     def set_tail(self, yield_below: int) -> None:
         """Tail migration (emdb_plan_set_tail): 0 off, -1 two or three per SM,

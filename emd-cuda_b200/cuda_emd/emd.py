@@ -128,15 +128,24 @@ class GPUBatchEMD:
         return self._config
 
     def warmup(self, N: int = 64) -> None:
-        """Tiny real calls (all-zero traces, emd.py:58-64) so that plan creation
-        and first-launch costs land here, not in a timed call: one with more
-        traces than SMs and one with a single trace, which take different kernel
-        instances."""
+        """Tiny real calls (an all-zero trace, emd.py:58-64) so that plan creation
+        and first-launch costs land here, not in a timed call: one on the kernel
+        instance that a batch of more traces than SMs takes, one on that of a
+        smaller batch.  Both with a single trace: scratch grows with the batch,
+        and what a warm-up of more traces than SMs allocates (25 MB) the first
+        real call would have to free."""
         import torch
-        dt = torch.float32 if self._config.f32 else torch.float64
-        sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-        for batch in (sms + 1, 1):
-            self(torch.zeros((batch, N), dtype=dt, device="cuda"))
+        f32 = self._config.f32
+        x = torch.zeros((1, N), dtype=torch.float32 if f32 else torch.float64, device="cuda")
+        plan = self._get_launcher()._plan
+        if plan.by_length():
+            # an automatic instance is numbered by its CTAs per SM
+            plan.set_variant(plan.query(N, f32)[1])
+            try:
+                self(x)
+            finally:
+                plan.set_variant(0)
+        self(x)
 
     def _get_launcher(self):
         if self._launcher is None:

@@ -1,0 +1,45 @@
+"""warmup() launches the kernel instances of small and of large batches, sizes no
+scratch for a large one, and leaves the plan as it was."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("real", ["double", "float"])
+@pytest.mark.parametrize("n", [64, 3000])
+def test_warmup_leaves_scratch_and_plan_as_they_were(real, n):
+    import torch
+    from cuda_emd import EMDKernelConfig, GPUBatchEMD, workloads as W
+    cfg = EMDKernelConfig(real_t=real)
+    X = torch.from_numpy(W.sinusoid_batch(200, n, seed=1).astype(cfg.dtype)).cuda()
+    first = GPUBatchEMD(cfg)                     # loads the modules
+    first.warmup(n)
+    plan = EMDKernelConfig(real_t=real).build()._plan
+    ctas = plan.query(n, first.config.f32)[1]
+    assert ctas == (4 if real == "float" else 2) if n == 3000 else ctas == (5 if real == "float" else 4)
+    emd = GPUBatchEMD(cfg)
+    emd._get_launcher()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    emd.warmup(n)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] < 8 << 20
+    assert emd._launcher._plan.by_length()
+    assert tuple(emd.last_debug[0].shape) == (1, cfg.max_imfs)
+    for a, b in zip(first(X), emd(X)):
+        assert torch.equal(a, b)
+
+
+def test_warmup_keeps_an_instance_that_was_set():
+    import torch
+    from cuda_emd import GPUBatchEMD
+    emd = GPUBatchEMD()
+    plan = emd._get_launcher()._plan
+    plan.set_variant(2)
+    emd.warmup()
+    assert plan._variant == 2
+    plan.set_variant(0)
+    plan.set_arena(60000)
+    emd.warmup()
+    assert (plan._variant, plan._arena) == (0, 60000)
