@@ -2156,7 +2156,8 @@ __global__ void __launch_bounds__(kThreads, 4) emd_envelope_kernel(EnvParams p) 
 // pair 0 <= a <= b <= n (the operands of A and B on the default time axis,
 // where knot spacings are integers <= 2N); mode 1: n pseudo-random pairs with
 // significands and exponents spread over [2^-600, 2^600] plus numerators
-// formed like the spline's h^2-scaled term over 6.  Counts mismatching bits.
+// formed like the spline's h^2-scaled term over 6.  Modes 2 and 3: the forms
+// without a reciprocal at hand, see there.  Counts mismatching bits.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {
   z += 0x9e3779b97f4a7c15ull;
@@ -2210,6 +2211,33 @@ __global__ void div_check_kernel(int mode, long long n, unsigned long long seed,
       if (slow) q = div_slow(a3, b3);
       if (__double_as_longlong(q) != __double_as_longlong(div_slow(a3, b3))) ++bad2;
     }
+  } else if (mode == 3) {
+    // the quotients as the kernels use them, without a fallback.  PCR rows:
+    // div_core for couplings from 2^-632 up and diagonals of spacings in [2^-100,
+    // 2^100) (solve_splines), [0] random, [1] the smallest couplings over all-ones,
+    // nearly all-ones and power-of-two significands; [2] segment quotients of
+    // a given axis: quot with recip, 0 <= a <= h, a from 2^-900 (eval_seg_q)
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+      const uint64_t h1 = mix64(seed ^ (uint64_t)i), h2 = mix64(h1 ^ 0x5bd1e995ull);
+      const uint64_t h3 = mix64(h2 ^ 0x9e3779b9ull);
+      const double ma = __longlong_as_double((long long)((h1 >> 12) | 0x3ff0000000000000ull));
+      const double mb = __longlong_as_double((long long)((h2 >> 12) | 0x3ff0000000000000ull));
+      const int eb = (int)(h3 % 211) - 105;
+      double a = ldexp(ma, -632 + (int)((h3 >> 8) % (unsigned)(eb + 634)));
+      if (h1 & 1) a = -a;
+      double b = ldexp(mb, eb);
+      if (__double_as_longlong(div_core(a, b)) != __double_as_longlong(div_slow(a, b))) ++bad0;
+      a = ldexp(ma, -632 + (int)((h3 >> 28) % 121));
+      b = (h2 & 4) ? __longlong_as_double(0x3fffffffffffffffll - (long long)((h2 >> 3) & 15)) : 1.0;
+      b = ldexp(b, eb);
+      if (h2 & 2) a = -a;
+      if (__double_as_longlong(div_core(a, b)) != __double_as_longlong(div_slow(a, b))) ++bad1;
+      const int eh = (int)((h3 >> 40) % 200) - 100;
+      const double h = ldexp(mb, eh);
+      a = (h1 & 2) ? h * ((double)((h1 >> 11) & 0xfffffffffffffull) * 0x1p-52)
+                   : ldexp(ma, -900 + (int)((h3 >> 48) % (unsigned)(eh + 900)));
+      if (__double_as_longlong(quot(a, h, recip(h))) != __double_as_longlong(div_slow(a, h))) ++bad2;
+    }
   } else {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
       uint64_t h1 = mix64(seed ^ (uint64_t)i), h2 = mix64(h1 ^ 0x5bd1e995ull);
@@ -2252,7 +2280,9 @@ cudaError_t launch_div_check(int mode, long long n, unsigned long long seed,
 // nearest 2.  mode 1: n pseudo-random pairs, [0] div_q with y = RN(1/b),
 // significands random and exponents in [-40, 40]; [1] div_core (the division for
 // `tiny` numerators) with exponents from -110 and of b in [-5, 23]; [2] div_core
-// on PCR-like rows, |a| <= |b|.  Counts mismatching bits.
+// on PCR-like rows, |a| <= |b|; mode 2: div_core alone, [0] numerators from 2^-102,
+// [1] the smallest over special significands, [2] every numerator of 2^-96 over
+// the 64 significands nearest 2.  Counts mismatching bits.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t mix64f(uint64_t z) {
   z += 0x9e3779b97f4a7c15ull;
@@ -2291,6 +2321,23 @@ __global__ void div_check_f32_kernel(int mode, long long n, unsigned long long s
     for (long long i = first; i < 64ll << 23; i += stride) {
       const float b = __int_as_float(0x3fffffff - (int)(i >> 23));             // 2 - (k + 1) 2^-23
       const float a = __int_as_float(0x3f800000 | (int)(i & 0x7fffff));
+      bad2 += wrong(div_core(a, b), a, b);
+    }
+  } else if (mode == 2) {
+    // div_core as the PCR rows use it, without a fallback: couplings from 2^-102
+    for (long long i = first; i < n; i += stride) {
+      const uint64_t h1 = mix64f(seed ^ (uint64_t)i), h2 = mix64f(h1 ^ 0x5bd1e995ull);
+      const uint64_t h3 = mix64f(h2 ^ 0x9e3779b9ull);
+      float a = rnd_float(h1, -102, 23), b = rnd_float(h2, -5, 23);
+      bad0 += wrong(div_core(a, b), a, b);
+      a = rnd_float(h3, -102, -80);
+      b = (h1 & 2) ? __int_as_float(0x3fffffff - (int)((h2 >> 3) & 63)) : 1.0f;
+      b = ldexpf(b, (int)((h3 >> 32) % 29) - 5);
+      bad1 += wrong(div_core(a, b), a, b);
+    }
+    for (long long i = first; i < 64ll << 23; i += stride) {
+      const float b = __int_as_float(0x3fffffff - (int)(i >> 23)) * 0x1p+22f;
+      const float a = __int_as_float(0x3f800000 | (int)(i & 0x7fffff)) * 0x1p-96f;
       bad2 += wrong(div_core(a, b), a, b);
     }
   } else {

@@ -271,10 +271,10 @@ class Plan:
 
 def check_division(mode: int, n: int, seed: int = 0) -> tuple[int, int, int]:
     """Self-test: mismatches of the kernels' own divisions vs the hardware
-    division, three counters per mode (mode 0/1: the reciprocal-based
-    division of the evaluation; mode 2: the PCR rows' branch-free division;
-    modes 3/4: the FP32 kernels' float quotients against the float division;
-    the header documents the cases)."""
+    division, three counters per mode (modes 0/1: quotients from a reciprocal;
+    mode 2: without one, behind a range test; mode 5: both as the kernels use
+    them, without; modes 3/4/6: the FP32 kernels' float quotients; the header
+    documents the cases)."""
     L = load()
     out = (ctypes.c_ulonglong * 3)()
     check(L.emdb_check_division(int(mode), int(n), int(seed), out), "emdb_check_division")

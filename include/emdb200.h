@@ -318,22 +318,29 @@ int emdb_mlp_adam(float* params, const float* grads, float* m, float* v, int n, 
 int emdb_mlp_infer_bf16(const uint16_t* params_bf16, const float* X, const float* mu,
                         const float* sd, int B, float* Y, void* stream);
 
-/* Self-test of the division the kernels use where a reciprocal is at hand
- * (no reference counterpart): counts results that differ in any bit from the
- * hardware IEEE division, in mismatches[3] (host array).  mode 0: every
- * integer pair 0 <= a <= b <= n (count in [0]); mode 1: n seeded random
- * cases each of [0] a/b over [2^-300, 2^300], [1] a/6, [2] a/b with
- * 0 <= a <= b, b in [1, 65537).  mode 2: the branch-free division the PCR
- * rows use (no reciprocal at hand), n seeded cases each of [0] a/b over
- * [2^-1100, 2^1100] (zeros, subnormals and infinities through its fallback),
- * [1] denominators with all-ones or power-of-two significands, [2] |a| <= |b|
- * within 2^+-40 of 1.  Modes 3 and 4: the FP32 kernels' float quotients
- * against the float division -- mode 3 every integer pair 0 <= a <= b <= n
- * through the reciprocal-based quotient; mode 4 n seeded cases each of [0]
- * the reciprocal-based quotient over [2^-40, 2^40], [1] the branch-free
- * quotient over [2^-140, 2^140] (zeros, subnormals, range edges through its
- * fallback), [2] PCR-like |a| <= |b| within 2^+-40 of 1.  Synchronous on the
- * current device. */
+/* Self-test of the quotients the kernels form without the division (no
+ * reference counterpart): counts results that differ in any bit from the
+ * hardware IEEE division, in mismatches[3] (host array).
+ * FP64.  mode 0: every integer pair 0 <= a <= b <= n from a reciprocal (count
+ * in [0]) and the kernels' reciprocal of every b (in [1]); mode 1: n seeded
+ * random cases each of [0] a/b over [2^-300, 2^300] from a reciprocal, [1] a/6,
+ * [2] a/b with 0 <= a <= b, b in [1, 65537); mode 2: the quotient without a
+ * reciprocal at hand behind its range test, n cases each of [0] a/b over
+ * [2^-1100, 2^1100] (zeros, subnormals and infinities divide), [1] denominators
+ * with all-ones or power-of-two significands, [2] |a| <= |b| within 2^+-40 of
+ * 1; mode 5: the quotients as the kernels use them, without a range test, n
+ * cases each of [0] the cyclic reduction's over couplings from 2^-632 and
+ * diagonals in [2^-105, 2^106), [1] its smallest couplings over special
+ * significands, [2] segment quotients of a given time axis, 0 <= a <= h, a from
+ * 2^-900, h in [2^-100, 2^100).
+ * FP32.  mode 3: every integer pair 0 <= a <= b <= n from [0] an IEEE and [1]
+ * the kernels' reciprocal, [2] every numerator over the 64 significands nearest
+ * 2; mode 4: n seeded cases each of [0] the quotient from an IEEE reciprocal
+ * over [2^-40, 2^40], [1] the one without, numerators from 2^-110 (below 2^-80 the
+ * division), denominators in [2^-5, 2^24), [2] the same with |a| <= |b|; mode 6:
+ * that quotient alone, [0] numerators from 2^-102, [1] those below 2^-79 over
+ * special significands, [2] every numerator of 2^-96 over the 64 significands
+ * nearest 2.  Synchronous on the current device. */
 int emdb_check_division(int mode, long long n, unsigned long long seed,
                         unsigned long long* mismatches);
 
