@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <chrono>
 #include <condition_variable>
 #include <cstdio>
@@ -479,6 +480,27 @@ int launch_common(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, 
   return EMDB_OK;
 }
 
+// Scratch for a launch of any batch of traces up to max_n, and for batches of
+// at most one trace per SM; none if it were more than kReserveMost (the default
+// config takes 97 MB, for float launches 122; it grows with max_extrema).
+constexpr size_t kReserveMost = size_t(256) << 20;
+
+template <typename R>
+int reserve(emdb_plan* p, int max_n) {
+  typename SiftKernels<R>::Params sp{}, wp{};
+  int grid = 0, wgrid = 0;
+  sp.batch = INT_MAX;
+  wp.batch = p->num_sms;
+  int rc = prepare_sift<R>(p, sp, max_n, &grid);
+  if (rc == EMDB_OK) rc = prepare_sift<R>(p, wp, max_n, &wgrid, hands_over<R>(p, sp.variant) ? 1 : 0);
+  if (rc) return rc;
+  const size_t bytes = std::max(sp.slab_stride * (size_t)grid, wp.slab_stride * (size_t)wgrid);
+  if (bytes > kReserveMost) return EMDB_OK;
+  size_t cont_stride = 0;
+  if (hands_over<R>(p, sp.variant)) rc = ensure_tail<R>(p->tail_dev, grid, max_n, &cont_stride);
+  return rc ? rc : ensure_slab(p, bytes);
+}
+
 }  // namespace
 
 extern "C" {
@@ -621,6 +643,18 @@ int emdb_plan_query(emdb_plan* p, int max_n, int* arena_bytes, int* ctas_per_sm,
 int emdb_plan_query_f32(emdb_plan* p, int max_n, int* arena_bytes, int* ctas_per_sm,
                         int* grid_max) {
   return plan_query<float>(p, max_n, arena_bytes, ctas_per_sm, grid_max);
+}
+
+int emdb_plan_reserve(emdb_plan* p, int max_n, int real_bytes) {
+  NvtxRange nvtx_range("emdb_plan_reserve");
+  if (!p) return fail(EMDB_ERR_INVALID, "plan is NULL");
+  if (max_n < 0 || (real_bytes != 8 && real_bytes != 4))
+    return fail(EMDB_ERR_INVALID, "max_n must be >= 0 and real_bytes 8 or 4");
+  std::lock_guard<std::mutex> lk(p->mu);
+  DeviceGuard g(p->device);
+  const int rc = real_bytes == 4 ? reserve<float>(p, max_n) : reserve<double>(p, max_n);
+  if (rc == EMDB_ERR_NOMEM) cudaGetLastError();   // the caller may go on without: no launch reports it
+  return rc;
 }
 
 int emdb_host_bytes(emdb_plan* p, unsigned long long* h2d, unsigned long long* d2h) {

@@ -39,7 +39,7 @@ EXPORTS = ("emdb_version", "emdb_plan_create", "emdb_plan_destroy", "emdb_plan_s
            "emdb_notify_create", "emdb_notify_reset", "emdb_notify_destroy",
            "emdb_run_ragged_notify", "emdb_pass_placement", "emdb_noalloc_status",
            "emdb_pack_rows", "emdb_run_f32", "emdb_run_ragged_f32", "emdb_envelope_f32",
-           "emdb_plan_query_f32", "emdb_plan_set_tail")
+           "emdb_plan_query_f32", "emdb_plan_set_tail", "emdb_plan_reserve")
 
 
 class EmdbConfig(ctypes.Structure):
@@ -80,6 +80,7 @@ def load() -> ctypes.CDLL:
         L.emdb_plan_set_variant.argtypes = [VP, I]
         L.emdb_plan_set_max_ctas.argtypes = [VP, I]
         L.emdb_plan_set_tail.argtypes = [VP, I]
+        L.emdb_plan_reserve.argtypes = [VP, I, I]
         L.emdb_plan_phase_clocks.argtypes = [VP, P, I, I]
         L.emdb_plan_query.argtypes = [VP, I, ctypes.POINTER(I), ctypes.POINTER(I), ctypes.POINTER(I)]
         L.emdb_run.argtypes = [VP, P, P, I, I, P, P, P, P, P, P, VP]
@@ -222,6 +223,10 @@ class Plan:
 
     def set_max_ctas(self, max_ctas: int) -> None:
         check(self.L.emdb_plan_set_max_ctas(self.handle, int(max_ctas)), "emdb_plan_set_max_ctas")
+
+    def reserve(self, max_n: int, f32: bool = False) -> None:
+        """Allocate the scratch of the plan's launches of traces up to max_n."""
+        check(self.L.emdb_plan_reserve(self.handle, int(max_n), 4 if f32 else 8), "emdb_plan_reserve")
 
     def query(self, max_n: int, f32: bool = False) -> tuple[int, int, int]:
         """(arena bytes, CTAs per SM, grid) the plan's launches use for traces

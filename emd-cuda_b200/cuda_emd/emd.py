@@ -131,13 +131,17 @@ class GPUBatchEMD:
         """Tiny real calls (an all-zero trace, emd.py:58-64) so that plan creation
         and first-launch costs land here, not in a timed call: one on the kernel
         instance that a batch of more traces than SMs takes, one on that of a
-        smaller batch.  Both with a single trace: scratch grows with the batch,
-        and what a warm-up of more traces than SMs allocates (25 MB) the first
-        real call would have to free."""
+        smaller batch.  The scratch for any batch is allocated at once (about
+        100 MB, most of it the same for all lengths): a call that has to grow it
+        waits for the driver twice, whatever the size."""
         import torch
         f32 = self._config.f32
         x = torch.zeros((1, N), dtype=torch.float32 if f32 else torch.float64, device="cuda")
         plan = self._get_launcher()._plan
+        try:
+            plan.reserve(N, f32)
+        except MemoryError:
+            pass                              # the calls allocate what they need
         if plan.by_length():
             # an automatic instance is numbered by its CTAs per SM
             plan.set_variant(plan.query(N, f32)[1])
