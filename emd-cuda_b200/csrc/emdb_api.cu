@@ -4,7 +4,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <climits>
 #include <chrono>
 #include <condition_variable>
 #include <cstdio>
@@ -28,14 +27,13 @@ struct emdb_plan {
   int variant = 0;            // kernel instance (register variant); 0 = by trace length
   int max_ctas = 0;           // cap on a launch's persistent grid (0 = resident CTAs)
   int tail = -1;              // tail migration: 0 off, -1 two or three per SM, > 0 that many
-  // tail migration's counters and records, one set for device launches and one
-  // for the host pipeline (whose launches run on streams of their own)
+  // tail migration's counters, one set for device launches and one for the host
+  // pipeline (whose launches run on streams of their own); the continuation
+  // records lie behind the launches' slabs, in the same allocation
   struct Tail {
     int* counters = nullptr;  // [0] traces in flight, [1] resume tickets, [2] traces started
     int* valid = nullptr;
     int valid_cap = 0;
-    char* cont = nullptr;     // continuation records
-    size_t cont_bytes = 0;
   } tail_dev, tail_host;
   int* d_ctl = nullptr;       // [0] sift queue, [1] status, [2] envelope queue
   unsigned long long* d_cnt = nullptr;  // [0] sift passes, [1] spilled passes, [2] / [3]
@@ -372,10 +370,14 @@ int prepare_sift(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, i
   return EMDB_OK;
 }
 
-// Device buffers of tail migration for `grid` CTAs and traces up to max_n.
+// Bytes of a continuation record for traces up to max_n.
 template <typename R>
-int ensure_tail(emdb_plan::Tail& t, int grid, int max_n, size_t* stride) {
-  *stride = al256(emdb::cont_data_off() + (size_t)std::max(max_n, 1) * sizeof(R));
+size_t record_bytes(int max_n) {
+  return al256(emdb::cont_data_off() + (size_t)std::max(max_n, 1) * sizeof(R));
+}
+
+// Counters of tail migration for `grid` CTAs.
+int ensure_tail(emdb_plan::Tail& t, int grid) {
   cudaError_t e = cudaSuccess;
   if (!t.counters) e = cudaMalloc(&t.counters, 3 * sizeof(int));
   if (e == cudaSuccess && grid > t.valid_cap) {
@@ -385,15 +387,7 @@ int ensure_tail(emdb_plan::Tail& t, int grid, int max_n, size_t* stride) {
     e = cudaMalloc(&t.valid, (size_t)grid * sizeof(int));
     if (e == cudaSuccess) t.valid_cap = grid;
   }
-  const size_t bytes = *stride * (size_t)grid;
-  if (e == cudaSuccess && bytes > t.cont_bytes) {
-    if (t.cont) cudaFree(t.cont);
-    t.cont = nullptr;
-    t.cont_bytes = 0;
-    e = cudaMalloc(&t.cont, bytes);
-    if (e == cudaSuccess) t.cont_bytes = bytes;
-  }
-  if (e != cudaSuccess) return cuda_fail(e, "allocating the tail-migration records");
+  if (e != cudaSuccess) return cuda_fail(e, "allocating the tail-migration counters");
   return EMDB_OK;
 }
 
@@ -405,12 +399,12 @@ bool hands_over(const emdb_plan* p, int variant) {
 }
 
 // Tail migration for launches of `grid` CTAs in all over `total` traces: zeroes
-// the counters and records on `st`, sets sp's fields, and makes rp (a resume
-// launch's parameters, from prepare_sift) take the records.
+// the counters on `st`, sets sp's fields, and makes rp (a resume launch's
+// parameters, from prepare_sift) take the records, which start at `cont`.
 template <typename R>
 int set_up_tail(const emdb_plan* p, const emdb_plan::Tail& t, typename SiftKernels<R>::Params& sp,
-                typename SiftKernels<R>::Params& rp, int grid, int total, size_t cont_stride,
-                cudaStream_t st) {
+                typename SiftKernels<R>::Params& rp, int grid, int total, char* cont,
+                size_t cont_stride, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(t.counters, 0, 3 * sizeof(int), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(t.valid, 0, (size_t)grid * sizeof(int), st);
   if (e != cudaSuccess) return cuda_fail(e, "tail reset");
@@ -425,14 +419,14 @@ int set_up_tail(const emdb_plan* p, const emdb_plan::Tail& t, typename SiftKerne
   // 4096 35.5; 28.0 / 27.7 / 27.1, 6,000 x 4096 101.5; 96.8 / 96.3 / 95.6, 300 x
   // 3000 9.8; 8.6 / 8.5 / 8.4.
   sp.yield_below = p->tail < 0 ? (sp.variant == 2 ? 2 : 3) * p->num_sms : p->tail;
-  sp.cont_buf = t.cont;
+  sp.cont_buf = cont;
   sp.cont_stride = cont_stride;
   sp.cont_valid = t.valid;
   sp.cont_cap = grid;
   sp.cont_ticket = t.counters + 1;
   sp.resume = 0;
   rp.active = rp.started = nullptr;
-  rp.cont_buf = t.cont;
+  rp.cont_buf = cont;
   rp.cont_stride = cont_stride;
   rp.cont_valid = t.valid;
   rp.cont_cap = grid;
@@ -441,34 +435,61 @@ int set_up_tail(const emdb_plan* p, const emdb_plan::Tail& t, typename SiftKerne
   return EMDB_OK;
 }
 
+// A launch of sp.batch traces up to max_n, and the resume launch that takes its
+// last traces over if it hands them over (tail migration).
+template <typename R>
+struct Launches {
+  int grid = 0, rgrid = 0;
+  bool tail = false;
+  typename SiftKernels<R>::Params rp{};
+  size_t slab = 0, cont_stride = 0;
+  // one allocation holds the slabs (the two launches run one after the other)
+  // and, behind them, the continuation records
+  size_t scratch() const { return slab + cont_stride * (size_t)grid; }
+};
+
+template <typename R>
+int prepare_launches(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, Launches<R>* l) {
+  int rc = prepare_sift<R>(p, sp, max_n, &l->grid);
+  if (rc) return rc;
+  l->slab = sp.slab_stride * (size_t)l->grid;
+  l->tail = hands_over<R>(p, sp.variant);
+  if (l->tail) {
+    l->rp = sp;
+    rc = prepare_sift<R>(p, l->rp, max_n, &l->rgrid, 1);
+    if (rc) return rc;
+    l->rgrid = std::min(l->rgrid, l->grid);
+    l->slab = std::max(l->slab, l->rp.slab_stride * (size_t)l->rgrid);
+    l->cont_stride = record_bytes<R>(max_n);
+  }
+  l->slab = al256(l->slab);
+  return EMDB_OK;
+}
+
+// The launches' scratch: at most one allocation, and one given back.
+template <typename R>
+int ensure_scratch(emdb_plan* p, const Launches<R>& l) {
+  const int rc = l.tail ? ensure_tail(p->tail_dev, l.grid) : EMDB_OK;
+  return rc ? rc : ensure_slab(p, l.scratch());
+}
+
 template <typename R = double>
 int launch_common(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, cudaStream_t st) {
-  int grid = 0;
-  int rc = prepare_sift<R>(p, sp, max_n, &grid);
+  Launches<R> l;
+  int rc = prepare_launches<R>(p, sp, max_n, &l);
+  if (rc == EMDB_OK) rc = ensure_scratch<R>(p, l);
   if (rc) return rc;
   // tail migration: the traces still in flight when the queue runs dry move
   // to a second launch of the 512-thread instance
-  const bool tail = hands_over<R>(p, sp.variant);
-  typename SiftKernels<R>::Params rp{};
-  int rgrid = 0;
-  size_t cont_stride = 0;
-  if (tail) {
-    rp = sp;
-    rc = prepare_sift<R>(p, rp, max_n, &rgrid, 1);
-    if (rc) return rc;
-    rgrid = std::min(rgrid, grid);
-    rc = ensure_tail<R>(p->tail_dev, grid, max_n, &cont_stride);
-    if (rc) return rc;
-  }
-  rc = ensure_slab(p, std::max(sp.slab_stride * (size_t)grid,
-                               tail ? rp.slab_stride * (size_t)rgrid : 0));
-  if (rc) return rc;
+  const bool tail = l.tail;
+  const int grid = l.grid, rgrid = l.rgrid;
+  typename SiftKernels<R>::Params& rp = l.rp;
   sp.queue = rp.queue = p->d_ctl;
   sp.slab = rp.slab = p->d_slab;
   cudaError_t e = cudaMemsetAsync(p->d_ctl, 0, sizeof(int), st);
   if (e != cudaSuccess) return cuda_fail(e, "queue reset");
   if (tail) {
-    rc = set_up_tail<R>(p, p->tail_dev, sp, rp, grid, sp.batch, cont_stride, st);
+    rc = set_up_tail<R>(p, p->tail_dev, sp, rp, grid, sp.batch, p->d_slab + l.slab, l.cont_stride, st);
     if (rc) return rc;
   }
   e = SiftKernels<R>::launch(sp, grid, st);
@@ -480,24 +501,25 @@ int launch_common(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, 
   return EMDB_OK;
 }
 
-// Scratch for a launch of any batch of traces up to max_n, and for batches of
-// at most one trace per SM; none if it were more than kReserveMost (the default
-// config takes 97 MB, for float launches 122; it grows with max_extrema).
+// Scratch for a launch of up to `batch` traces of up to max_n samples; none if it
+// were more than kReserveMost.  A smaller batch never takes more than the most
+// traces that still start on the 512-thread instance (one per SM) or `batch`.
 constexpr size_t kReserveMost = size_t(256) << 20;
 
 template <typename R>
-int reserve(emdb_plan* p, int max_n) {
-  typename SiftKernels<R>::Params sp{}, wp{};
-  int grid = 0, wgrid = 0;
-  sp.batch = INT_MAX;
-  wp.batch = p->num_sms;
-  int rc = prepare_sift<R>(p, sp, max_n, &grid);
-  if (rc == EMDB_OK) rc = prepare_sift<R>(p, wp, max_n, &wgrid, hands_over<R>(p, sp.variant) ? 1 : 0);
-  if (rc) return rc;
-  const size_t bytes = std::max(sp.slab_stride * (size_t)grid, wp.slab_stride * (size_t)wgrid);
+int reserve(emdb_plan* p, int batch, int max_n) {
+  size_t bytes = 0;
+  Launches<R> l;
+  for (int b : {std::min(batch, p->num_sms), batch}) {
+    typename SiftKernels<R>::Params sp{};
+    sp.batch = b;
+    l = Launches<R>();
+    const int rc = prepare_launches<R>(p, sp, max_n, &l);
+    if (rc) return rc;
+    bytes = std::max(bytes, l.scratch());
+  }
   if (bytes > kReserveMost) return EMDB_OK;
-  size_t cont_stride = 0;
-  if (hands_over<R>(p, sp.variant)) rc = ensure_tail<R>(p->tail_dev, grid, max_n, &cont_stride);
+  const int rc = l.tail ? ensure_tail(p->tail_dev, l.grid) : EMDB_OK;
   return rc ? rc : ensure_slab(p, bytes);
 }
 
@@ -557,7 +579,6 @@ int emdb_plan_destroy(emdb_plan* p) {
     for (emdb_plan::Tail* t : {&p->tail_dev, &p->tail_host}) {
       if (t->counters) cudaFree(t->counters);
       if (t->valid) cudaFree(t->valid);
-      if (t->cont) cudaFree(t->cont);
     }
     if (p->d_ctl) cudaFree(p->d_ctl);
     if (p->d_cnt) cudaFree(p->d_cnt);
@@ -645,14 +666,15 @@ int emdb_plan_query_f32(emdb_plan* p, int max_n, int* arena_bytes, int* ctas_per
   return plan_query<float>(p, max_n, arena_bytes, ctas_per_sm, grid_max);
 }
 
-int emdb_plan_reserve(emdb_plan* p, int max_n, int real_bytes) {
+int emdb_plan_reserve(emdb_plan* p, int batch, int max_n, int real_bytes) {
   NvtxRange nvtx_range("emdb_plan_reserve");
   if (!p) return fail(EMDB_ERR_INVALID, "plan is NULL");
-  if (max_n < 0 || (real_bytes != 8 && real_bytes != 4))
-    return fail(EMDB_ERR_INVALID, "max_n must be >= 0 and real_bytes 8 or 4");
+  if (batch < 0 || max_n < 0 || (real_bytes != 8 && real_bytes != 4))
+    return fail(EMDB_ERR_INVALID, "batch and max_n must be >= 0 and real_bytes 8 or 4");
+  if (batch == 0) return EMDB_OK;
   std::lock_guard<std::mutex> lk(p->mu);
   DeviceGuard g(p->device);
-  const int rc = real_bytes == 4 ? reserve<float>(p, max_n) : reserve<double>(p, max_n);
+  const int rc = real_bytes == 4 ? reserve<float>(p, batch, max_n) : reserve<double>(p, batch, max_n);
   if (rc == EMDB_ERR_NOMEM) cudaGetLastError();   // the caller may go on without: no launch reports it
   return rc;
 }
@@ -839,18 +861,22 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
   if (tail) {
     rp.batch = batch;
     int rc = prepare_sift<double>(p, rp, N, &rgrid, 1);
-    if (rc == EMDB_OK) rc = ensure_tail<double>(p->tail_host, grid_all, N, &cont_stride);
+    if (rc == EMDB_OK) rc = ensure_tail(p->tail_host, grid_all);
     if (rc) return rc;
     rgrid = std::min(rgrid, grid_all);
     slab_need = std::max(slab_need, (size_t)rgrid * rp.slab_stride);
+    cont_stride = record_bytes<double>(N);
   }
-  if (slab_need > p->group_slab_bytes) {
+  // the slabs and, behind them, the continuation records
+  slab_need = al(slab_need);
+  const size_t scratch = slab_need + cont_stride * (size_t)grid_all;
+  if (scratch > p->group_slab_bytes) {
     if (p->d_group_slab) cudaFree(p->d_group_slab);
     p->d_group_slab = nullptr;
     p->group_slab_bytes = 0;
-    e = cudaMalloc(&p->d_group_slab, slab_need);
+    e = cudaMalloc(&p->d_group_slab, scratch);
     if (e != cudaSuccess) return cuda_fail(e, "allocating host-pipeline spill slabs");
-    p->group_slab_bytes = slab_need;
+    p->group_slab_bytes = scratch;
   }
 
   // inputs group by group on the caller's stream; each group launches on its
@@ -861,7 +887,8 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
   if (e == cudaSuccess && T) e = cudaMemcpyAsync(d_T, T, n * 8, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cuda_fail(e, "host-pipeline set-up");
   if (tail) {
-    int rc = set_up_tail<double>(p, p->tail_host, base, rp, grid_all, batch, cont_stride, st);
+    int rc = set_up_tail<double>(p, p->tail_host, base, rp, grid_all, batch,
+                                 p->d_group_slab + slab_need, cont_stride, st);
     if (rc) return rc;
   }
   unsigned long long h2d = (unsigned long long)(B * n * 8 + (T ? n * 8 : 0)), d2h = 0;

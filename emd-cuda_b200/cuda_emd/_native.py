@@ -80,7 +80,7 @@ def load() -> ctypes.CDLL:
         L.emdb_plan_set_variant.argtypes = [VP, I]
         L.emdb_plan_set_max_ctas.argtypes = [VP, I]
         L.emdb_plan_set_tail.argtypes = [VP, I]
-        L.emdb_plan_reserve.argtypes = [VP, I, I]
+        L.emdb_plan_reserve.argtypes = [VP, I, I, I]
         L.emdb_plan_phase_clocks.argtypes = [VP, P, I, I]
         L.emdb_plan_query.argtypes = [VP, I, ctypes.POINTER(I), ctypes.POINTER(I), ctypes.POINTER(I)]
         L.emdb_run.argtypes = [VP, P, P, I, I, P, P, P, P, P, P, VP]
@@ -224,9 +224,10 @@ class Plan:
     def set_max_ctas(self, max_ctas: int) -> None:
         check(self.L.emdb_plan_set_max_ctas(self.handle, int(max_ctas)), "emdb_plan_set_max_ctas")
 
-    def reserve(self, max_n: int, f32: bool = False) -> None:
-        """Allocate the scratch of the plan's launches of traces up to max_n."""
-        check(self.L.emdb_plan_reserve(self.handle, int(max_n), 4 if f32 else 8), "emdb_plan_reserve")
+    def reserve(self, batch: int, max_n: int, f32: bool = False) -> None:
+        """Allocate the scratch of launches of up to `batch` traces up to max_n."""
+        check(self.L.emdb_plan_reserve(self.handle, int(batch), int(max_n), 4 if f32 else 8),
+              "emdb_plan_reserve")
 
     def query(self, max_n: int, f32: bool = False) -> tuple[int, int, int]:
         """(arena bytes, CTAs per SM, grid) the plan's launches use for traces

@@ -127,19 +127,20 @@ class GPUBatchEMD:
     def config(self) -> EMDKernelConfig:
         return self._config
 
-    def warmup(self, N: int = 64) -> None:
+    def warmup(self, N: int = 64, batch: int | None = None) -> None:
         """Tiny real calls (an all-zero trace, emd.py:58-64) so that plan creation
         and first-launch costs land here, not in a timed call: one on the kernel
         instance that a batch of more traces than SMs takes, one on that of a
-        smaller batch.  The scratch for any batch is allocated at once (about
-        100 MB, most of it the same for all lengths): a call that has to grow it
-        waits for the driver twice, whatever the size."""
+        smaller batch.  Their scratch is allocated here for batches of up to
+        `batch` traces of N samples (default: one per SM, 25 MB, most of it the
+        same for every length); a call that needs more allocates it."""
         import torch
         f32 = self._config.f32
         x = torch.zeros((1, N), dtype=torch.float32 if f32 else torch.float64, device="cuda")
         plan = self._get_launcher()._plan
         try:
-            plan.reserve(N, f32)
+            plan.reserve(batch or torch.cuda.get_device_properties(plan.device).multi_processor_count,
+                         N, f32)
         except MemoryError:
             pass                              # the calls allocate what they need
         if plan.by_length():

@@ -100,15 +100,14 @@ int emdb_plan_set_tail(emdb_plan* plan, int yield_below);
 /* Arena and CTAs/SM the plan would use for traces up to max_n. */
 int emdb_plan_query(emdb_plan* plan, int max_n, int* arena_bytes, int* ctas_per_sm,
                     int* grid_max);
-/* Allocate the scratch that a launch of any batch of traces up to max_n
- * samples needs (real_bytes 8: emdb_run and emdb_run_ragged, 4: their float
- * forms), so that the first such launch allocates nothing: scratch grows with
- * the batch until the GPU is full, and a growth inside a call frees and
- * allocates, which costs the driver as long for 1 MB as for 100.  Nothing is
- * allocated if it were more than 256 MB (a max_extrema far above the default):
- * scratch then grows with the calls.  No reference
+/* Allocate the scratch that launches of up to `batch` traces of up to max_n
+ * samples need (real_bytes 8: emdb_run and emdb_run_ragged, 4: their float
+ * forms), so that they allocate nothing.  Scratch grows with the batch until the
+ * GPU is full, and a growth inside a call frees and allocates, for which the
+ * driver takes about 0.3 and 0.4 ms whatever the size.  Nothing is allocated if
+ * it were more than 256 MB: scratch then grows with the calls.  No reference
  * counterpart (its scratch is a CuPy array per call, kernels.py:1354-1361). */
-int emdb_plan_reserve(emdb_plan* plan, int max_n, int real_bytes);
+int emdb_plan_reserve(emdb_plan* plan, int batch, int max_n, int real_bytes);
 /* Smallest arena (bytes) that holds a trace of max_n samples: its proto-IMF,
  * control block and scan masks; every knot then lives in the global slab.
  * No reference counterpart (the reference sizes one fixed knot buffer per

@@ -18,15 +18,17 @@ def test_warmup_allocates_the_scratch_and_keeps_the_plan(real, n):
     plan = EMDKernelConfig(real_t=real).build()._plan
     ctas = plan.query(n, first.config.f32)[1]
     assert ctas == (4 if real == "float" else 2) if n == 3000 else ctas == (5 if real == "float" else 4)
-    first(X)                                     # and fills torch's cache of outputs
-    emd = GPUBatchEMD(cfg)
-    emd.warmup(n)
-    torch.cuda.synchronize()
-    assert tuple(emd.last_debug[0].shape) == (1, cfg.max_imfs)
-    free = torch.cuda.mem_get_info()[0]
-    emd(X)
-    torch.cuda.synchronize()
-    assert free - torch.cuda.mem_get_info()[0] < 4 << 20
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for batch, x in ((None, X[:sms]), (900, X), (900, X[:sms]), (900, X[:500])):
+        first(x)                                 # fills torch's cache of outputs
+        emd = GPUBatchEMD(cfg)
+        emd.warmup(n, batch)
+        torch.cuda.synchronize()
+        assert tuple(emd.last_debug[0].shape) == (1, cfg.max_imfs)
+        free = torch.cuda.mem_get_info()[0]
+        emd(x)
+        torch.cuda.synchronize()
+        assert free - torch.cuda.mem_get_info()[0] < 4 << 20, batch
     assert emd._launcher._plan.by_length()
     for a, b in zip(first(X), emd(X)):
         assert torch.equal(a, b)
