@@ -134,7 +134,8 @@ struct Ctl {
   int job;
   int head[2][kMaxNbsym + 1];  // first NB+1 extrema indices per side (0 = max, 1 = min)
   int tail[2][kMaxNbsym + 1];  // tail[q][k] = index of extremum n_q-1-k
-  int unused[40];              // keeps the block's size: it decides the longest trace a CTA takes
+  int zero_first;              // the scanned trace starts with a zero (N > kFallbackFrom)
+  int unused[39];              // keeps the block's size: it decides the longest trace a CTA takes
   int lsym, rsym;
   int kbase[2], kcnt[2];
   int dbg_n[kMaxImfsCap], dbg_e[kMaxImfsCap], dbg_z[kMaxImfsCap];
@@ -161,7 +162,7 @@ __host__ __device__ constexpr int scan_slots() {
 }
 
 // Per-warp scan counts live right after the control block, one 16-byte word a
-// warp: maxima | minima << 16, sign changes, zero-run ends, flags (kScan*)
+// warp: maxima | minima << 16, sign changes, zero-run ends, fallback trigger
 // (room for 5 ints a warp).
 struct SmemLayout {
   Ctl* ctl;
@@ -594,8 +595,6 @@ struct TimeAxis {
 // Extrema: count pass (find_extrema_parallel semantics, kernels.py:231-349,
 // with the serial scan's plateau rule, kernels.py:157-200).
 // ---------------------------------------------------------------------------
-// Flags of a warp's scan word
-enum : uint32_t { kScanTrig = 1, kScanZeroFirst = 2 };
 // Longest trace whose zero-crossing count no chunk fallback can change
 constexpr int kFallbackFrom = kThreads * 128;
 
@@ -660,13 +659,7 @@ __device__ __forceinline__ void extrema_count(const SmemLayout& L, int N, int sl
     zc += __popc(__ballot_sync(kFull, sc));
   }
   trig = __any_sync(kFull, trig);
-  if (lane == 0) {
-    // what extrema_scan decides by has to be read here: after its barrier
-    // other warps may be writing the residue into imf[] already
-    const bool zero_first = slot == 0 && N > kFallbackFrom && imf[0] == real(0);
-    L.wc[slot] = make_uint4(run, (uint32_t)zc, (uint32_t)zre,
-                            (trig ? kScanTrig : 0u) | (zero_first ? kScanZeroFirst : 0u));
-  }
+  if (lane == 0) L.wc[slot] = make_uint4(run, (uint32_t)zc, (uint32_t)zre, trig ? 1u : 0u);
 }
 
 struct ExtInfo {
@@ -675,7 +668,6 @@ struct ExtInfo {
   uint32_t off;           // this warp's rank offsets: maxima | minima << 16
   bool overflow;
   bool trig;              // serial-fallback trigger (exact zeros / flat runs)
-  bool zero_first;        // N > kFallbackFrom and the first sample is zero
 };
 
 // After the count pass + barrier.  Reproduces the parallel/serial split of
@@ -693,8 +685,7 @@ __device__ __forceinline__ ExtInfo extrema_totals(const SmemLayout& L, int warp,
   const uint32_t zc = __reduce_add_sync(kFull, w.y);
   ExtInfo e;
   e.off = __reduce_add_sync(kFull, lane < warp ? w.x : 0u);
-  e.trig = __any_sync(kFull, (w.w & kScanTrig) != 0u);
-  e.zero_first = __any_sync(kFull, (w.w & kScanZeroFirst) != 0u);
+  e.trig = __any_sync(kFull, w.w != 0u);
   e.n_zer = (int)zc;
   if (e.trig || L.ctl->chunk_bad) e.n_zer += (int)__reduce_add_sync(kFull, w.z);
   const int tot_max = (int)(tot & 0xffffu), tot_min = (int)(tot >> 16);
@@ -731,16 +722,19 @@ __device__ void chunk_fallback_check(const SmemLayout& L, int N, int tid) {
 // and its warp's rank offsets.  Nothing here reads imf[] after the last
 // barrier: the caller may write it at once (the emission of a row does), and a
 // warp that came late to a test on imf[] would enter the fallback's barriers
-// alone.
+// alone.  So thread 0 looks at the first sample before it.
 template <int NT>
 __device__ __forceinline__ ExtInfo extrema_scan(const SmemLayout& L, int N, int tid, int warp,
                                                 int lane, int max_extrema) {
   constexpr int NS = scan_slots<NT>();
   extrema_count<NS>(L, N, warp, lane);
-  if (tid == 0) L.ctl->chunk_bad = 0;
+  if (tid == 0) {
+    L.ctl->chunk_bad = 0;
+    if (N > kFallbackFrom) L.ctl->zero_first = L.imf[0] == real(0);
+  }
   __syncthreads();
   ExtInfo e = extrema_totals<NS>(L, warp, lane, max_extrema);
-  if (e.zero_first && !e.trig) {
+  if (N > kFallbackFrom && L.ctl->zero_first && !e.trig) {
     chunk_fallback_check(L, N, tid);
     e = extrema_totals<NS>(L, warp, lane, max_extrema);
   }
