@@ -784,7 +784,8 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
     if (e != cudaSuccess) return cuda_fail(e, "allocating host-pipeline staging");
     p->stage_bytes = total;
   }
-  constexpr int kMaxChunks = 256, kMinChunk = 8;
+  constexpr int kMaxChunks = 256, kMinChunk = 8, kMostMinChunk = 64;
+  constexpr size_t kMinChunkBytes = size_t(2) << 20;
   constexpr int kG = emdb_plan::kGroups;
   if (!p->copy_stream) {
     e = cudaStreamCreateWithFlags(&p->copy_stream, cudaStreamNonBlocking);
@@ -806,9 +807,16 @@ int emdb_run_host(emdb_plan* p, const double* signals, const double* T, int batc
   // when its slowest trace is done, so few traces a chunk let most rows cross
   // the bus during the sift (B200, 2,048 x 2048 seismic, chunks of 64 / 32 / 16 /
   // 8 / 4 traces: 12.5 / 11.4 / 10.6 / 9.9 / 9.9 ms, with the hand-over below; 13.3
-  // and 10.0 without and with it at 8).  Groups are whole chunks (4 groups for
-  // large batches, so the first launch starts after a quarter of the input copy).
-  const int chunk = std::max(kMinChunk, (batch + kMaxChunks - 1) / kMaxChunks);
+  // and 10.0 without and with it at 8).  But a copy takes about 5 us however
+  // short, which a batch of short traces does not hide: a chunk has at least
+  // 2 MB of rows (dense; 64 traces are enough).  Floors of 0 / 1 / 2 / 4 MB, ms: 4,096 x
+  // 300 tones 2.81 / 2.42 / 2.15 / 2.17, 1,024 x 512 1.48 / 1.27 / 1.20 / 1.26, 2,048 x
+  // 700 3.18 / 2.86 / 2.54 / 2.43, 2,048 x 2048 seismic 10.2 / 10.4 / 10.0 / 10.5.  Groups
+  // are whole chunks (4 groups for large batches, so the first launch starts
+  // after a quarter of the input copy).
+  const int full = (int)std::min<size_t>(
+      kMostMinChunk, kMinChunkBytes / std::max<size_t>(1, (size_t)mi * n * sizeof(double)));
+  const int chunk = std::max({kMinChunk, full, (batch + kMaxChunks - 1) / kMaxChunks});
   const int nchunk = (batch + chunk - 1) / chunk;
   const int ngroup = batch >= 1024 ? kG : 1;
   volatile unsigned* flag = p->h_chunk_flag;
