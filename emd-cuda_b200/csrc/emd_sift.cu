@@ -948,7 +948,19 @@ __device__ __forceinline__ const real2& pair_at(const char* p) {
   return *reinterpret_cast<const real2*>(p);
 }
 
-// The PCR levels from stride s on with the division itself, rows of two systems
+// The quotient with its range test: FP64 from the approximate reciprocal where
+// that is exact.
+__device__ __forceinline__ real div_any(real a, real b) {
+#if EMDB_F32
+  return a / b;
+#else
+  bool slow = false;
+  const real q = div_nb(a, b, slow);
+  return slow ? div_slow(a, b) : q;
+#endif
+}
+
+// The PCR levels from stride s on, each quotient tested, rows of two systems
 // in buffer `cur` (kernels.py:651-668, in the reference's operation order);
 // the result ends up in buffer 1.  The whole CTA calls it, for the systems that
 // the levels in solve_splines do not cover.
@@ -970,8 +982,8 @@ __device__ __noinline__ void pcr_levels_any(char* b0, char* b1, int m0, int m1, 
       const real2 o = pair_at(own), p = pair_at(own + kBD);
       const real2 ol = pair_at(l), pl = pair_at(l + kBD);
       const real2 orr = pair_at(rr), pr = pair_at(rr + kBD);
-      const real alpha = hl ? o.x / pl.x : real(0);
-      const real beta = hr ? o.y / pr.x : real(0);
+      const real alpha = hl ? div_any(o.x, pl.x) : real(0);
+      const real beta = hr ? div_any(o.y, pr.x) : real(0);
       char* to = dst + row_at(r);
       pair_at(to) = real2{-alpha * ol.x, -beta * orr.y};
       pair_at(to + kBD) = real2{p.x - alpha * ol.y - beta * orr.x,
@@ -1059,8 +1071,10 @@ __device__ __forceinline__ real pcr_last(const char* own, const char* l, const c
 // pcr_levels_any, and so do the levels past the fifth where the vote on those
 // fails (its window for d is 2^23 either way of the middle row's).
 // Returns (the same in every thread) whether the evaluation needs no test of
-// spacings and moments: the condition on spacings above and every moment zero
-// or in [2^-700, 2^900).
+// spacings and moments: on the integer axis the condition on spacings above, on
+// a given one spacings in [2^-100, 2^100) -- however far from each other, so an
+// axis with a gap of any length keeps it -- and every moment zero or in [2^-700,
+// 2^900).
 // FP32: the same on the integer axis.  A coupling entering the fourth level is
 // a spacing times eight multipliers h_k / (2 (h_k + h_k+1)), each at least a
 // quarter, or a quarter of h_k / h_k+1 where spacings rise: with at most four
@@ -1099,6 +1113,7 @@ __device__ __forceinline__ bool solve_splines(const Knots& K, int kbase0, int kb
   const int z0 = m0 > 0 ? m0 + 1 : 0, zt = z0 + (m1 > 0 ? m1 + 1 : 0);
   const unsigned href = kInt ? 0u : mag(xy0[1].x - xy0[0].x) - (12u << kFrac);
   bool odd = false;
+  bool far = false;           // given axis: a spacing that the evaluation's quotients don't take
 #pragma unroll 1
   for (int zb = (tid >> 5) * 31; zb < zt; zb += (NT / 32) * 31) {
     const int z = zb + (tid & 31);
@@ -1111,7 +1126,10 @@ __device__ __forceinline__ bool solve_splines(const Knots& K, int kbase0, int kb
       h = p1.x - p0.x;
       sl = (p1.y - p0.y) / h;
       if (kInt) odd |= !(h >= real(1) && h <= real(kMaxIntSeg));
-      else if (kDouble) odd |= !(h > real(0)) || mag(h) - href >= (24u << kFrac);
+      else if (kDouble) {
+        odd |= !(h > real(0)) || mag(h) - href >= (24u << kFrac);
+        far |= !(h > real(0)) || mag(h) - ((kBias - 100u) << kFrac) >= (200u << kFrac);
+      }
     }
     const real hm = __shfl_up_sync(kFull, h, 1), sm = __shfl_up_sync(kFull, sl, 1);
     if (z < zt && (tid & 31) != 0 && g > 0) {
@@ -1132,7 +1150,7 @@ __device__ __forceinline__ bool solve_splines(const Knots& K, int kbase0, int kb
   }
   if (!kInt && kDouble) odd |= href - ((kBias - 100u) << kFrac) >= (176u << kFrac);
   const bool plain = !__syncthreads_or(odd);
-  odd = !plain;
+  odd = kInt ? !plain : far;
   EMDB_PH(&C, 2);
   bool fused = false;
   int s = 1;
