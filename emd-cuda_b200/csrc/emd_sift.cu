@@ -50,18 +50,17 @@
 
 #include "emdb_internal.cuh"
 
+// Settled when the passes were longer (16,384 x 2048 seismic took 79 ms, now 53):
+// one sift-pass instance for the on-chip placements and one for the off-chip
+// ones (208.4k signals/s; one instance for all 195.6k, one per placement 184.9k),
+// the six end-of-pass trees spread over the warps (188.1k on one warp):
+// instruction supply decides as much as FP64 latency.
 // Tuning knobs (compile-time; results are identical for every setting):
-// Settled: one sift-pass instance for the on-chip placements and one for the
-// off-chip ones (16,384 x 2048 seismic 208.4k signals/s; one instance for all
-// 195.6k, one per placement 184.9k), the six end-of-pass trees spread over the
-// warps (188.1k on one warp): instruction supply decides as much as FP64
-// latency.
 //  EMDB_LANE_UNROLL  wide instances: unroll factor of the lane-sum loops (the
 //                  loads of a lane's samples in flight at once).  With the
 //                  six sums split over the 128-lane groups, B200, 512 threads
-//                  1024 x 8192 seismic / 256 threads 2048 x 4096 (ms): 4:
-//                  296.7 / 47.5, 8: 290.0 / 47.5, 16: 289.9 / 46.8; the sums
-//                  on the first 128 threads only (no split): 293.0 / 46.7.
+//                  1024 x 8192 seismic / 256 threads 2048 x 4096 (ms): 4: 145.5 /
+//                  47.8, 8: 143.0 / 47.4, 16: 142.5 / 47.3.
 #ifndef EMDB_LANE_UNROLL
 #define EMDB_LANE_UNROLL 16
 #endif
@@ -96,7 +95,7 @@ constexpr int kPhases = 10;
 // double and rounded once, as in the reference source compiled with REAL_T =
 // float.  Its quotients (div_q from an IEEE reciprocal; on the integer axis quot
 // and div_core from the approximate one) are self-tested against the float
-// division by emdb_check_division modes 3 and 4; the one double quotient per
+// division by emdb_check_division modes 3, 4 and 6; the one double quotient per
 // envelope sample (the reference's "/ 6.0") is formed from RN(1/6) and its
 // residual (div6), which equals the double division.
 #ifndef EMDB_F32

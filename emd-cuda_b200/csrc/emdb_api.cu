@@ -307,8 +307,9 @@ int prepare_sift(emdb_plan* p, typename SiftKernels<R>::Params& sp, int max_n, i
   // force_variant: that instance at its automatic arena (the tail's resume launch)
   // A batch of at most one trace per SM goes to the 512-thread instance
   // directly, where tail migration would move it anyway after a first launch
-  // that only starts it (B200, host clock, one 1024-sample
-  // trace: 233 / 223 us a call).
+  // that only starts it (B200, host clock, us a call with that pair / directly,
+  // medians of 8 blocks in turn, which spread by 1 to 5 %: one 1024-sample trace
+  // 171 / 157, 8 x 300 192 / 180, 96 x 1501 seismic 1,437 / 1,422).
   if (!force_variant && p->variant == 0 && p->arena_override == 0 && p->tail != 0 &&
       sp.batch <= p->num_sms)
     force_variant = 1;

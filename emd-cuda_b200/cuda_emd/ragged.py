@@ -91,8 +91,10 @@ class Tier:
         self.plan = _native.Plan(cfg.to_c(), device)
         # the tier launches share the GPU (forked streams, the learned split's
         # capped wide launch beside the light one): no tail migration, whose
-        # whole-SM resume launch assumes a launch that owns the GPU (measured:
-        # the learned step fell from 2.07 to 2.64 s with it on)
+        # whole-SM resume launch assumes a launch that owns the GPU.  Where the
+        # long tiers run whole-SM CTAs it changes nothing (2,048 and 8,192 mixed
+        # traces 54.2 and 162.1 ms either way); with 128-thread CTAs in them, on an
+        # earlier kernel, the learned step took 2.64 s with it and 2.07 without
         self.plan.set_tail(0)
         self.arena = 0
         self.variant = 4

@@ -388,8 +388,10 @@ class EMDServer:
             p.set_variant(variant)
             p.set_arena(arena)
             # the plan's tail migration stays on: a serving launch is small,
-            # so its traces move to whole SMs once its queue is empty -- the
-            # measured sweeps favour it at 70 % load and above
+            # so its traces move to whole SMs once its queue is empty (B200,
+            # 160 requests, six warm runs each, on / off: median p99 420 / 700 ms
+            # at 500 traces/s and 510 / 1,090 at 1,000; 8.1-9.1k / 6.1-8.5k traces/s
+            # at saturation)
             _native.check(p.L.emdb_run_ragged_notify(
                 p.handle, vals.data_ptr(), offs.data_ptr(), int(cnt), int(e), None, 1,
                 order.data_ptr(), imfs.data_ptr(), n_imfs.data_ptr(), ovf.data_ptr(),

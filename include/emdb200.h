@@ -73,7 +73,8 @@ int emdb_plan_set_arena(emdb_plan* plan, int arena_bytes);
  * 2 = two 256-thread CTAs per SM; same results bit for bit; 0 (the default)
  * = by trace length: 4 up to 2048 samples, 2 up to 4096, 1 beyond; for float
  * launches 5 up to 2048, 4 up to 4096, 2 up to 16384, 1 beyond (4 when an arena
- * was set).  The ragged autotuner sets one per tier.  A launch whose traces
+ * was set); with tail migration on (emdb_plan_set_tail), 1 for any launch of at
+ * most one trace per SM.  The ragged autotuner sets one per tier.  A launch whose traces
  * do not fit the plan's instance runs on the wide instance at the full
  * shared-memory arena, with the proto-IMF in global memory when shared
  * memory cannot hold it, so any trace length runs. */
@@ -97,7 +98,9 @@ int emdb_plan_set_max_ctas(emdb_plan* plan, int max_ctas);
  * (dense seismic): 2,048 x 2048 samples 11.4 -> 8.6 ms, 16,384 x 2048 54.0 ->
  * 52.5 ms, 1,024 x 4096 35.5 -> 27.1 ms. */
 int emdb_plan_set_tail(emdb_plan* plan, int yield_below);
-/* Arena and CTAs/SM the plan would use for traces up to max_n. */
+/* Arena and CTAs/SM the plan uses for traces up to max_n: those of the instance
+ * that the plan names or that the length selects (a launch of at most one trace
+ * per SM may run on another, see emdb_plan_set_variant). */
 int emdb_plan_query(emdb_plan* plan, int max_n, int* arena_bytes, int* ctas_per_sm,
                     int* grid_max);
 /* Allocate the scratch that launches of up to `batch` traces of up to max_n
