@@ -1771,9 +1771,6 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
     SmemLayout L = carve<NT, kGImf>(smem, N, p.arena_bytes, gimf);
     Ctl& C = *L.ctl;
     real* imf = L.imf;
-    // a record holds the longest trace the launch was announced (max_n); a
-    // longer one that fits the arena all the same finishes here
-    const bool hand_over = migrate && cont_data_off() + (size_t)N * sizeof(real) <= p.cont_stride;
     if (migrate && tid == 0) {
       atomicAdd(p.active, 1);
       atomicAdd(p.started, 1);
@@ -1843,14 +1840,17 @@ __global__ void __launch_bounds__(NT, kMinBlocks) emd_sift_kernel(SiftParams p) 
         }
       }
       if (!emit) {
-        if (hand_over && (n & 3) == 0) {
+        if (migrate && (n & 3) == 0) {
           // every trace has started and few remain: hand this one to the
           // 512-thread instance at this pass boundary (checked every fourth
-          // pass: the two L2 reads and the barrier cost ~1 % per pass)
+          // pass: the two L2 reads and the barrier cost ~1 % per pass).  A record
+          // holds the longest trace the launch was announced (max_n); a longer
+          // one that fits the arena all the same finishes here
           int want = 0;
           if (tid == 0)
             want = *reinterpret_cast<volatile int*>(p.started) >= p.total &&
-                   *reinterpret_cast<volatile int*>(p.active) <= p.yield_below;
+                   *reinterpret_cast<volatile int*>(p.active) <= p.yield_below &&
+                   cont_data_off() + (size_t)N * sizeof(real) <= p.cont_stride;
           if (__syncthreads_or(want)) {
             yielded = true;
             n_yield = n;
